@@ -1260,11 +1260,12 @@ int pbf_mlp_gradients(pbf_mlp_trainer* tr, const float* d_feat, const float* d_t
 
 int pbf_mlp_train_step(pbf_mlp_trainer* tr, const float* d_feat, const float* d_target, int batch, float lr,
                        float* h_loss, void* stream) {
-    int rc = pbf_mlp_gradients(tr, d_feat, d_target, batch, nullptr, nullptr, nullptr, stream);
-    if (rc) return rc;
+    if (!tr || !d_feat || !d_target) return fail(PBF_ERR_INVALID, "null argument");
+    if (batch < 1 || batch > tr->max_batch) return fail(PBF_ERR_INVALID, "batch must lie in [1, max_batch]");
     if (!(lr > 0.0f) || !std::isfinite(lr)) return fail(PBF_ERR_INVALID, "learning rate must be positive");
     cudaStream_t st = (cudaStream_t)stream;
-    if (mlp_adam(tr->t, lr, 0.9f, 0.999f, 1e-8f, st)) return fail(PBF_ERR_CUDA, "Adam kernels failed");
+    if (mlp_train_step(tr->t, d_feat, d_target, batch, lr, 0.9f, 0.999f, 1e-8f, st))
+        return fail(PBF_ERR_CUDA, "training kernels failed");
     if (h_loss) {
         CK(cudaStreamSynchronize(st));
         int err = 0;

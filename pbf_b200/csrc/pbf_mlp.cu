@@ -90,39 +90,18 @@ int tc_gemm_bf16(const void* A, const void* B, float* D, int N, int K, int* err,
 }
 
 // ---------------------------------------------------------------------------
-// Forward pass over 128-row tiles (persistent CTAs). TRAIN additionally saves
-// what the backward pass needs and computes the output-layer gradients.
+// Inference over 128-row tiles (persistent CTAs).
 // ---------------------------------------------------------------------------
-// Per-slot gradient partials of the training forward pass: loss, db4, dw4[64].
-constexpr int FWD_PART = 66;
-
-// out[i] = sum over parts p = 0, 1, ... of part[p * stride + i], in that order
-// (deterministic: the gradients are the same bits on every run)
-__global__ void k_sum_parts(const float* __restrict__ part, int nparts, int stride, int count,
-                            float* __restrict__ out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    float s = 0.0f;
-    for (int q = 0; q < nparts; ++q) s += part[(size_t)q * stride + i];
-    out[i] = s;
-}
-
 struct FwdIO {
     const uint16_t* w;   // bf16 weights
     const float* b;      // biases and constants
     const float* feat;   // raw features [n][12]
     int n;
-    // inference outputs
     float* out;
     float4* q;
     float* lam_acc;
     float clamp;  // trust-region factor around q.w (0: none)
     int floor;    // 1: lambda0 at least as strong as q.w (same sign, magnitude >= |q.w|)
-    // training
-    const float* target;  // [n]
-    float inv_batch;
-    uint16_t *x16, *h1, *h2, *g1, *g2, *dz3;  // [n][16] and [n][64] bf16
-    float* part;  // per tile and warp: loss, db4, dw4[64] (FWD_PART floats; summed by k_sum_parts)
     int* err;
     // failure injection (the bounded-wait test only): no MMA is issued or
     // committed, so every wait on the barrier runs out after wait_limit polls
@@ -136,18 +115,15 @@ constexpr int FWD_SW3 = FWD_SW2 + 64 * 64 * 2;          // [64 x 64]   8 KB
 constexpr int FWD_SX = FWD_SW3 + 64 * 64 * 2;           // [128 x 16]  4 KB
 constexpr int FWD_SH1 = FWD_SX + 128 * 16 * 2;          // [128 x 64] 16 KB
 constexpr int FWD_SH2 = FWD_SH1 + 128 * 64 * 2;         // [128 x 64] 16 KB
-constexpr int FWD_SH3F = FWD_SH2 + 128 * 64 * 2;        // [128 x 64] fp32 32 KB (training)
-constexpr int FWD_SMEM_INFER = FWD_SH3F;
-constexpr int FWD_SMEM_TRAIN = FWD_SH3F + 128 * 64 * 4;
+constexpr int FWD_SMEM_INFER = FWD_SH2 + 128 * 64 * 2;
 
-template <bool TRAIN>
 __global__ void __launch_bounds__(128, 1) k_mlp_fwd(FwdIO io) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint64_t mbar;
     __shared__ uint32_t tmem_slot;
     __shared__ float sb[MLP_NUM_BIASES];
     __shared__ float sw4[64];
-    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const int t = threadIdx.x, warp = t >> 5;
     if (warp == 0) tmem_alloc(&tmem_slot, TMEM_COLS_FWD);
     if (t == 0) mbar_init(&mbar, 1);
     stage_weight(smem + FWD_SW1, io.w + W1_OFF, 64, 16);
@@ -182,11 +158,6 @@ __global__ void __launch_bounds__(128, 1) k_mlp_fwd(FwdIO io) {
                 pk[i] = (uint32_t)bf16_bits(xf[2 * i]) | ((uint32_t)bf16_bits(xf[2 * i + 1]) << 16);
             *reinterpret_cast<uint4*>(smem + FWD_SX + kmajor_offset(t, 0, 128)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
             *reinterpret_cast<uint4*>(smem + FWD_SX + kmajor_offset(t, 8, 128)) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-            if (TRAIN && valid) {
-                uint4* dst = reinterpret_cast<uint4*>(io.x16 + (size_t)row * 16);
-                dst[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                dst[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-            }
         }
         // ---- layer 1: TMEM cols [0, 64)
         sync_for_mma();
@@ -200,24 +171,14 @@ __global__ void __launch_bounds__(128, 1) k_mlp_fwd(FwdIO io) {
             float v[16];
             tmem_ld16(lane_base + 16 * c, v);
             tmem_wait_ld();
-            float g[16];
 #pragma unroll
             for (int i = 0; i < 16; i += 2) {
                 const float2 z = vadd(make_float2(v[i], v[i + 1]), make_float2(sb[B1_OFF + 16 * c + i], sb[B1_OFF + 16 * c + i + 1]));
-                g[i] = TRAIN ? gelu_grad(z.x) : 0.0f;
-                g[i + 1] = TRAIN ? gelu_grad(z.y) : 0.0f;
                 const float2 hh = gelu2(z);
                 v[i] = hh.x;
                 v[i + 1] = hh.y;
             }
             put_row64(smem + FWD_SH1, t, v, 16 * c);
-            if (TRAIN && valid) {
-#pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    io.h1[(size_t)row * 64 + 16 * c + i] = bf16_bits(v[i]);
-                    io.g1[(size_t)row * 64 + 16 * c + i] = bf16_bits(g[i]);
-                }
-            }
         }
         // ---- layer 2: TMEM cols [64, 128)
         sync_for_mma();
@@ -231,24 +192,14 @@ __global__ void __launch_bounds__(128, 1) k_mlp_fwd(FwdIO io) {
             float v[16];
             tmem_ld16(lane_base + 64 + 16 * c, v);
             tmem_wait_ld();
-            float g[16];
 #pragma unroll
             for (int i = 0; i < 16; i += 2) {
                 const float2 z = vadd(make_float2(v[i], v[i + 1]), make_float2(sb[B2_OFF + 16 * c + i], sb[B2_OFF + 16 * c + i + 1]));
-                g[i] = TRAIN ? gelu_grad(z.x) : 0.0f;
-                g[i + 1] = TRAIN ? gelu_grad(z.y) : 0.0f;
                 const float2 hh = gelu2(z);
                 v[i] = hh.x;
                 v[i + 1] = hh.y;
             }
             put_row64(smem + FWD_SH2, t, v, 16 * c);
-            if (TRAIN && valid) {
-#pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    io.h2[(size_t)row * 64 + 16 * c + i] = bf16_bits(v[i]);
-                    io.g2[(size_t)row * 64 + 16 * c + i] = bf16_bits(g[i]);
-                }
-            }
         }
         // ---- layer 3: TMEM cols [0, 64) again (layer 1's values were consumed
         // before layer 2 was issued), then the output layer on CUDA cores
@@ -259,7 +210,6 @@ __global__ void __launch_bounds__(128, 1) k_mlp_fwd(FwdIO io) {
         }
         if (!wait_mma(&mbar, phase, io.err, io.wait_limit)) { alive = false; break; }
         float y = sb[B4_OFF];
-        float* h3f = reinterpret_cast<float*>(smem + FWD_SH3F) + t * 64;
 #pragma unroll 1
         for (int c = 0; c < 4; ++c) {
             float v[16];
@@ -274,59 +224,21 @@ __global__ void __launch_bounds__(128, 1) k_mlp_fwd(FwdIO io) {
                 hs[i + 1] = hh.y;
             }
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const float z = v[i] + sb[B3_OFF + 16 * c + i];
-                const float h = hs[i];
-                y = __fmaf_rn(h, sw4[16 * c + i], y);
-                if (TRAIN) {
-                    h3f[16 * c + i] = h;
-                    // the derivative is stored in dz3 for now and scaled once dy is known
-                    if (valid) io.dz3[(size_t)row * 64 + 16 * c + i] = bf16_bits(gelu_grad(z));
-                }
-            }
+            for (int i = 0; i < 16; ++i) y = __fmaf_rn(hs[i], sw4[16 * c + i], y);
         }
-        if (!TRAIN) {
-            if (valid) {
-                float lam0 = y * sb[OSCALE_OFF];
-                if (io.q && io.clamp > 0.0f) {
-                    // trust region around the plain lambda of the same pass (q.w):
-                    // same sign, at most clamp times its magnitude
-                    const float lp = reinterpret_cast<const float*>(io.q)[4 * (size_t)row + 3];
-                    const float a = io.clamp * lp;
-                    const float f0 = io.floor ? lp : 0.0f;  // the weak end of the interval
-                    lam0 = fminf(fmaxf(lam0, fminf(a, f0)), fmaxf(a, f0));
-                }
-                if (io.out) io.out[row] = lam0;
-                if (io.q) reinterpret_cast<float*>(io.q)[4 * (size_t)row + 3] = lam0;
-                if (io.lam_acc) io.lam_acc[row] = lam0;
+        if (valid) {
+            float lam0 = y * sb[OSCALE_OFF];
+            if (io.q && io.clamp > 0.0f) {
+                // trust region around the plain lambda of the same pass (q.w):
+                // same sign, at most clamp times its magnitude
+                const float lp = reinterpret_cast<const float*>(io.q)[4 * (size_t)row + 3];
+                const float a = io.clamp * lp;
+                const float f0 = io.floor ? lp : 0.0f;  // the weak end of the interval
+                lam0 = fminf(fmaxf(lam0, fminf(a, f0)), fmaxf(a, f0));
             }
-        } else {
-            // loss = mean (y - target/scale)^2 ; dy = 2 (y - t) / B
-            const float r = valid ? (y - io.target[row] / sb[OSCALE_OFF]) : 0.0f;
-            const float dy = 2.0f * r * io.inv_batch;
-            float l = r * r * io.inv_batch, db = dy;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                l += __shfl_xor_sync(0xffffffffu, l, o);
-                db += __shfl_xor_sync(0xffffffffu, db, o);
-            }
-            // this warp's sums go to its own slot; k_sum_parts adds the slots in a
-            // fixed order, so the gradients do not depend on the blocks' timing
-            float* slot = io.part + ((size_t)tile * 4 + warp) * FWD_PART;
-            if (lane == 0) {
-                slot[0] = l;
-                slot[1] = db;
-            }
-            for (int nn = 0; nn < 64; ++nn) {
-                float gwn = dy * h3f[nn];
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) gwn += __shfl_xor_sync(0xffffffffu, gwn, o);
-                if (lane == 0) slot[2 + nn] = gwn;
-                if (valid) {
-                    const size_t at = (size_t)row * 64 + nn;
-                    io.dz3[at] = bf16_bits(dy * sw4[nn] * bf16_val(io.dz3[at]));
-                }
-            }
+            if (io.out) io.out[row] = lam0;
+            if (io.q) reinterpret_cast<float*>(io.q)[4 * (size_t)row + 3] = lam0;
+            if (io.lam_acc) io.lam_acc[row] = lam0;
         }
     }
     fence_before_sync();
@@ -335,130 +247,343 @@ __global__ void __launch_bounds__(128, 1) k_mlp_fwd(FwdIO io) {
 }
 
 // ---------------------------------------------------------------------------
-// Backward through one hidden layer (Kin inputs, 64 outputs) for 128-row tiles:
-//   dW[64 x Kin] += dZ^T H   and db += column sums of dZ  (one MMA: a ones row is
-//                                                           appended to H^T)
-//   dH = dZ W, dZ_prev = dH * gelu'(Z_prev)                 (second MMA, if any)
+// Training: one kernel evaluates a 128-row tile forward and backward with every
+// activation kept in shared memory (the network's state of a tile is 200 KB), and
+// one sums the tiles' gradients in a fixed order and applies Adam.
+//
+// Forward as in inference, keeping H1, H2 (BF16, both as the next product's
+// K-major A tile and transposed) and gelu' of each layer (BF16, registers).
+// Backward through a hidden layer with Kin inputs:
+//   dW[64 x Kin] = dZ^T H and db = column sums of dZ  (one MMA: a ones row is
+//                                                      appended to H^T)
+//   dH = dZ W, dZ_prev = dH * gelu'(Z_prev)           (second MMA, if any)
+// A tile is a chain of six tensor-core round trips with an epilogue each, so its
+// latency is what counts: 512 threads share each epilogue, 16 columns of one row
+// per thread (warp w reads TMEM lanes 32 (w & 3) and columns 16 (w >> 2), so one
+// tcgen05.ld per thread and product). Batch 4,096: 204 us per step with a kernel
+// per layer and direction (activations stored 2 bytes at a time, one launch per
+// gradient sum), see the measured time at k_mlp_reduce.
 // ---------------------------------------------------------------------------
-struct BwdIO {
-    const uint16_t* dz;     // [n][64]
-    const uint16_t* h;      // [n][Kin] layer input (bf16)
-    const uint16_t* w;      // W [64][Kin]
-    const uint16_t* gprev;  // [n][Kin] gelu' of the layer input, null for the first layer
-    uint16_t* dz_prev;      // [n][Kin] out, null for the first layer
-    float* part;            // per tile: dW [64][Kin] then db [64] (summed by k_sum_parts)
+// Programmatic dependent launch: let the next kernel of the stream start its
+// prologue; wait until the kernels before are complete and their writes visible.
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+struct TrainIO {
+    const uint16_t* w;    // bf16 weights
+    const float* b;       // biases and constants
+    const float* feat;    // raw features [n][12]
+    const float* target;  // [n]
+    float* part;          // per tile: PART_TILE floats
     int n;
+    float inv_batch;
     int* err;
 };
+// gradient partials of a tile: dW3 | db3, dW2 | db2, dW1 | db1, then per warp of
+// rows loss, db4, dw4[64]
+constexpr int PART_L3 = 0, PART_L2 = PART_L3 + 64 * 64 + 64, PART_L1 = PART_L2 + 64 * 64 + 64;
+constexpr int PART_OUT = PART_L1 + 64 * 16 + 64, PART_WARP = 66, PART_TILE = PART_OUT + 4 * PART_WARP;
 
-template <int KIN>
-__global__ void __launch_bounds__(128, 1) k_mlp_bwd(BwdIO io) {
-    constexpr int NB = KIN + 16;  // H^T rows plus the ones row (padded to a multiple of 16)
-    // TMEM: dW | db in columns [0, NB), dH in [128, 128 + KIN). The first layer
-    // (KIN = 16) has no dH and needs 128 columns; its smaller footprint lets 3
-    // CTAs share an SM, and 3 x 128 columns stay within the SM's 512.
-    constexpr uint32_t TCOLS = KIN == 16 ? 128 : 256;
+constexpr int TR_THREADS = 512;
+constexpr int TR_W1 = 0;                           // [64 x 16]
+constexpr int TR_W2 = TR_W1 + 64 * 16 * 2;         // [64 x 64]
+constexpr int TR_W3 = TR_W2 + 64 * 64 * 2;
+constexpr int TR_W2T = TR_W3 + 64 * 64 * 2;        // W^T, B of dH
+constexpr int TR_W3T = TR_W2T + 64 * 64 * 2;
+constexpr int TR_X = TR_W3T + 64 * 64 * 2;         // [128 x 16]
+constexpr int TR_XT = TR_X + 128 * 16 * 2;         // [32 x 128]: X^T, the ones row, zeros
+constexpr int TR_H1 = TR_XT + 32 * 128 * 2;        // [128 x 64]
+constexpr int TR_H1T = TR_H1 + 128 * 64 * 2;       // [80 x 128]
+constexpr int TR_H2 = TR_H1T + 80 * 128 * 2;
+constexpr int TR_H2T = TR_H2 + 128 * 64 * 2;
+constexpr int TR_DZ = TR_H2T + 80 * 128 * 2;       // [128 x 64]
+constexpr int TR_DZT = TR_DZ + 128 * 64 * 2;       // [128 x 128], rows 64.. zero
+constexpr int TR_H3F = TR_DZT + 128 * 128 * 2;     // [128][65] fp32
+constexpr int TR_SMEM = TR_H3F + 128 * 65 * 4;
+
+// 16 BF16 values of columns c0.. of row `row` into a K-major [128 x 64] tile
+__device__ __forceinline__ void put_bits16(uint8_t* s, int row, int c0, const uint16_t (&h)[16]) {
+    uint32_t pk[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) pk[i] = (uint32_t)h[2 * i] | ((uint32_t)h[2 * i + 1] << 16);
+    *reinterpret_cast<uint4*>(s + kmajor_offset(row, c0, 128)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+    *reinterpret_cast<uint4*>(s + kmajor_offset(row, c0 + 8, 128)) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+}
+// the same values into column `row` of the transposed tile of R rows
+__device__ __forceinline__ void put_bits16_t(uint8_t* s, int R, int row, int c0, const uint16_t (&h)[16]) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) *reinterpret_cast<uint16_t*>(s + kmajor_offset(c0 + i, row, R)) = h[i];
+}
+
+__global__ void __launch_bounds__(TR_THREADS, 1) k_mlp_train(TrainIO io) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint8_t* sDZ = smem;                       // [128 x 64]  A of dH = dZ W
-    uint8_t* sDZT = sDZ + 128 * 64 * 2;        // [128 x 128] A of dW (rows 64.. zero)
-    uint8_t* sHT = sDZT + 128 * 128 * 2;       // [NB x 128]  B of dW
-    uint8_t* sWT = sHT + NB * 128 * 2;         // [KIN x 64]  B of dH
     __shared__ uint64_t mbar;
     __shared__ uint32_t tmem_slot;
-    const int t = threadIdx.x, warp = t >> 5;
-    const bool with_dh = io.dz_prev != nullptr && TCOLS >= 128 + KIN;
-    if (warp == 0) tmem_alloc(&tmem_slot, TCOLS);
+    __shared__ float sb[MLP_NUM_BIASES];
+    __shared__ float sw4[64];
+    __shared__ float s_dy[128];
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const int m = 32 * (warp & 3) + lane;  // this thread's row of the tile
+    const int cq = warp >> 2, c0 = 16 * cq;  // and its 16 columns
+    if (warp == 0) tmem_alloc(&tmem_slot, 256);
     if (t == 0) mbar_init(&mbar, 1);
-    if (with_dh) stage_weight_t(sWT, io.w, KIN);
-    // rows 64..127 of dZ^T stay zero
-    for (int i = t; i < 64 * 128 / 8; i += 128) {
-        const int r = 64 + i / 16, j = i % 16;
-        *reinterpret_cast<uint4*>(sDZT + kmajor_offset(r, 8 * j, 128)) = make_uint4(0, 0, 0, 0);
+    // what stays zero: rows 64.. of dZ^T, the rows after the ones rows
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    for (int i = t; i < 64 * 16; i += TR_THREADS)
+        *reinterpret_cast<uint4*>(smem + TR_DZT + kmajor_offset(64 + i / 16, 8 * (i % 16), 128)) = zero;
+    for (int i = t; i < 16 * 16; i += TR_THREADS) {
+        *reinterpret_cast<uint4*>(smem + TR_H1T + kmajor_offset(64 + i / 16, 8 * (i % 16), 80)) = zero;
+        *reinterpret_cast<uint4*>(smem + TR_H2T + kmajor_offset(64 + i / 16, 8 * (i % 16), 80)) = zero;
+        *reinterpret_cast<uint4*>(smem + TR_XT + kmajor_offset(16 + i / 16, 8 * (i % 16), 32)) = zero;
     }
+    // everything above overlaps the end of the kernel before (the reduction that
+    // wrote these weights); nothing below does
+    pdl_launch();
+    pdl_wait();
+    stage_weight(smem + TR_W1, io.w + W1_OFF, 64, 16);
+    stage_weight(smem + TR_W2, io.w + W2_OFF, 64, 64);
+    stage_weight(smem + TR_W3, io.w + W3_OFF, 64, 64);
+    stage_weight_t(smem + TR_W2T, io.w + W2_OFF, 64);
+    stage_weight_t(smem + TR_W3T, io.w + W3_OFF, 64);
+    for (int i = t; i < MLP_NUM_BIASES; i += TR_THREADS) sb[i] = io.b[i];
+    if (t < 64) sw4[t] = bf16_val(io.w[W4_OFF + t]);
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
     const uint32_t tbase = tmem_slot;
-    const uint32_t lane_base = tmem_addr(tbase, 32 * warp, 0);
+    const uint32_t lane_base = tmem_addr(tbase, 32 * (warp & 3), c0);
+    float* h3f = reinterpret_cast<float*>(smem + TR_H3F);
     uint32_t phase = 0;
-    const int ntiles = (io.n + TILE - 1) / TILE;
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int m = t;
-        const int row = tile * TILE + m;
-        const bool valid = row < io.n;
-        // dZ row m -> sDZ row m and column m of sDZT
-        for (int j = 0; j < 8; ++j) {
-            uint4 v = make_uint4(0, 0, 0, 0);
-            if (valid) v = *reinterpret_cast<const uint4*>(io.dz + (size_t)row * 64 + 8 * j);
-            *reinterpret_cast<uint4*>(sDZ + kmajor_offset(m, 8 * j, 128)) = v;
-            const uint16_t* e = reinterpret_cast<const uint16_t*>(&v);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) *reinterpret_cast<uint16_t*>(sDZT + kmajor_offset(8 * j + i, m, 128)) = e[i];
-        }
-        // H row m -> column m of sHT, then the ones row and zero padding
-        for (int k = 0; k < KIN; ++k)
-            *reinterpret_cast<uint16_t*>(sHT + kmajor_offset(k, m, NB)) = valid ? io.h[(size_t)row * KIN + k] : 0;
-        for (int k = KIN; k < NB; ++k)
-            *reinterpret_cast<uint16_t*>(sHT + kmajor_offset(k, m, NB)) = (k == KIN && valid) ? 0x3F80 : 0;
+    bool alive = true;
+    // one product (two with a second B) and the wait for it; false: the wait expired
+    auto product = [&](int a, int bt, int N, int K, int a2, int b2) {
         sync_for_mma();
         if (t == 0) {
-            gemm_issue(tbase, sDZT, sHT, NB, 128, 0);  // dW | db in TMEM cols [0, NB)
-            if (with_dh) gemm_issue(tbase + 128, sDZ, sWT, KIN, 64, 0);  // dH in cols [128, 128 + KIN)
+            gemm_issue(tbase, smem + a, smem + bt, N, K, 0);
+            if (a2 >= 0) gemm_issue(tbase + 128, smem + a2, smem + b2, 64, 64, 0);
             commit(&mbar);
         }
-        if (!wait_mma(&mbar, phase, io.err)) break;
-        if (warp < 2) {  // rows 0..63 of the dW product: output unit m, into this tile's slot
-            float* slot = io.part + (size_t)tile * (64 * KIN + 64);
-#pragma unroll 1
-            for (int c = 0; c < NB / 16; ++c) {
-                float v[16];
-                tmem_ld16(lane_base + 16 * c, v);
-                tmem_wait_ld();
+        return wait_mma(&mbar, phase, io.err);
+    };
+    const int ntiles = (io.n + TILE - 1) / TILE;
+    for (int tile = blockIdx.x; tile < ntiles && alive; tile += gridDim.x) {
+        const int row = tile * TILE + m;
+        const bool valid = row < io.n;
+        float* part = io.part + (size_t)tile * PART_TILE;
+        // normalised features -> BF16, four per thread
+        {
+            uint16_t xb[4];
 #pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    const int k = 16 * c + i;
-                    if (k < KIN) slot[m * KIN + k] = v[i];
-                    else if (k == KIN) slot[64 * KIN + m] = v[i];
-                }
+            for (int i = 0; i < 4; ++i) {
+                const int k = 4 * cq + i;
+                const float xf = valid && k < MLP_IN
+                                     ? (io.feat[(size_t)row * MLP_IN + k] - sb[FMEAN_OFF + k]) * sb[FISTD_OFF + k]
+                                     : 0.0f;
+                xb[i] = bf16_bits(xf);
+                *reinterpret_cast<uint16_t*>(smem + TR_XT + kmajor_offset(k, m, 32)) = xb[i];
+            }
+            *reinterpret_cast<uint2*>(smem + TR_X + kmajor_offset(m, 4 * cq, 128)) =
+                make_uint2((uint32_t)xb[0] | ((uint32_t)xb[1] << 16), (uint32_t)xb[2] | ((uint32_t)xb[3] << 16));
+            if (cq == 0) {
+                const uint16_t one = valid ? 0x3F80 : 0;  // the ones row: db comes out of the dW product
+                *reinterpret_cast<uint16_t*>(smem + TR_XT + kmajor_offset(16, m, 32)) = one;
+                *reinterpret_cast<uint16_t*>(smem + TR_H1T + kmajor_offset(64, m, 80)) = one;
+                *reinterpret_cast<uint16_t*>(smem + TR_H2T + kmajor_offset(64, m, 80)) = one;
             }
         }
-        if (with_dh) {
-#pragma unroll 1
-            for (int c = 0; c < KIN / 16; ++c) {
-                float v[16];
-                tmem_ld16(lane_base + 128 + 16 * c, v);
-                tmem_wait_ld();
-                if (valid) {
+        const float tgt = t < TILE && valid ? io.target[row] : 0.0f;
+        uint16_t g1[16], g2[16], g3[16];
+        // ---- hidden layers 1 and 2
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        const size_t at = (size_t)row * KIN + 16 * c + i;
-                        io.dz_prev[at] = bf16_bits(v[i] * bf16_val(io.gprev[at]));
-                    }
+        for (int l = 0; l < 2; ++l) {
+            alive = l == 0 ? product(TR_X, TR_W1, 64, 16, -1, -1) : product(TR_H1, TR_W2, 64, 64, -1, -1);
+            if (!alive) break;
+            const float* bias = sb + (l == 0 ? B1_OFF : B2_OFF) + c0;
+            uint16_t(&g)[16] = l == 0 ? g1 : g2;
+            float v[16];
+            tmem_ld16(lane_base, v);
+            tmem_wait_ld();
+            uint16_t h[16];
+#pragma unroll
+            for (int i = 0; i < 16; i += 2) {
+                const float2 z = vadd(make_float2(v[i], v[i + 1]), make_float2(bias[i], bias[i + 1]));
+                g[i] = bf16_bits(gelu_grad(z.x));
+                g[i + 1] = bf16_bits(gelu_grad(z.y));
+                const float2 hh = gelu2(z);
+                h[i] = bf16_bits(hh.x);
+                h[i + 1] = bf16_bits(hh.y);
+            }
+            put_bits16(smem + (l == 0 ? TR_H1 : TR_H2), m, c0, h);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) h[i] = valid ? h[i] : 0;
+            put_bits16_t(smem + (l == 0 ? TR_H1T : TR_H2T), 80, m, c0, h);
+        }
+        if (!alive) break;
+        // ---- layer 3, kept in FP32
+        alive = product(TR_H2, TR_W3, 64, 64, -1, -1);
+        if (!alive) break;
+        {
+            float v[16];
+            tmem_ld16(lane_base, v);
+            tmem_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 16; i += 2) {
+                const float2 hh = gelu2(vadd(make_float2(v[i], v[i + 1]),
+                                             make_float2(sb[B3_OFF + c0 + i], sb[B3_OFF + c0 + i + 1])));
+                h3f[m * 65 + c0 + i] = hh.x;
+                h3f[m * 65 + c0 + i + 1] = hh.y;
+            }
+#pragma unroll
+            for (int i = 0; i < 16; ++i) g3[i] = bf16_bits(gelu_grad(v[i] + sb[B3_OFF + c0 + i]));
+        }
+        __syncthreads();
+        // ---- output layer: loss = mean (y - target/scale)^2 ; dy = 2 (y - t) / B
+        if (t < TILE) {  // thread t is row t here: warps 0 .. 3 have m = t
+            float y = sb[B4_OFF];
+#pragma unroll 16
+            for (int i = 0; i < 64; ++i) y = __fmaf_rn(h3f[t * 65 + i], sw4[i], y);
+            const float r = valid ? (y - tgt / sb[OSCALE_OFF]) : 0.0f;
+            const float dy = 2.0f * r * io.inv_batch;
+            s_dy[t] = dy;
+            float l = r * r * io.inv_batch, db = dy;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                l += __shfl_xor_sync(0xffffffffu, l, o);
+                db += __shfl_xor_sync(0xffffffffu, db, o);
+            }
+            // this warp's sums go to its own slot; the slots are added in a fixed
+            // order, so the gradients do not depend on the blocks' timing
+            if (lane == 0) {
+                part[PART_OUT + warp * PART_WARP] = l;
+                part[PART_OUT + warp * PART_WARP + 1] = db;
+            }
+        }
+        __syncthreads();
+        {
+            uint16_t dz[16];
+            const float dy = s_dy[m];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) dz[i] = valid ? bf16_bits(dy * sw4[c0 + i] * bf16_val(g3[i])) : 0;
+            put_bits16(smem + TR_DZ, m, c0, dz);
+            put_bits16_t(smem + TR_DZT, 128, m, c0, dz);
+        }
+        if (t >= 256) {  // dw4: column nn of 32 rows, added as a butterfly over 32 lanes would
+            const int wr = (t - 256) >> 6, nn = t & 63;
+            float a[32];
+#pragma unroll
+            for (int i = 0; i < 32; ++i) a[i] = s_dy[32 * wr + i] * h3f[(32 * wr + i) * 65 + nn];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int i = 0; i < o; ++i) a[i] = a[i] + a[i + o];
+            part[PART_OUT + wr * PART_WARP + 2 + nn] = a[0];
+        }
+        // ---- backward through layers 3, 2 and 1
+#pragma unroll
+        for (int l = 3; l >= 1; --l) {
+            alive = l == 3   ? product(TR_DZT, TR_H2T, 80, 128, TR_DZ, TR_W3T)
+                    : l == 2 ? product(TR_DZT, TR_H1T, 80, 128, TR_DZ, TR_W2T)
+                             : product(TR_DZT, TR_XT, 32, 128, -1, -1);
+            if (!alive) break;
+            const int kin = l == 1 ? 16 : 64;
+            float* dst = part + (l == 3 ? PART_L3 : l == 2 ? PART_L2 : PART_L1);
+            if ((warp & 3) < 2) {  // rows 0 .. 63 of the dW product: output unit m
+                if (c0 < kin) {
+                    float v[16];
+                    tmem_ld16(lane_base, v);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int i = 0; i < 16; i += 4)
+                        *reinterpret_cast<float4*>(dst + m * kin + c0 + i) =
+                            make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
                 }
+                if (cq == 1) {  // the column of the ones row
+                    float v[16];
+                    tmem_ld16(tmem_addr(tbase, 32 * (warp & 3), kin), v);
+                    tmem_wait_ld();
+                    dst[64 * kin + m] = v[0];
+                }
+            }
+            if (l > 1) {
+                const uint16_t(&g)[16] = l == 3 ? g2 : g1;
+                float v[16];
+                tmem_ld16(lane_base + 128, v);
+                tmem_wait_ld();
+                uint16_t dz[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) dz[i] = valid ? bf16_bits(v[i] * bf16_val(g[i])) : 0;
+                put_bits16(smem + TR_DZ, m, c0, dz);
+                put_bits16_t(smem + TR_DZT, 128, m, c0, dz);
             }
         }
     }
     fence_before_sync();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tbase, TCOLS);
+    if (warp == 0) tmem_dealloc(tbase, 256);
 }
 
-// ---------------------------------------------------------------------------
-// Adam on the FP32 master parameters; refreshes the BF16 weights
-// ---------------------------------------------------------------------------
-__global__ void k_adam(float* p, float* m, float* v, const float* g, int n, float lr, float b1, float b2, float eps,
-                       float c1, float c2, uint16_t* p16) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.0f - b1) * gi;
-    const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    const float upd = lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-    const float pi = p[i] - upd;
-    p[i] = pi;
-    if (p16) p16[i] = bf16_bits(pi);
+struct AdamIO {
+    float *pw, *pb, *mw, *mb, *vw, *vb;  // parameters and moments of weights and biases
+    uint16_t* w16;
+    float lr, b1, b2, eps, c1, c2;
+};
+
+// Gradients of all parameters (one thread each) and the loss: the tiles' partials
+// in tile order, p = 0, 1, ... (deterministic: the same bits on every run), and
+// with ADAM the parameter's Adam step on the FP32 masters, refreshing the BF16
+// weights. Bound by the latency of its loads, so they are issued 32 at a time.
+constexpr int REDUCE_UNROLL = 32;
+template <bool ADAM>
+__global__ void __launch_bounds__(64) k_mlp_reduce(const float* __restrict__ part, int tiles, float* __restrict__ gw,
+                                                   float* __restrict__ gb, float* __restrict__ loss, AdamIO a) {
+    const int i = blockIdx.x * 64 + threadIdx.x;
+    const int j = i - MLP_NUM_WEIGHTS;  // >= 0: bias j, then the loss
+    if (j > MLP_NUM_TRAINED_BIASES) return;
+    // where the parameter lies in a slot; output-layer slots are one per warp of rows
+    int at;
+    bool out = false;
+    if (j < 0) {
+        if (i < W2_OFF) at = PART_L1 + (i - W1_OFF);
+        else if (i < W3_OFF) at = PART_L2 + (i - W2_OFF);
+        else if (i < W4_OFF) at = PART_L3 + (i - W3_OFF);
+        else { at = PART_OUT + 2 + (i - W4_OFF); out = true; }
+    } else if (j < B2_OFF) at = PART_L1 + 64 * 16 + (j - B1_OFF);
+    else if (j < B3_OFF) at = PART_L2 + 64 * 64 + (j - B2_OFF);
+    else if (j < B4_OFF) at = PART_L3 + 64 * 64 + (j - B3_OFF);
+    else { at = PART_OUT + (j == B4_OFF ? 1 : 0); out = true; }
+    pdl_wait();  // the partials of the training kernel before this one
+    float s = 0.0f;
+    const int slots = out ? 4 * tiles : tiles;
+    for (int q0 = 0; q0 < slots; q0 += REDUCE_UNROLL) {
+        float v[REDUCE_UNROLL];
+#pragma unroll
+        for (int u = 0; u < REDUCE_UNROLL; ++u) {
+            const int q = q0 + u;
+            const size_t o = out ? (size_t)(q >> 2) * PART_TILE + (q & 3) * PART_WARP : (size_t)q * PART_TILE;
+            v[u] = q < slots ? part[o + at] : 0.0f;
+        }
+#pragma unroll
+        for (int u = 0; u < REDUCE_UNROLL; ++u)
+            if (q0 + u < slots) s += v[u];
+    }
+    if (j == MLP_NUM_TRAINED_BIASES) {
+        *loss = s;
+        return;
+    }
+    if (j < 0) gw[i] = s;
+    else gb[j] = s;
+    if (ADAM) {
+        const int k = j < 0 ? i : j;
+        float *p = j < 0 ? a.pw : a.pb, *mo = j < 0 ? a.mw : a.mb, *ve = j < 0 ? a.vw : a.vb;
+        const float mi = a.b1 * mo[k] + (1.0f - a.b1) * s;
+        const float vi = a.b2 * ve[k] + (1.0f - a.b2) * s * s;
+        mo[k] = mi;
+        ve[k] = vi;
+        const float upd = a.lr * (mi / a.c1) / (sqrtf(vi / a.c2) + a.eps);
+        const float pi = p[k] - upd;
+        p[k] = pi;
+        if (j < 0) a.w16[k] = bf16_bits(pi);
+    }
 }
 
 __global__ void k_to_bf16(const float* p, uint16_t* q, int n) {
@@ -485,7 +610,7 @@ int mlp_infer(const uint16_t* w_bf16, const float* b, const float* feat, int n, 
     if (n <= 0) return 0;
     static bool attr = false;
     if (!attr) {
-        if (cudaFuncSetAttribute(k_mlp_fwd<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, FWD_SMEM_INFER) !=
+        if (cudaFuncSetAttribute(k_mlp_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, FWD_SMEM_INFER) !=
             cudaSuccess)
             return -1;
         attr = true;
@@ -505,14 +630,14 @@ int mlp_infer(const uint16_t* w_bf16, const float* b, const float* feat, int n, 
     // one another's tensor-core waits
     const int tiles = (n + TILE - 1) / TILE;
     const int grid = tiles < 4 * sm_count() ? tiles : 4 * sm_count();
-    k_mlp_fwd<false><<<grid, 128, FWD_SMEM_INFER, st>>>(io);
+    k_mlp_fwd<<<grid, 128, FWD_SMEM_INFER, st>>>(io);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
 int mlp_infer_uncommitted(const uint16_t* w_bf16, const float* b, const float* feat, int n, float* out,
                           long long wait_limit, int* err, cudaStream_t st) {
     if (n <= 0) return 0;
-    if (cudaFuncSetAttribute(k_mlp_fwd<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, FWD_SMEM_INFER) !=
+    if (cudaFuncSetAttribute(k_mlp_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, FWD_SMEM_INFER) !=
         cudaSuccess)
         return -1;
     FwdIO io{};
@@ -525,7 +650,7 @@ int mlp_infer_uncommitted(const uint16_t* w_bf16, const float* b, const float* f
     io.no_commit = 1;
     io.wait_limit = wait_limit;
     const int tiles = (n + TILE - 1) / TILE;
-    k_mlp_fwd<false><<<tiles, 128, FWD_SMEM_INFER, st>>>(io);
+    k_mlp_fwd<<<tiles, 128, FWD_SMEM_INFER, st>>>(io);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -533,10 +658,9 @@ struct MlpTrainer {
     int cap = 0;
     float *w32 = nullptr, *b32 = nullptr, *mw = nullptr, *vw = nullptr, *mb = nullptr, *vb = nullptr;
     float *gw = nullptr, *gb = nullptr, *loss = nullptr;
-    float* part = nullptr;  // gradient partials per tile (and warp), summed in a fixed order
+    float* part = nullptr;  // gradient partials per tile, summed in a fixed order
     int* err = nullptr;
-    uint16_t *w16 = nullptr, *x16 = nullptr, *h1 = nullptr, *h2 = nullptr, *g1 = nullptr, *g2 = nullptr,
-             *dz3 = nullptr, *dz2 = nullptr, *dz1 = nullptr;
+    uint16_t* w16 = nullptr;
     int step = 0;
 };
 
@@ -559,17 +683,8 @@ MlpTrainer* mlp_trainer_create(int max_batch, const float* w32, const float* b32
     A((void**)&t->loss, sizeof(float));
     A((void**)&t->err, sizeof(int));
     A((void**)&t->w16, sizeof(uint16_t) * MLP_NUM_WEIGHTS);
-    const size_t cap = (size_t)max_batch;
-    A((void**)&t->x16, sizeof(uint16_t) * cap * 16);
-    A((void**)&t->h1, sizeof(uint16_t) * cap * 64);
-    A((void**)&t->h2, sizeof(uint16_t) * cap * 64);
-    A((void**)&t->g1, sizeof(uint16_t) * cap * 64);
-    A((void**)&t->g2, sizeof(uint16_t) * cap * 64);
-    A((void**)&t->dz3, sizeof(uint16_t) * cap * 64);
-    A((void**)&t->dz2, sizeof(uint16_t) * cap * 64);
-    A((void**)&t->dz1, sizeof(uint16_t) * cap * 64);
-    const size_t tiles = (cap + TILE - 1) / TILE;
-    A((void**)&t->part, sizeof(float) * tiles * std::max<size_t>(64 * 64 + 64, 4 * FWD_PART));
+    const size_t tiles = ((size_t)max_batch + TILE - 1) / TILE;
+    A((void**)&t->part, sizeof(float) * tiles * PART_TILE);
     if (!ok) {
         mlp_trainer_destroy(t);
         return nullptr;
@@ -587,76 +702,57 @@ MlpTrainer* mlp_trainer_create(int max_batch, const float* w32, const float* b32
 void mlp_trainer_destroy(MlpTrainer* t) {
     if (!t) return;
     void* ps[] = {t->w32, t->b32, t->mw, t->vw, t->mb, t->vb, t->gw, t->gb, t->loss, t->err, t->w16,
-                  t->x16, t->h1, t->h2, t->g1, t->g2, t->dz3, t->dz2, t->dz1, t->part};
+                  t->part};
     for (void* p : ps)
         if (p) cudaFree(p);
     delete t;
 }
 
-int mlp_gradients(MlpTrainer* t, const float* feat, const float* target, int B, cudaStream_t st) {
-    if (B <= 0 || B > t->cap) return -1;
-    static bool attr = false;
-    if (!attr) {
-        if (cudaFuncSetAttribute(k_mlp_fwd<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, FWD_SMEM_TRAIN) !=
-                cudaSuccess ||
-            cudaFuncSetAttribute(k_mlp_bwd<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 128 * 64 * 2 + 128 * 128 * 2 + 80 * 128 * 2 + 64 * 64 * 2) != cudaSuccess ||
-            cudaFuncSetAttribute(k_mlp_bwd<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 128 * 64 * 2 + 128 * 128 * 2 + 32 * 128 * 2 + 16 * 64 * 2) != cudaSuccess)
-            return -1;
-        attr = true;
-    }
-    cudaMemsetAsync(t->gw, 0, sizeof(float) * MLP_NUM_WEIGHTS, st);
-    cudaMemsetAsync(t->gb, 0, sizeof(float) * MLP_NUM_BIASES, st);
-    cudaMemsetAsync(t->loss, 0, sizeof(float), st);
-    const int tiles = (B + TILE - 1) / TILE;
-    const int grid = tiles < sm_count() ? tiles : sm_count();
-    FwdIO f{};
-    f.w = t->w16;
-    f.b = t->b32;
-    f.feat = feat;
-    f.n = B;
-    f.target = target;
-    f.inv_batch = 1.0f / (float)B;
-    f.x16 = t->x16;
-    f.h1 = t->h1;
-    f.h2 = t->h2;
-    f.g1 = t->g1;
-    f.g2 = t->g2;
-    f.dz3 = t->dz3;
-    f.part = t->part;
-    f.err = t->err;
-    k_mlp_fwd<true><<<grid, 128, FWD_SMEM_TRAIN, st>>>(f);
-    // the output layer's sums: loss, db4, dw4 (each its own sum over the slots)
-    k_sum_parts<<<1, 64, 0, st>>>(t->part, tiles * 4, FWD_PART, 1, t->loss);
-    k_sum_parts<<<1, 64, 0, st>>>(t->part + 1, tiles * 4, FWD_PART, 1, t->gb + B4_OFF);
-    k_sum_parts<<<1, 64, 0, st>>>(t->part + 2, tiles * 4, FWD_PART, 64, t->gw + W4_OFF);
-    // hidden layers: dW then db of each, from its per-tile slots
-    auto layer_sums = [&](int kin, float* gw, float* gb) {
-        const int stride = 64 * kin + 64;
-        k_sum_parts<<<(64 * kin + 255) / 256, 256, 0, st>>>(t->part, tiles, stride, 64 * kin, gw);
-        k_sum_parts<<<1, 64, 0, st>>>(t->part + 64 * kin, tiles, stride, 64, gb);
-    };
-    BwdIO b3{t->dz3, t->h2, t->w16 + W3_OFF, t->g2, t->dz2, t->part, B, t->err};
-    k_mlp_bwd<64><<<grid, 128, 128 * 64 * 2 + 128 * 128 * 2 + 80 * 128 * 2 + 64 * 64 * 2, st>>>(b3);
-    layer_sums(64, t->gw + W3_OFF, t->gb + B3_OFF);
-    BwdIO b2{t->dz2, t->h1, t->w16 + W2_OFF, t->g1, t->dz1, t->part, B, t->err};
-    k_mlp_bwd<64><<<grid, 128, 128 * 64 * 2 + 128 * 128 * 2 + 80 * 128 * 2 + 64 * 64 * 2, st>>>(b2);
-    layer_sums(64, t->gw + W2_OFF, t->gb + B2_OFF);
-    BwdIO b1{t->dz1, t->x16, t->w16 + W1_OFF, nullptr, nullptr, t->part, B, t->err};
-    k_mlp_bwd<16><<<grid, 128, 128 * 64 * 2 + 128 * 128 * 2 + 32 * 128 * 2 + 16 * 64 * 2, st>>>(b1);
-    layer_sums(16, t->gw + W1_OFF, t->gb + B1_OFF);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+// Launch with programmatic stream serialisation (the kernel calls pdl_wait before
+// it reads what the kernels before it wrote).
+template <typename... P, typename... A>
+static int launch_pdl(void (*k)(P...), int grid, int block, int smem, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, k, P(args)...) == cudaSuccess ? 0 : -1;
 }
 
-int mlp_adam(MlpTrainer* t, float lr, float beta1, float beta2, float eps, cudaStream_t st) {
+// The tiles' gradient partials of a batch; the caller sums them.
+static int launch_train(MlpTrainer* t, const float* feat, const float* target, int B, cudaStream_t st) {
+    if (B <= 0 || B > t->cap) return -1;
+    // (per call: the attribute belongs to the current device)
+    if (cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, TR_SMEM) != cudaSuccess)
+        return -1;
+    const int tiles = (B + TILE - 1) / TILE;
+    const int grid = tiles < sm_count() ? tiles : sm_count();
+    const TrainIO io{t->w16, t->b32, feat, target, t->part, B, 1.0f / (float)B, t->err};
+    return launch_pdl(k_mlp_train, grid, TR_THREADS, TR_SMEM, st, io);
+}
+
+constexpr int REDUCE_BLOCKS = (MLP_NUM_WEIGHTS + MLP_NUM_TRAINED_BIASES + 1 + 63) / 64;
+
+int mlp_gradients(MlpTrainer* t, const float* feat, const float* target, int B, cudaStream_t st) {
+    if (launch_train(t, feat, target, B, st)) return -1;
+    return launch_pdl(k_mlp_reduce<false>, REDUCE_BLOCKS, 64, 0, st, t->part, (B + TILE - 1) / TILE, t->gw, t->gb,
+                      t->loss, AdamIO{});
+}
+
+int mlp_train_step(MlpTrainer* t, const float* feat, const float* target, int B, float lr, float beta1, float beta2,
+                   float eps, cudaStream_t st) {
+    if (launch_train(t, feat, target, B, st)) return -1;
     t->step += 1;
-    const float c1 = 1.0f - powf(beta1, (float)t->step), c2 = 1.0f - powf(beta2, (float)t->step);
-    k_adam<<<(MLP_NUM_WEIGHTS + 255) / 256, 256, 0, st>>>(t->w32, t->mw, t->vw, t->gw, MLP_NUM_WEIGHTS, lr, beta1,
-                                                           beta2, eps, c1, c2, t->w16);
-    k_adam<<<1, 256, 0, st>>>(t->b32, t->mb, t->vb, t->gb, MLP_NUM_TRAINED_BIASES, lr, beta1, beta2, eps, c1, c2,
-                              nullptr);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    const AdamIO a{t->w32, t->b32, t->mw, t->mb, t->vw, t->vb, t->w16, lr, beta1, beta2, eps,
+                   1.0f - powf(beta1, (float)t->step), 1.0f - powf(beta2, (float)t->step)};
+    return launch_pdl(k_mlp_reduce<true>, REDUCE_BLOCKS, 64, 0, st, t->part, (B + TILE - 1) / TILE, t->gw, t->gb,
+                      t->loss, a);
 }
 
 int mlp_read(MlpTrainer* t, float* w32, float* b32, float* gw, float* gb, float* loss, int* err) {

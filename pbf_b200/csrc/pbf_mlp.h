@@ -53,10 +53,11 @@ struct MlpTrainer;
 MlpTrainer* mlp_trainer_create(int max_batch, const float* w32, const float* b32);
 void mlp_trainer_destroy(MlpTrainer* t);
 // Gradients of the mean squared error of (network output) vs target / output
-// scale over a batch; accumulates into the trainer's gradient buffers (cleared first).
+// scale over a batch, into the trainer's gradient buffers.
 int mlp_gradients(MlpTrainer* t, const float* feat, const float* target, int B, cudaStream_t st);
-// One Adam step with the current gradients.
-int mlp_adam(MlpTrainer* t, float lr, float beta1, float beta2, float eps, cudaStream_t st);
+// The same gradients and one Adam step with them.
+int mlp_train_step(MlpTrainer* t, const float* feat, const float* target, int B, float lr, float beta1, float beta2,
+                   float eps, cudaStream_t st);
 int mlp_read(MlpTrainer* t, float* w32, float* b32, float* gw, float* gb, float* loss, int* err);
 const uint16_t* mlp_weights_bf16(MlpTrainer* t);
 const float* mlp_biases(MlpTrainer* t);
