@@ -80,6 +80,9 @@ struct DevStats {
     long long total_iters;  // adaptive: corrections applied since upload
 };
 
+// The cell counts follow the stats in one allocation, so an upload clears both at once.
+constexpr size_t kStatsBytes = (sizeof(DevStats) + 255) / 256 * 256;
+
 // Profiling stages (pbf_stage_times)
 enum Stage { ST_HASH, ST_SCAN, ST_SCATTER, ST_REORDER, ST_NEIGHBORS, ST_LAMBDA, ST_DP, ST_VELOCITY, ST_CURL,
              ST_VORT, ST_COPY, ST_MEASURE, ST_MLP, ST_COUNT };
@@ -223,6 +226,24 @@ cudaError_t staging_malloc(void** p, size_t bytes) {
     return cudaMalloc(p, bytes);
 }
 
+// The calling thread's mapped host word (null when it cannot be had); freed when
+// the thread ends. The caller synchronises before it returns, so one per thread
+// is enough for any number of streams.
+int* scan_error_word() {
+    struct Word {
+        int* p = nullptr;
+        ~Word() {
+            if (p) cudaFreeHost(p);
+        }
+    };
+    thread_local Word w;
+    if (!w.p && cudaHostAlloc((void**)&w.p, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        w.p = nullptr;
+    }
+    return w.p;
+}
+
 // Frees whatever part of a HostPipe exists (null members are skipped).
 void free_host_pipe(HostPipe* hp) {
     if (!hp) return;
@@ -247,7 +268,7 @@ template <typename T> int dalloc(T** p, size_t count) {
 void free_all(pbf_solver* s) {
     void* ptrs[] = {s->Sx, s->Sv, s->Px, s->Pv, s->Pxold, s->Q, s->omega, s->vw, s->xpred_dbg, s->dp_dbg, s->vort_dbg,
                     s->visc_dbg, s->rho_dbg, s->Sperm, s->Pperm, s->cell, s->ticket, s->tmp, s->cell_sorted,
-                    s->ncnt, s->nbr, s->cnt, s->cell_start, s->hash_dbg, s->lam_acc, s->lam_prev_sorted, s->lam0,
+                    s->ncnt, s->nbr, s->cell_start, s->hash_dbg, s->lam_acc, s->lam_prev_sorted, s->lam0,
                     s->feat, s->scan_ws, s->dstats, s->staging, s->scenes_d, s->sid, s->mlp_w, s->mlp_b};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -415,7 +436,11 @@ int enqueue_substep(pbf_solver* s, cudaStream_t st) {
     // and counts -- was done by the previous substep's vorticity pass, or by the
     // upload or grid build that set the state)
     if (dbg) cudaMemcpyAsync(s->hash_dbg, s->cell, sizeof(int) * n, cudaMemcpyDeviceToDevice, st);
-    P(ST_SCAN, [&] { launch_scan(s->cnt, s->cell_start, s->nkeys, s->scan_ws, err, st); });
+    // (the scan also clears the per-substep slots of the stats; the error bits stay)
+    P(ST_SCAN, [&] {
+        launch_scan(s->cnt, s->cell_start, s->nkeys, s->scan_ws, (int*)ds, (int)(offsetof(DevStats, err) / sizeof(int)),
+                    err, st);
+    });
     P(ST_SCATTER, [&] { launch_scatter(n, s->cell, s->ticket, s->cell_start, s->tmp, err, st); });
     // the substep's total lambda is tracked when features are computed (warm
     // start, or recording features for training)
@@ -429,7 +454,6 @@ int enqueue_substep(pbf_solver* s, cudaStream_t st) {
     if (dbg) launch_copy4(n, s->Px, s->xpred_dbg, st);
     P(ST_NEIGHBORS, [&] { launch_neighbors(kp, s->Px, s->cell_start, s->nbr, s->ncnt, st); });
 
-    cudaMemsetAsync(ds, 0, offsetof(DevStats, err), st);  // per-substep slots; keeps the error bits
     const int iters = s->para.iterations;
     float* acc = feats ? s->lam_acc : nullptr;
     // First correction with features: the feature pass computes the plain lambda
@@ -704,12 +728,16 @@ int create_common(const pbf_solver_parameter* para, int nscenes, const pbf_scene
     AL(s->Sperm, n); AL(s->Pperm, n); AL(s->cell, n); AL(s->ticket, n); AL(s->tmp, n); AL(s->cell_sorted, n);
     AL(s->ncnt, n);
     AL(s->nbr, (size_t)ext->max_neighbors * s->stride);
-    AL(s->cnt, (size_t)s->nkeys);
     AL(s->cell_start, (size_t)s->nkeys + 1);
     AL(s->lam_acc, n); AL(s->lam_prev_sorted, n); AL(s->lam0, n);
     AL(s->feat, n * (size_t)MLP_IN);
     AL(s->staging, 6 * n);
-    AL(s->dstats, 1);
+    {
+        char* both = nullptr;
+        AL(both, kStatsBytes + sizeof(int) * (size_t)s->nkeys);
+        s->dstats = reinterpret_cast<DevStats*>(both);
+        s->cnt = reinterpret_cast<int*>(both + kStatsBytes);
+    }
     if (dbg) {
         AL(s->xpred_dbg, n); AL(s->dp_dbg, n); AL(s->vort_dbg, n); AL(s->visc_dbg, n); AL(s->rho_dbg, n);
         AL(s->hash_dbg, n);
@@ -719,8 +747,9 @@ int create_common(const pbf_solver_parameter* para, int nscenes, const pbf_scene
         AL(s->sid, n);
     }
     {
-        const size_t ws = scan_status_bytes(s->nkeys);
+        const size_t ws = scan_keep_bytes(s->nkeys);
         cudaError_t e = cudaMalloc(&s->scan_ws, ws);
+        if (e == cudaSuccess) e = cudaMemset(s->scan_ws, 0, ws);  // once: the scan leaves it ready
         if (e != cudaSuccess) {
             free_all(s);
             delete s;
@@ -780,14 +809,10 @@ int pbf_upload_device(pbf_solver* s, const float* d_pos, const float* d_vel, int
     if (!s || !d_pos || !d_vel) return fail(PBF_ERR_INVALID, "null argument");
     if (n != s->n) return fail(PBF_ERR_INVALID, "n (%d) differs from nParticles (%d)", n, s->n);
     cudaStream_t st = (cudaStream_t)stream;
-    CK(cudaMemsetAsync(s->dstats, 0, sizeof(DevStats), st));
-    launch_from_aos(n, d_pos, d_vel, s->Sx, s->Sv, s->Sperm, &s->dstats->err, st);
-    CK(cudaGetLastError());
-    CK(cudaMemsetAsync(s->lam_acc, 0, sizeof(float) * n, st));
-    // the first substep's grid hash (later substeps get theirs from the
-    // vorticity pass before them)
-    CK(cudaMemsetAsync(s->cnt, 0, sizeof(int) * (size_t)s->nkeys, st));
-    launch_hash(s->kp, true, s->Sx, s->Sv, s->cell, s->ticket, s->cnt, &s->dstats->err, st);
+    // the stats and, right after them, the cell counts
+    CK(cudaMemsetAsync(s->dstats, 0, kStatsBytes + sizeof(int) * (size_t)s->nkeys, st));
+    launch_upload(s->kp, d_pos, d_vel, s->Sx, s->Sv, s->Sperm, s->lam_acc, s->cell, s->ticket, s->cnt, &s->dstats->err,
+                  st);
     CK(cudaGetLastError());
     s->last_stream = st;
     s->uploaded = true;
@@ -829,7 +854,7 @@ int pbf_step(pbf_solver* s, int substeps, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     for (int i = 0; i < substeps; ++i) CK(cudaGraphLaunch(s->exec, st));
     if (s->bound_pos && substeps > 0) {
-        launch_to_aos(s->n, s->Sx, s->Sperm, s->bound_pos, &s->dstats->err, st);
+        launch_to_aos(s->n, s->Sx, nullptr, s->Sperm, s->bound_pos, nullptr, &s->dstats->err, st);
         CK(cudaGetLastError());
     }
     s->last_stream = st;
@@ -1014,7 +1039,7 @@ int pbf_build_grid(pbf_solver* s, void* stream) {
     CK(cudaMemsetAsync(s->cnt, 0, sizeof(int) * (size_t)s->nkeys, st));  // drop the next substep's counts
     launch_hash(kp, false, s->Sx, s->Sv, s->cell, s->ticket, s->cnt, err, st);
     if (s->hash_dbg) CK(cudaMemcpyAsync(s->hash_dbg, s->cell, sizeof(int) * s->n, cudaMemcpyDeviceToDevice, st));
-    launch_scan(s->cnt, s->cell_start, s->nkeys, s->scan_ws, err, st);
+    launch_scan(s->cnt, s->cell_start, s->nkeys, s->scan_ws, nullptr, 0, err, st);
     launch_scatter(s->n, s->cell, s->ticket, s->cell_start, s->tmp, err, st);
     launch_reorder(kp, false, s->Sx, s->Sv, s->Sperm, s->cell, s->cell_start, s->tmp, s->Px, s->Pv, s->Pxold, s->Pperm,
                    s->cell_sorted, nullptr, nullptr, err, st);
@@ -1036,8 +1061,8 @@ int pbf_download_device(pbf_solver* s, float* d_pos, float* d_vel, void* stream)
     if (!s) return fail(PBF_ERR_INVALID, "null handle");
     if (!s->uploaded) return fail(PBF_ERR_STATE, "pbf_download before pbf_upload");
     cudaStream_t st = (cudaStream_t)stream;
-    if (d_pos) launch_to_aos(s->n, s->Sx, s->Sperm, d_pos, &s->dstats->err, st);
-    if (d_vel) launch_to_aos(s->n, s->Sv, s->Sperm, d_vel, &s->dstats->err, st);
+    if (d_pos) launch_to_aos(s->n, s->Sx, s->Sv, s->Sperm, d_pos, d_vel, &s->dstats->err, st);
+    else if (d_vel) launch_to_aos(s->n, s->Sv, nullptr, s->Sperm, d_vel, nullptr, &s->dstats->err, st);
     CK(cudaGetLastError());
     s->last_stream = st;
     return PBF_OK;
@@ -1329,12 +1354,15 @@ int pbf_scan_exclusive_i32(const int* d_in, int* d_out, int n, void* d_ws, size_
     if (ws_bytes < pbf_scan_workspace_bytes(n)) return fail(PBF_ERR_INVALID, "workspace too small");
     cudaStream_t st = (cudaStream_t)stream;
     int* err = (int*)((char*)d_ws + scan_status_bytes(n));
-    CK(cudaMemsetAsync(err, 0, sizeof(int), st));
-    launch_scan_const(d_in, d_out, n, d_ws, err, st);
+    // An expired wait is reported through a mapped host word of this thread, read
+    // after the synchronisation, instead of a copy of the device word.
+    int* word = scan_error_word();
+    if (!word) return fail(PBF_ERR_ALLOC, "host allocation failed");
+    *word = 0;
+    launch_scan_const(d_in, d_out, n, d_ws, scan_status_bytes(n) + sizeof(int), err, word, st);
     CK(cudaGetLastError());
-    int herr = 0;
-    CK(cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    const int herr = *(volatile int*)word;
     if (herr) return fail(PBF_ERR_DEVICE, "scan error bits 0x%x", herr);
     return PBF_OK;
 }

@@ -78,17 +78,32 @@ __global__ void __launch_bounds__(256, 8) k_hash(KParams p, const float4* __rest
 // ---------------------------------------------------------------------------
 // a3 + a4: exclusive scan of the cell counts with decoupled look-back; writes
 // cell_start[0..m) and cell_start[m] = total, and clears the counts for the next
-// substep. Status words: (flag << 32) | value, flag 1 = tile aggregate,
-// 2 = inclusive prefix. Tiles are numbered in launch order by an atomic ticket,
-// so every predecessor is already running and the wait always ends; the wait is
-// bounded anyway and reports DEVERR_SCAN_TIMEOUT.
+// substep. Status words: (epoch << 34) | (flag << 32) | value, flag 1 = tile
+// aggregate, 2 = inclusive prefix. Tiles are numbered in launch order by an atomic
+// ticket, so every predecessor is already running and the wait always ends; the
+// wait is bounded anyway and reports DEVERR_SCAN_TIMEOUT.
+//
+// The workspace is the status words, then the ticket counter and the epoch. With
+// KEEP (the solver's own workspace, zeroed once) the last ticket's block resets
+// the counter and advances the epoch, which invalidates this run's words, so a
+// substep needs no memset; other callers' workspaces are cleared before the launch.
+// KEEP also writes the cleared counts only where there were any: most cells of a
+// large grid are empty, and the pass is bound by its bytes (65.6 M keys, 4.7 M
+// particles: 194 us -> 144 us with 524 MB instead of 786).
 // ---------------------------------------------------------------------------
-constexpr int SCAN_THREADS = 256;
 constexpr long long SCAN_SPIN_LIMIT = 1ll << 22;
-// Counts per thread: 32 (tiles of 8,192), or 64 (tiles of 16,384) above 2^22
-// counts, where half as many tiles shorten the look-back chains.
+// Tiles of 8,192 counts, or of 16,384 above 2^22 counts, where half as many tiles
+// shorten the look-back chains (65.6 M keys, mostly empty: 144 us against 173 with
+// 8,192 and 234 with 4,096). The solver's own scan takes 4,096 up to 2^19 counts,
+// where 8,192 leave most SMs idle (25,000 keys: 4.3 against 4.7 us; 1.02 M keys:
+// 8.8 against 7.4). A look-back window of the whole block instead of a warp was
+// slower at every size (two barriers per window and more polls: 1.02 M keys 10.4
+// against 8.8 us at 4,096, 65.6 M keys 302 against 234).
+constexpr int SCAN_THREADS = 256;
+constexpr int SCAN_SMALL_MAX = 1 << 19;
 constexpr int SCAN_LARGE_MIN = (1 << 22) + 1;
-__host__ __device__ constexpr int scan_items(int m) { return m >= SCAN_LARGE_MIN ? 64 : 32; }
+static int scan_tile(int m) { return m >= SCAN_LARGE_MIN ? 16384 : 8192; }
+constexpr unsigned SCAN_EPOCHS = 1u << 30;
 
 __device__ __forceinline__ void st_release_u64(unsigned long long* a, unsigned long long v) {
     asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(a), "l"(v) : "memory");
@@ -100,32 +115,49 @@ __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long
 }
 
 // VEC: cnt and out are 16-byte aligned; each lane moves four consecutive counts
-// per access (int4), four rounds of 128 per warp instead of sixteen of 32.
+// per access (int4), rounds of 128 per warp instead of 32.
 // silent_tile >= 0 (the failure-injection test only): that tile publishes no
 // status, so its successors' look-back waits run out after spin_limit polls.
-template <bool VEC, int SCAN_ITEMS>
+template <bool VEC, bool KEEP, int ITEMS>
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan(int* __restrict__ cnt, int* __restrict__ out, int m,
-                                                       unsigned long long* __restrict__ status,
-                                                       int* __restrict__ tile_counter, int* __restrict__ err,
-                                                       int clear, int silent_tile, long long spin_limit) {
-    constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
+                                                       unsigned long long* __restrict__ status, int tiles,
+                                                       int* __restrict__ err, int* host_err, int silent_tile,
+                                                       long long spin_limit, int* __restrict__ zero, int nzero) {
+    constexpr int TILE = SCAN_THREADS * ITEMS, WARPS = SCAN_THREADS / 32;
     __shared__ int s_tile;
-    __shared__ int s_warp[SCAN_THREADS / 32];
-    __shared__ int s_excl, s_tot;
+    __shared__ unsigned s_epoch;
+    __shared__ int s_warp[WARPS];
+    __shared__ int s_excl;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    if (t == 0) s_tile = atomicAdd(tile_counter, 1);
+    if (t == 0) {
+        int* counter = reinterpret_cast<int*>(status + tiles);
+        unsigned* epoch = reinterpret_cast<unsigned*>(counter + 1);
+        const unsigned e = KEEP ? *reinterpret_cast<volatile unsigned*>(epoch) : 0u;
+        __threadfence();  // the epoch is read before the ticket that lets it advance
+        const int tile = atomicAdd(counter, 1);
+        if (KEEP && tile == tiles - 1) {  // every block has its ticket and its epoch
+            *counter = 0;
+            *epoch = (e + 1) % SCAN_EPOCHS;
+        }
+        s_tile = tile;
+        s_epoch = e;
+    }
     __syncthreads();
     const int tile = s_tile;
+    if (KEEP && tile == 0)  // words of the caller to be cleared along the way
+        for (int i = t; i < nzero; i += SCAN_THREADS) zero[i] = 0;
+    const unsigned long long ep = (unsigned long long)s_epoch << 34;
 
     // Warp w owns elements [tile * TILE + w * 32 ITEMS, + 32 ITEMS) in rounds of consecutive
     // elements (coalesced: 32 counts per round, or 128 as int4 when VEC); each
     // round is scanned across the warp and carried into the next.
-    const long long wbase = (long long)tile * SCAN_TILE + (long long)warp * (32 * SCAN_ITEMS);
-    int item[SCAN_ITEMS];
+    const long long wbase = (long long)tile * TILE + (long long)warp * (32 * ITEMS);
+    int item[ITEMS];
     int carry = 0;  // warp-exclusive offset of the round
+    unsigned filled = 0u;  // rounds (int4 groups) of this lane that hold a count
     if (VEC) {
 #pragma unroll
-        for (int r = 0; r < SCAN_ITEMS / 4; ++r) {
+        for (int r = 0; r < ITEMS / 4; ++r) {
             const long long i0 = wbase + r * 128 + lane * 4;
             if (i0 + 3 < m) {
                 const int4 q = *reinterpret_cast<const int4*>(cnt + i0);
@@ -136,9 +168,10 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan(int* __restrict__ cnt, in
             }
         }
 #pragma unroll
-        for (int r = 0; r < SCAN_ITEMS / 4; ++r) {
+        for (int r = 0; r < ITEMS / 4; ++r) {
             const int a0 = item[4 * r], a1 = a0 + item[4 * r + 1], a2 = a1 + item[4 * r + 2];
             const int tot = a2 + item[4 * r + 3];
+            if (KEEP) filled |= tot != 0 ? 1u << r : 0u;
             int incl = tot;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -154,12 +187,12 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan(int* __restrict__ cnt, in
         }
     } else {
 #pragma unroll
-        for (int q = 0; q < SCAN_ITEMS; ++q) {
+        for (int q = 0; q < ITEMS; ++q) {
             const long long idx = wbase + q * 32 + lane;
             item[q] = idx < m ? cnt[idx] : 0;
         }
 #pragma unroll
-        for (int q = 0; q < SCAN_ITEMS; ++q) {
+        for (int q = 0; q < ITEMS; ++q) {
             int incl = item[q];
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -173,94 +206,85 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan(int* __restrict__ cnt, in
     }
     if (lane == 0) s_warp[warp] = carry;  // the warp's total
     __syncthreads();
+    // every thread: the sum of the warps before its own, and of all
+    int before = 0, total = 0;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) {
+        const int v = s_warp[w];
+        before += w < warp ? v : 0;
+        total += v;
+    }
+    // decoupled look-back by one warp, 32 predecessors per window
+    const bool publish = tile != silent_tile;
+    if (t == 0 && publish)
+        st_release_u64(&status[tile], ep | ((tile == 0 ? 2ull : 1ull) << 32) | (unsigned)total);
     if (warp == 0) {
-        int w = lane < SCAN_THREADS / 32 ? s_warp[lane] : 0;
-        int wi = w;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, wi, o);
-            if (lane >= o) wi += y;
-        }
-        if (lane < SCAN_THREADS / 32) s_warp[lane] = wi - w;  // exclusive warp offsets
-        const int total = __shfl_sync(0xffffffffu, wi, SCAN_THREADS / 32 - 1);
-        // decoupled look-back
         int excl = 0;
-        const bool publish = tile != silent_tile;
-        if (tile == 0) {
-            if (lane == 0 && publish) st_release_u64(&status[0], (2ull << 32) | (unsigned)total);
-        } else {
-            if (lane == 0 && publish) st_release_u64(&status[tile], (1ull << 32) | (unsigned)total);
-            int pos = tile - 1;  // highest tile not yet folded in
-            bool done = false;
-            while (!done) {
-                const int look = pos - lane;
-                unsigned long long s = 0;
-                if (look >= 0) {
-                    long long spins = 0;
-                    s = ld_acquire_u64(&status[look]);
-                    while ((s >> 32) == 0ull) {
-                        if (++spins > spin_limit) {
-                            atomicOr(err, DEVERR_SCAN_TIMEOUT);
-                            s = 2ull << 32;  // give up: treat as prefix 0 so the tile finishes
-                            break;
-                        }
-                        __nanosleep(64);
-                        s = ld_acquire_u64(&status[look]);
+        bool done = tile == 0;
+        for (int pos = tile - 1; !done; pos -= 32) {
+            const int look = pos - lane;
+            bool prefix = true;  // before tile 0: an empty prefix
+            int val = 0;
+            if (look >= 0) {
+                long long spins = 0;
+                unsigned long long s = ld_acquire_u64(&status[look]);
+                while ((s & ~0x3ffffffffull) != ep || ((s >> 32) & 3ull) == 0ull) {
+                    if (++spins > spin_limit) {
+                        atomicOr(err, DEVERR_SCAN_TIMEOUT);
+                        if (host_err) *(volatile int*)host_err = DEVERR_SCAN_TIMEOUT;
+                        s = 2ull << 32;  // give up: treat as prefix 0 so the tile finishes
+                        break;
                     }
-                } else {
-                    s = 2ull << 32;  // before tile 0: an empty prefix
+                    __nanosleep(32);
+                    s = ld_acquire_u64(&status[look]);
                 }
-                const unsigned flag = (unsigned)(s >> 32);
-                const int val = (int)(unsigned)(s & 0xffffffffu);
-                const unsigned prefix_mask = __ballot_sync(0xffffffffu, flag == 2u);
-                const int stop = prefix_mask ? __ffs(prefix_mask) - 1 : 31;
-                int contrib = lane <= stop ? val : 0;
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) contrib += __shfl_xor_sync(0xffffffffu, contrib, o);
-                excl += contrib;
-                if (prefix_mask) done = true;
-                else pos -= 32;
+                prefix = ((s >> 32) & 3ull) == 2ull;
+                val = (int)(unsigned)(s & 0xffffffffull);
             }
-            if (lane == 0 && publish) st_release_u64(&status[tile], (2ull << 32) | (unsigned)(excl + total));
+            const unsigned pm = __ballot_sync(0xffffffffu, prefix);
+            const int stop = pm ? __ffs(pm) - 1 : 31;
+            int contrib = lane <= stop ? val : 0;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) contrib += __shfl_xor_sync(0xffffffffu, contrib, o);
+            excl += contrib;
+            done = pm != 0u;
         }
-        if (lane == 0) {
-            s_excl = excl;
-            s_tot = total;
-        }
+        if (lane == 0) s_excl = excl;
     }
     __syncthreads();
-    const int off = s_excl + s_warp[warp];
+    const int excl = s_excl;
+    if (t == 0 && publish && tile > 0)
+        st_release_u64(&status[tile], ep | (2ull << 32) | (unsigned)(excl + total));
+    const int off = excl + before;
     if (VEC) {
 #pragma unroll
-        for (int r = 0; r < SCAN_ITEMS / 4; ++r) {
+        for (int r = 0; r < ITEMS / 4; ++r) {
             const long long i0 = wbase + r * 128 + lane * 4;
             if (i0 + 3 < m) {
                 *reinterpret_cast<int4*>(out + i0) =
                     make_int4(off + item[4 * r], off + item[4 * r + 1], off + item[4 * r + 2], off + item[4 * r + 3]);
-                if (clear) *reinterpret_cast<int4*>(cnt + i0) = make_int4(0, 0, 0, 0);
+                // (most cells of a large grid are empty: those need no write)
+                if (KEEP && (filled >> r & 1u)) *reinterpret_cast<int4*>(cnt + i0) = make_int4(0, 0, 0, 0);
             } else {
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
                     if (i0 + e < m) {
                         out[i0 + e] = off + item[4 * r + e];
-                        if (clear) cnt[i0 + e] = 0;
+                        if (KEEP) cnt[i0 + e] = 0;
                     }
             }
         }
     } else {
 #pragma unroll
-        for (int q = 0; q < SCAN_ITEMS; ++q) {
+        for (int q = 0; q < ITEMS; ++q) {
             const long long idx = wbase + q * 32 + lane;
             if (idx < m) {
                 out[idx] = off + item[q];
-                if (clear) cnt[idx] = 0;
+                if (KEEP) cnt[idx] = 0;
             }
         }
     }
-    if (tile == (int)(((long long)m - 1) / SCAN_TILE) && threadIdx.x == SCAN_THREADS - 1) {
-        // the last tile writes the grand total at out[m] (its inclusive prefix)
-        out[m] = s_excl + s_tot;
-    }
+    if (tile == tiles - 1 && t == 0) out[m] = excl + total;  // the grand total
 }
 
 // ---------------------------------------------------------------------------
@@ -564,17 +588,40 @@ __global__ void __launch_bounds__(256) k_density_error(KParams p, const float4* 
 // ---------------------------------------------------------------------------
 // layout kernels
 // ---------------------------------------------------------------------------
-__global__ void k_from_aos(int n, const float* __restrict__ pos, const float* __restrict__ vel, float4* __restrict__ x,
-                           float4* __restrict__ v, int* __restrict__ perm, int* __restrict__ err) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float px = pos[3 * i], py = pos[3 * i + 1], pz = pos[3 * i + 2];
-    const float vx = vel[3 * i], vy = vel[3 * i + 1], vz = vel[3 * i + 2];
-    if (!(isfinite(px) && isfinite(py) && isfinite(pz) && isfinite(vx) && isfinite(vy) && isfinite(vz)))
-        atomicOr(err, DEVERR_NONFINITE);
-    x[i] = make_float4(px, py, pz, 0.0f);
-    v[i] = make_float4(vx, vy, vz, 0.0f);
-    perm[i] = i;
+// Upload: AoS to the float4 state in particle order, the total lambda cleared, and
+// the first substep's grid hash (a1 + a2) of the state while it is in registers
+// (later substeps get theirs from the vorticity pass before them). One pass of 24 B
+// read and 48 B written per particle, instead of a conversion, a clear and a hash
+// that reads the state again (with the single clear before it and the one-pass
+// download, a frame of 4,080 particles and two substeps went from 252 to 234 us).
+__global__ void __launch_bounds__(256, 6) k_upload(KParams p, const float* __restrict__ pos,
+                                                   const float* __restrict__ vel, float4* __restrict__ x,
+                                                   float4* __restrict__ v, int* __restrict__ perm,
+                                                   float* __restrict__ lam_acc, int* __restrict__ cell,
+                                                   int* __restrict__ ticket, int* __restrict__ cnt,
+                                                   int* __restrict__ err) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    int key = -1;
+    if (i < p.n) {
+        f3 xi = {pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]};
+        f3 vi = {vel[3 * i], vel[3 * i + 1], vel[3 * i + 2]};
+        bool fine = isfinite(xi.x) && isfinite(xi.y) && isfinite(xi.z) && isfinite(vi.x) && isfinite(vi.y) &&
+                    isfinite(vi.z);
+        x[i] = make_float4(xi.x, xi.y, xi.z, 0.0f);
+        v[i] = make_float4(vi.x, vi.y, vi.z, 0.0f);
+        perm[i] = (int)i;
+        lam_acc[i] = 0.0f;
+        const SceneView sc = scene_of(p, (int)i);
+        predict(p, sc, xi, vi);
+        fine = fine && isfinite(xi.x) && isfinite(xi.y) && isfinite(xi.z);
+        if (!fine) atomicOr(err, DEVERR_NONFINITE);
+        key = cell_key(p, sc, xi);
+    }
+    const int tk = warp_histogram(key, cnt);
+    if (key >= 0) {
+        cell[i] = key;
+        ticket[i] = tk;
+    }
 }
 
 // The state in slot order: AoS x and v, the loaded index of each slot, the key
@@ -604,12 +651,14 @@ __global__ void k_sorted_state(int n, const float4* __restrict__ x, const float4
     if (rank) rank[k] = k - cell_start[c];
 }
 
-// slot order -> original order, AoS xyz
-__global__ void k_to_aos(int n, const float4* __restrict__ a, const int* __restrict__ perm, float* __restrict__ out,
-                         int* __restrict__ err) {
+// slot order -> original order, AoS xyz: a to out and, when both are given, a2 to
+// out2 in the same pass over perm
+__global__ void __launch_bounds__(256) k_to_aos(int n, const float4* __restrict__ a, const float4* __restrict__ a2,
+                                                const int* __restrict__ perm, float* __restrict__ out,
+                                                float* __restrict__ out2, int* __restrict__ err) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
-    const int o = perm[k];
+    const long long o = perm[k];
     if (o < 0 || o >= n) {
         atomicOr(err, DEVERR_BAD_INDEX);
         return;
@@ -618,6 +667,12 @@ __global__ void k_to_aos(int n, const float4* __restrict__ a, const int* __restr
     out[3 * o] = q.x;
     out[3 * o + 1] = q.y;
     out[3 * o + 2] = q.z;
+    if (out2) {
+        const float4 r = a2[k];
+        out2[3 * o] = r.x;
+        out2[3 * o + 1] = r.y;
+        out2[3 * o + 2] = r.z;
+    }
 }
 
 __global__ void k_copy4(int n, const float4* __restrict__ a, float4* __restrict__ b) {
@@ -719,48 +774,50 @@ void launch_hash(const KParams& p, bool predict_on, const float4* x, const float
 }
 
 // tile count in 64-bit arithmetic (m + tile - 1 would overflow an int near INT_MAX)
-static int scan_tiles(int m) {
-    const long long tile = (long long)SCAN_THREADS * scan_items(m);
-    return (int)(((long long)m + tile - 1) / tile);
-}
+static int tiles_of(int m, int tile) { return (int)(((long long)m + tile - 1) / tile); }
 
-size_t scan_status_bytes(int m) { return (size_t)scan_tiles(m) * sizeof(unsigned long long) + 16; }
+size_t scan_status_bytes(int m) { return (size_t)tiles_of(m, scan_tile(m)) * sizeof(unsigned long long) + 16; }
 
 template <bool VEC>
-static void launch_scan_kernel(int* cnt, int* out, int m, unsigned long long* status, int* counter, int* err,
-                               int clear, cudaStream_t st, int silent_tile = -1,
-                               long long spin_limit = SCAN_SPIN_LIMIT) {
-    const int tiles = scan_tiles(m);
-    if (scan_items(m) == 64)
-        k_scan<VEC, 64><<<tiles, SCAN_THREADS, 0, st>>>(cnt, out, m, status, counter, err, clear, silent_tile,
-                                                         spin_limit);
+static void launch_scan_cleared(int* cnt, int* out, int m, void* ws, int* err, int* host_err, cudaStream_t st,
+                                int silent_tile = -1, long long spin_limit = SCAN_SPIN_LIMIT) {
+    unsigned long long* status = (unsigned long long*)ws;
+    const int tiles = tiles_of(m, scan_tile(m));
+    if (scan_tile(m) == 16384)
+        k_scan<VEC, false, 64><<<tiles, SCAN_THREADS, 0, st>>>(cnt, out, m, status, tiles, err, host_err, silent_tile,
+                                                                spin_limit, nullptr, 0);
     else
-        k_scan<VEC, 32><<<tiles, SCAN_THREADS, 0, st>>>(cnt, out, m, status, counter, err, clear, silent_tile,
-                                                         spin_limit);
+        k_scan<VEC, false, 32><<<tiles, SCAN_THREADS, 0, st>>>(cnt, out, m, status, tiles, err, host_err, silent_tile,
+                                                                spin_limit, nullptr, 0);
 }
 
-void launch_scan(int* cnt, int* out, int m, void* status_ws, int* err, cudaStream_t st) {
-    unsigned long long* status = (unsigned long long*)status_ws;
-    int* counter = (int*)(status + scan_tiles(m));
-    cudaMemsetAsync(status_ws, 0, scan_status_bytes(m), st);
-    if (aligned16(cnt) && aligned16(out)) launch_scan_kernel<true>(cnt, out, m, status, counter, err, 1, st);
-    else launch_scan_kernel<false>(cnt, out, m, status, counter, err, 1, st);
+static int keep_tile(int m) { return m <= SCAN_SMALL_MAX ? 4096 : scan_tile(m); }
+size_t scan_keep_bytes(int m) { return (size_t)tiles_of(m, keep_tile(m)) * sizeof(unsigned long long) + 16; }
+
+void launch_scan(int* cnt, int* out, int m, void* ws, int* zero, int nzero, int* err, cudaStream_t st) {
+    unsigned long long* status = (unsigned long long*)ws;
+    const int tile = keep_tile(m), tiles = tiles_of(m, tile);
+    auto go = [&](auto kernel) {
+        kernel<<<tiles, SCAN_THREADS, 0, st>>>(cnt, out, m, status, tiles, err, nullptr, -1, SCAN_SPIN_LIMIT, zero, nzero);
+    };
+    if (tile == 4096) go(k_scan<true, true, 16>);
+    else if (tile == 8192) go(k_scan<true, true, 32>);
+    else go(k_scan<true, true, 64>);
 }
 
-void launch_scan_const(const int* in, int* out, int m, void* status_ws, int* err, cudaStream_t st) {
-    unsigned long long* status = (unsigned long long*)status_ws;
-    int* counter = (int*)(status + scan_tiles(m));
-    cudaMemsetAsync(status_ws, 0, scan_status_bytes(m), st);
-    if (aligned16(in) && aligned16(out)) launch_scan_kernel<true>(const_cast<int*>(in), out, m, status, counter, err, 0, st);
-    else launch_scan_kernel<false>(const_cast<int*>(in), out, m, status, counter, err, 0, st);
+void launch_scan_const(const int* in, int* out, int m, void* ws, size_t clear_bytes, int* err, int* host_err,
+                       cudaStream_t st) {
+    cudaMemsetAsync(ws, 0, clear_bytes, st);
+    if (aligned16(in) && aligned16(out))
+        launch_scan_cleared<true>(const_cast<int*>(in), out, m, ws, err, host_err, st);
+    else
+        launch_scan_cleared<false>(const_cast<int*>(in), out, m, ws, err, host_err, st);
 }
 
-void launch_scan_silent_tile(const int* in, int* out, int m, void* status_ws, int* err, int silent_tile,
+void launch_scan_silent_tile(const int* in, int* out, int m, void* ws, int* err, int silent_tile,
                              long long spin_limit, cudaStream_t st) {
-    unsigned long long* status = (unsigned long long*)status_ws;
-    int* counter = (int*)(status + scan_tiles(m));
-    cudaMemsetAsync(status_ws, 0, scan_status_bytes(m), st);
-    launch_scan_kernel<false>(const_cast<int*>(in), out, m, status, counter, err, 0, st, silent_tile, spin_limit);
+    cudaMemsetAsync(ws, 0, scan_status_bytes(m), st);
+    launch_scan_cleared<false>(const_cast<int*>(in), out, m, ws, err, nullptr, st, silent_tile, spin_limit);
 }
 
 void launch_scatter(int n, const int* cell, const int* ticket, const int* cell_start, int* tmp, int* err,
@@ -827,13 +884,14 @@ void launch_density_error(const KParams& p, const float4* x, const int* nbr, con
     k_density_error<<<blocks_for(p.n, 256), 256, 0, st>>>(p, x, nbr, ncnt, max_bits, sum, skip);
 }
 
-void launch_from_aos(int n, const float* pos, const float* vel, float4* x, float4* v, int* perm, int* err,
-                     cudaStream_t st) {
-    k_from_aos<<<blocks_for(n, 256), 256, 0, st>>>(n, pos, vel, x, v, perm, err);
+void launch_upload(const KParams& p, const float* pos, const float* vel, float4* x, float4* v, int* perm,
+                   float* lam_acc, int* cell, int* ticket, int* cnt, int* err, cudaStream_t st) {
+    k_upload<<<blocks_for(p.n, 256), 256, 0, st>>>(p, pos, vel, x, v, perm, lam_acc, cell, ticket, cnt, err);
 }
 
-void launch_to_aos(int n, const float4* a, const int* perm, float* out, int* err, cudaStream_t st) {
-    k_to_aos<<<blocks_for(n, 256), 256, 0, st>>>(n, a, perm, out, err);
+void launch_to_aos(int n, const float4* a, const float4* a2, const int* perm, float* out, float* out2, int* err,
+                   cudaStream_t st) {
+    k_to_aos<<<blocks_for(n, 256), 256, 0, st>>>(n, a, a2, perm, out, out2, err);
 }
 
 void launch_sorted_state(int n, const float4* x, const float4* v, const int* perm, const int* cell_sorted,

@@ -14,10 +14,17 @@ namespace pbf {
 
 void launch_hash(const KParams& p, bool predict_on, const float4* x, const float4* v, int* cell, int* ticket, int* cnt,
                  int* err, cudaStream_t st);
+// The solver's scan (16-byte aligned arrays; clears the counts): a workspace of
+// scan_keep_bytes(m), zeroed once, that the scan leaves ready for the next. Also
+// clears nzero words at zero, before anything after the scan can use them.
+size_t scan_keep_bytes(int m);
+void launch_scan(int* cnt, int* out, int m, void* ws, int* zero, int nzero, int* err, cudaStream_t st);
+// The same scan with the input left unchanged and any workspace of
+// scan_status_bytes(m); clear_bytes of it (at least those) are cleared first.
+// host_err (a mapped host word, or null) also receives an expired wait's bit.
 size_t scan_status_bytes(int m);
-void launch_scan(int* cnt, int* out, int m, void* status_ws, int* err, cudaStream_t st);
-// same scan, input left unchanged
-void launch_scan_const(const int* in, int* out, int m, void* status_ws, int* err, cudaStream_t st);
+void launch_scan_const(const int* in, int* out, int m, void* ws, size_t clear_bytes, int* err, int* host_err,
+                       cudaStream_t st);
 // failure injection (tests): tile silent_tile publishes no status and the
 // look-back gives up after spin_limit polls (input left unchanged)
 void launch_scan_silent_tile(const int* in, int* out, int m, void* status_ws, int* err, int silent_tile,
@@ -59,9 +66,13 @@ void launch_vort(const KParams& p, bool debug, const float4* x, const float4* vw
                  float4* visc, int* cell, int* ticket, int* hist, int* err, cudaStream_t st);
 void launch_density_error(const KParams& p, const float4* x, const int* nbr, const int* ncnt,
                           unsigned long long* max_bits, double* sum, const int* skip, cudaStream_t st);
-void launch_from_aos(int n, const float* pos, const float* vel, float4* x, float4* v, int* perm, int* err,
-                     cudaStream_t st);
-void launch_to_aos(int n, const float4* a, const int* perm, float* out, int* err, cudaStream_t st);
+// AoS positions and velocities to the state in particle order, lam_acc cleared,
+// and the first substep's grid hash (counts added to cnt, which is zero).
+void launch_upload(const KParams& p, const float* pos, const float* vel, float4* x, float4* v, int* perm,
+                   float* lam_acc, int* cell, int* ticket, int* cnt, int* err, cudaStream_t st);
+// Slot order to original order: a to out and (when out2 is not null) a2 to out2.
+void launch_to_aos(int n, const float4* a, const float4* a2, const int* perm, float* out, float* out2, int* err,
+                   cudaStream_t st);
 void launch_copy4(int n, const float4* a, float4* b, cudaStream_t st);
 void launch_sorted_state(int n, const float4* x, const float4* v, const int* perm, const int* cell_sorted,
                          const int* cell_start, float* pos, float* vel, int* ids, int* key, int* rank,

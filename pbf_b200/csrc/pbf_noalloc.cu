@@ -71,8 +71,9 @@ int pbf_scan_exclusive_i32_noalloc(const int* d_in, int* d_out, int n, void* str
     if (((status + 15) & ~(size_t)15) + sizeof(int) > (size_t)kScratchBytes)
         return fail(PBF_ERR_INVALID, "n needs more scan tiles than the allocation-free scratch holds");
     int* err = (int*)((char*)scratch + ((status + 15) & ~(size_t)15));
-    if (cudaMemsetAsync(err, 0, sizeof(int), st) != cudaSuccess) return fail(PBF_ERR_CUDA, "clearing the error word");
-    pbf::launch_scan_const(d_in, d_out, n, scratch, err, st);  // clears the status words, then scans
+    // clears the status words and the error word after them, then scans
+    pbf::launch_scan_const(d_in, d_out, n, scratch, (size_t)((char*)(err + 1) - (char*)scratch), err, nullptr,
+                           st);
     if (cudaGetLastError() != cudaSuccess) return fail(PBF_ERR_CUDA, "scan launch failed");
     int h = 0;
     if (cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
