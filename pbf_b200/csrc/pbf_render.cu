@@ -2,13 +2,13 @@
 // passes (src/renderapp.cpp:400-466) as CUDA kernels on device images.
 //
 //   pass                      reference shader             here
-//   sprite depth + depth test shaders/depth.vert, .frag    k_splat<false>: one thread per
-//                                                          particle, atomicMin on (depth, -z)
-//   curvature-flow smoothing  shaders/smooth.frag (x60)    k_smooth, ping-pong images
-//   additive thickness        shaders/thickness.frag       k_splat<true>: 64-bit fixed point
-//   normals from depth        shaders/normal.frag          k_normals
+//   sprite depth + depth test shaders/depth.vert, .frag    k_splat: one thread per particle,
+//   additive thickness        shaders/thickness.frag       atomicMin on (depth, -z), 64-bit
+//                                                          fixed-point atomicAdd
+//   curvature-flow smoothing  shaders/smooth.frag (x60)    k_smooth: SMOOTH_STEPS passes of a tile
 //   room (background)         shaders/background.frag      k_room: one ray per pixel
-//   fluid shading             shaders/shadingParticle.frag k_shade
+//   normals from depth        shaders/normal.frag          k_shade: normal and shading of
+//   fluid shading             shaders/shadingParticle.frag one pixel
 //
 // Images are width x height, row 0 at the bottom (the GL window convention);
 // texture reads use the texel the reference's NEAREST / REPEAT sampling picks.
@@ -60,11 +60,14 @@ __device__ __forceinline__ float dot3(float ax, float ay, float az, float bx, fl
     return (ax * bx + ay * by) + az * bz;
 }
 
-// Sprite depth (THICK false) or thickness (THICK true) of one particle per thread.
-template <bool THICK>
+// Sprite depth and thickness of one particle per thread (a warp per sprite with a
+// pixel per lane was slower: 69 against 57 us for 4.2 M fragments, its lanes idle on
+// small sprites). Most fragments lie behind what is already there, so a fragment
+// reads the pixel first, possibly a stale value, which is never below the current
+// one, and divides exactly and takes the atomic minimum only when an approximate
+// quotient, far closer than its margin, does not already place it behind.
 __global__ void __launch_bounds__(256) k_splat(Cam c, const float* __restrict__ pos, int n, int stride,
-                                               unsigned long long* __restrict__ depth,
-                                               unsigned long long* __restrict__ thick) {
+                                               unsigned long long* depth, unsigned long long* thick) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float* q = pos + (size_t)i * stride;
@@ -87,51 +90,63 @@ __global__ void __launch_bounds__(256) k_splat(Cam c, const float* __restrict__ 
     // pixels whose centres lie in [w - half, w + half)
     const int x0 = max((int)ceilf(wx - half - 0.5f), 0), x1 = min((int)ceilf(wx + half - 0.5f) - 1, c.w - 1);
     const int y0 = max((int)ceilf(wy - half - 0.5f), 0), y1 = min((int)ceilf(wy + half - 0.5f) - 1, c.h - 1);
-    for (int yy = y0; yy <= y1; ++yy)
+    for (int yy = y0; yy <= y1; ++yy) {
+        // gl_PointCoord (origin at the upper left), then
+        // vNormal.xy = vec2(2, -2) * gl_PointCoord + vec2(-1, 1)
+        const float t = 0.5f - ((float)yy + 0.5f - wy) / size;
+        const float ny = -2.0f * t + 1.0f;
         for (int xx = x0; xx <= x1; ++xx) {
-            // gl_PointCoord (origin at the upper left), then
-            // vNormal.xy = vec2(2, -2) * gl_PointCoord + vec2(-1, 1)
             const float s = ((float)xx + 0.5f - wx) / size + 0.5f;
-            const float t = 0.5f - ((float)yy + 0.5f - wy) / size;
-            const float nx = 2.0f * s + -1.0f, ny = -2.0f * t + 1.0f;
+            const float nx = 2.0f * s + -1.0f;
             const float d2 = nx * nx + ny * ny;
             if (d2 > 1.0f) continue;
-            const float nz = sqrtf(1.0f - d2);
             const size_t pix = (size_t)yy * c.w + xx;
-            if (THICK) {
-                // thickness = 2 * vNormal.z * radius, summed (GL_ONE, GL_ONE blending)
-                const float th = 2.0f * nz * c.radius;
-                atomicAdd(thick + pix, (unsigned long long)llrintf(th * kThickScale));
-            } else {
-                // surfacePos = viewPos.xyz + radius * vNormal; depth = -surfacePos.z
-                const float sx = vx + c.radius * nx, sy = vy + c.radius * ny, sz = vz + c.radius * nz;
-                const float qz = row4(c.P, 2, sx, sy, sz), qw = row4(c.P, 3, sx, sy, sz);
-                float fd = 0.5f * (qz / qw) + 0.5f;  // gl_FragDepth
-                fd = fminf(fmaxf(fd, 0.0f), 1.0f);
-                const unsigned long long key =
-                    ((unsigned long long)__float_as_uint(fd) << 32) | (unsigned long long)__float_as_uint(-sz);
-                atomicMin(depth + pix, key);
-            }
+            const unsigned long long cur = __ldca(depth + pix);
+            const float nz = sqrtf(1.0f - d2);
+            // thickness = 2 * vNormal.z * radius, summed (GL_ONE, GL_ONE blending)
+            const float th = 2.0f * nz * c.radius;
+            atomicAdd(thick + pix, (unsigned long long)llrintf(th * kThickScale));
+            // surfacePos = viewPos.xyz + radius * vNormal; depth = -surfacePos.z
+            const float sx = vx + c.radius * nx, sy = vy + c.radius * ny, sz = vz + c.radius * nz;
+            const float qz = row4(c.P, 2, sx, sy, sz), qw = row4(c.P, 3, sx, sy, sz);
+            // behind (an empty pixel's bits are a NaN, which compares false)
+            if (0.5f * __fdividef(qz, qw) + 0.5f > __uint_as_float((unsigned)(cur >> 32)) + 1e-5f) continue;
+            float fd = 0.5f * (qz / qw) + 0.5f;  // gl_FragDepth
+            fd = fminf(fmaxf(fd, 0.0f), 1.0f);
+            const unsigned long long key =
+                ((unsigned long long)__float_as_uint(fd) << 32) | (unsigned long long)__float_as_uint(-sz);
+            if (key < cur) atomicMin(depth + pix, key);
         }
+    }
 }
 
-__global__ void k_clear(unsigned long long* __restrict__ depth, unsigned long long* __restrict__ thick, size_t m) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m) return;
-    depth[i] = ~0ull;
-    thick[i] = 0ull;
-}
+// Smoothing tiles: SMOOTH_X x SMOOTH_Y pixels, SMOOTH_STEPS steps per launch.
+constexpr int SMOOTH_STEPS = 6, SMOOTH_THREADS = 512;
+constexpr int SMOOTH_X = 64 - 2 * SMOOTH_STEPS, SMOOTH_Y = 16;
+constexpr int SMOOTH_W = 64, SMOOTH_H = SMOOTH_Y + 2 * SMOOTH_STEPS;
 
-// depth texture (0 where no sprite: the reference clears it to 0) and thickness
-__global__ void k_resolve(const unsigned long long* __restrict__ depth, const unsigned long long* __restrict__ thick,
-                          float* __restrict__ z, float* __restrict__ zraw, float* __restrict__ th, size_t m) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m) return;
-    const unsigned long long d = depth[i];
-    const float v = d == ~0ull ? 0.0f : __uint_as_float((unsigned)(d & 0xffffffffull));
-    z[i] = v;
-    zraw[i] = v;
-    th[i] = (float)(long long)thick[i] * (1.0f / kThickScale);
+// Depth texture (0 where no sprite: the reference clears it to 0), in both images
+// the smoothing alternates between, and thickness, one smoothing tile per block;
+// tiles with fluid enter the list (tiles[0]: their number) the smoothing runs over.
+// A smoothing step keeps empty pixels empty, so the others stay as written here.
+__global__ void __launch_bounds__(256) k_resolve(const unsigned long long* __restrict__ depth,
+                                                 const unsigned long long* __restrict__ thick, float* __restrict__ z,
+                                                 float* __restrict__ z1, float* __restrict__ zraw,
+                                                 float* __restrict__ th, int w, int h, int* __restrict__ tiles) {
+    bool any = false;
+    for (int i = threadIdx.x; i < SMOOTH_X * SMOOTH_Y; i += 256) {
+        const int x = blockIdx.x * SMOOTH_X + i % SMOOTH_X, y = blockIdx.y * SMOOTH_Y + i / SMOOTH_X;
+        if (x >= w || y >= h) continue;
+        const size_t o = (size_t)y * w + x;
+        const unsigned long long d = depth[o];
+        const float v = d == ~0ull ? 0.0f : __uint_as_float((unsigned)(d & 0xffffffffull));
+        z[o] = v;
+        z1[o] = v;
+        zraw[o] = v;
+        th[o] = (float)(long long)thick[o] * (1.0f / kThickScale);
+        any = any || v > 0.0f;
+    }
+    if (__syncthreads_or(any) && threadIdx.x == 0) tiles[1 + atomicAdd(tiles, 1)] = blockIdx.y * gridDim.x + blockIdx.x;
 }
 
 // texel (x, y) with GL_REPEAT wrapping
@@ -141,56 +156,98 @@ __device__ __forceinline__ float tex(const float* __restrict__ a, int x, int y, 
     return a[(size_t)y * w + x];
 }
 
-// smooth.frag: one explicit curvature-flow step of the depth image
-__global__ void __launch_bounds__(256) k_smooth(const float* __restrict__ zin, float* __restrict__ zout, int w, int h,
-                                                float Fx, float Fy) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
-    if (x >= w) return;
-    const float Cx = 2.0f / ((float)w * Fx), Cy = 2.0f / ((float)h * Fy);
-    const float z = tex(zin, x, y, w, h);
-    float out = 0.0f;
-    if (z > 0.0f) {
-        const float zpx = tex(zin, x + 1, y, w, h), zmx = tex(zin, x - 1, y, w, h);
-        const float dzdx = (zpx == 0.0f || zmx == 0.0f) ? 0.0f : (zpx - zmx) * 0.5f;
-        const float dz2dx2 = (zpx + zmx) - 2.0f * z;
-        const float zpy = tex(zin, x, y + 1, w, h), zmy = tex(zin, x, y - 1, w, h);
-        const float dzdy = (zpy == 0.0f || zmy == 0.0f) ? 0.0f : (zpy - zmy) * 0.5f;
-        const float dz2dy2 = (zpy + zmy) - 2.0f * z;
-        const float zpp = tex(zin, x + 1, y + 1, w, h), zpm = tex(zin, x + 1, y - 1, w, h);
-        const float zmp = tex(zin, x - 1, y + 1, w, h), zmm = tex(zin, x - 1, y - 1, w, h);
-        const float dz2dxdy = (((zpp + zmm) - zmp) - zpm) * 0.25f;
-        const float nx = -Cy * dzdx, ny = Cx * dzdy, nz = (Cx * Cy) * z;
-        const float D = dot3(nx, ny, nz, nx, ny, nz);
-        const float Cx2 = Cx * Cx, Cy2 = Cy * Cy;
-        const float dDdx = 2.0f * (((Cy2 * dzdx) * dz2dx2 + (Cx2 * dzdy) * dz2dxdy) + ((Cx2 * Cy2) * z) * dzdx);
-        const float dDdy = 2.0f * (((Cy2 * dzdx) * dz2dxdy + (Cx2 * dzdy) * dz2dy2) + ((Cx2 * Cy2) * z) * dzdy);
-        const float Ex = (0.5f * dzdx) * dDdx - dz2dx2 * D;
-        const float Ey = (0.5f * dzdy) * dDdy - dz2dy2 * D;
-        const float H = (0.5f * (Cy * Ex + Cx * Ey)) / (D * sqrtf(D));
-        out = z - H * 0.01f;
-        if (out < 0.0f) out = z;
+// Constants of the smoothing and normal passes, the same float expressions the
+// shaders evaluate per fragment, evaluated once on the host.
+struct Flow {
+    float Cx, Cy;      // 2 / (w Fx), 2 / (h Fy)
+    float Cx2, Cy2;    // squares
+    float CxCy, Cx2Cy2;
+};
+
+// smooth.frag: SMOOTH_STEPS explicit curvature-flow steps of the depth image (fewer
+// when `steps` says so). A block stages a tile with a border of `steps` pixels and
+// applies the steps in shared memory, each on a region one pixel narrower, so an
+// image's 60 steps take 10 launches instead of 60 (a step of an 800 x 800 image is
+// about 1 us of arithmetic in a 3.9 us launch). The resident blocks stride over the
+// list of tiles with fluid: with a block per tile the empty ones, most of an image,
+// took longer than the others. 60 steps of an 800 x 800 image that is 9 % fluid:
+// 236 us a step a launch; 137 with six steps and a block per tile; 93 with the list
+// (107 with four steps and tiles of 56 x 4, 121 with ten and 44 x 8, 93 with 52 x 8).
+__global__ void __launch_bounds__(SMOOTH_THREADS) k_smooth(const float* __restrict__ zin, float* __restrict__ zout,
+                                                           int w, int h, int steps, Flow f,
+                                                           const int* __restrict__ tiles, int tiles_x) {
+    __shared__ float s[2][SMOOTH_H][SMOOTH_W];
+    const int sw = SMOOTH_X + 2 * steps, sh = SMOOTH_Y + 2 * steps;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // GL_REPEAT; far borders of a small image wrap more than once
+    auto wrap = [](int v, int m) {
+        if (v >= 0 && v < m) return v;
+        v %= m;
+        return v < 0 ? v + m : v;
+    };
+    const int count = tiles[0];
+    for (int q = blockIdx.x; q < count; q += gridDim.x) {
+        const int tile = tiles[1 + q];
+        const int tx = tile % tiles_x * SMOOTH_X, ty = tile / tiles_x * SMOOTH_Y;
+        const int xa = wrap(tx - steps + lane, w), xb = wrap(tx - steps + lane + 32, w);
+        for (int ly = warp; ly < sh; ly += SMOOTH_THREADS / 32) {
+            const float* row = zin + (size_t)wrap(ty - steps + ly, h) * w;
+            s[0][ly][lane] = row[xa];
+            s[0][ly][lane + 32] = lane + 32 < sw ? row[xb] : 0.0f;
+        }
+        __syncthreads();
+        int b = 0;
+        for (int k = 1; k <= steps; ++k) {
+            // a warp per half row of 32 pixels
+            for (int i = 2 * k + warp; i < 2 * (sh - k); i += SMOOTH_THREADS / 32) {
+                const int ly = i >> 1, lx = lane + 32 * (i & 1);
+                if (lx < k || lx >= sw - k) continue;
+                const float z = s[b][ly][lx];
+                float out = 0.0f;
+                if (z > 0.0f) {
+                    const float zpx = s[b][ly][lx + 1], zmx = s[b][ly][lx - 1];
+                    const float dzdx = (zpx == 0.0f || zmx == 0.0f) ? 0.0f : (zpx - zmx) * 0.5f;
+                    const float dz2dx2 = (zpx + zmx) - 2.0f * z;
+                    const float zpy = s[b][ly + 1][lx], zmy = s[b][ly - 1][lx];
+                    const float dzdy = (zpy == 0.0f || zmy == 0.0f) ? 0.0f : (zpy - zmy) * 0.5f;
+                    const float dz2dy2 = (zpy + zmy) - 2.0f * z;
+                    const float zpp = s[b][ly + 1][lx + 1], zpm = s[b][ly - 1][lx + 1];
+                    const float zmp = s[b][ly + 1][lx - 1], zmm = s[b][ly - 1][lx - 1];
+                    const float dz2dxdy = (((zpp + zmm) - zmp) - zpm) * 0.25f;
+                    const float nx = -f.Cy * dzdx, ny = f.Cx * dzdy, nz = f.CxCy * z;
+                    const float D = dot3(nx, ny, nz, nx, ny, nz);
+                    const float dDdx =
+                        2.0f * (((f.Cy2 * dzdx) * dz2dx2 + (f.Cx2 * dzdy) * dz2dxdy) + (f.Cx2Cy2 * z) * dzdx);
+                    const float dDdy =
+                        2.0f * (((f.Cy2 * dzdx) * dz2dxdy + (f.Cx2 * dzdy) * dz2dy2) + (f.Cx2Cy2 * z) * dzdy);
+                    const float Ex = (0.5f * dzdx) * dDdx - dz2dx2 * D;
+                    const float Ey = (0.5f * dzdy) * dDdy - dz2dy2 * D;
+                    const float H = (0.5f * (f.Cy * Ex + f.Cx * Ey)) / (D * sqrtf(D));
+                    out = z - H * 0.01f;
+                    if (out < 0.0f) out = z;
+                }
+                s[b ^ 1][ly][lx] = out;
+            }
+            __syncthreads();
+            b ^= 1;
+        }
+        for (int ly = warp; ly < SMOOTH_Y; ly += SMOOTH_THREADS / 32)
+            for (int lx = lane; lx < SMOOTH_X; lx += 32)
+                if (tx + lx < w && ty + ly < h) zout[(size_t)(ty + ly) * w + tx + lx] = s[b][ly + steps][lx + steps];
+        __syncthreads();  // the next tile is staged over this one
     }
-    zout[(size_t)y * w + x] = out;
 }
 
 // normal.frag
-__global__ void __launch_bounds__(256) k_normals(const float* __restrict__ zin, float4* __restrict__ nrm, int w, int h,
-                                                 float Fx, float Fy) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
-    if (x >= w) return;
-    const float Cx = 2.0f / ((float)w * Fx), Cy = 2.0f / ((float)h * Fy);
-    const float z = tex(zin, x, y, w, h);
-    float4 n = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (z > 0.0f) {
-        const float zpx = tex(zin, x + 1, y, w, h), zmx = tex(zin, x - 1, y, w, h);
-        const float dzdx = (zpx == 0.0f || zmx == 0.0f) ? 0.0f : (zpx - zmx) * 0.5f;
-        const float zpy = tex(zin, x, y + 1, w, h), zmy = tex(zin, x, y - 1, w, h);
-        const float dzdy = (zpy == 0.0f || zmy == 0.0f) ? 0.0f : (zpy - zmy) * 0.5f;
-        const float nx = -Cy * dzdx, ny = Cx * dzdy, nz = (Cx * Cy) * z;
-        const float len = sqrtf(dot3(nx, ny, nz, nx, ny, nz));
-        n = make_float4(nx / len, ny / len, nz / len, 0.0f);
-    }
-    nrm[(size_t)y * w + x] = n;
+__device__ __forceinline__ float4 normal_at(const float* __restrict__ zin, int x, int y, int w, int h, float z,
+                                            const Flow& f) {
+    const float zpx = tex(zin, x + 1, y, w, h), zmx = tex(zin, x - 1, y, w, h);
+    const float dzdx = (zpx == 0.0f || zmx == 0.0f) ? 0.0f : (zpx - zmx) * 0.5f;
+    const float zpy = tex(zin, x, y + 1, w, h), zmy = tex(zin, x, y - 1, w, h);
+    const float dzdy = (zpy == 0.0f || zmy == 0.0f) ? 0.0f : (zpy - zmy) * 0.5f;
+    const float nx = -f.Cy * dzdx, ny = f.Cx * dzdy, nz = f.CxCy * z;
+    const float len = sqrtf(dot3(nx, ny, nz, nx, ny, nz));
+    return make_float4(nx / len, ny / len, nz / len, 0.0f);
 }
 
 __device__ __forceinline__ float quant8(float v) {  // an 8-bit normalised texel
@@ -199,10 +256,15 @@ __device__ __forceinline__ float quant8(float v) {  // an 8-bit normalised texel
 
 // The room of the reference app (left, right and back walls and the floor of a
 // box, src/renderapp.cpp:58-85) lit by background.frag, one ray per pixel; the
-// clear colour 0.75 where no wall is hit.
-__global__ void __launch_bounds__(256) k_room(Cam c, float4* __restrict__ out) {
+// clear colour 0.75 where no wall is hit. Also clears the sprite images and the
+// list of tiles.
+__global__ void __launch_bounds__(256) k_room(Cam c, float4* __restrict__ out, unsigned long long* __restrict__ depth,
+                                              unsigned long long* __restrict__ thick, int* __restrict__ tiles) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
     if (x >= c.w) return;
+    if (x == 0 && y == 0) tiles[0] = 0;
+    depth[(size_t)y * c.w + x] = ~0ull;
+    thick[(size_t)y * c.w + x] = 0ull;
     // view-space direction through the pixel centre, then to world space
     const float ux = (2.0f * ((float)x + 0.5f) / (float)c.w - 1.0f) / c.P[0];
     const float uy = (2.0f * ((float)y + 0.5f) / (float)c.h - 1.0f) / c.P[5];
@@ -241,20 +303,22 @@ __global__ void __launch_bounds__(256) k_room(Cam c, float4* __restrict__ out) {
     out[(size_t)y * c.w + x] = make_float4(quant8(col.x), quant8(col.y), quant8(col.z), 1.0f);
 }
 
-// shadingParticle.frag
-__global__ void __launch_bounds__(256) k_shade(Cam c, const float* __restrict__ z_img,
-                                               const float* __restrict__ th_img, const float4* __restrict__ n_img,
+// normal.frag and shadingParticle.frag
+__global__ void __launch_bounds__(256) k_shade(Cam c, Flow fl, const float* __restrict__ z_img,
+                                               const float* __restrict__ th_img, float4* __restrict__ n_img,
                                                const float4* __restrict__ room, float4* __restrict__ out) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
     if (x >= c.w) return;
     const size_t pix = (size_t)y * c.w + x;
     const float z = z_img[pix];
     if (!(z > 0.0f)) {
+        n_img[pix] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         out[pix] = room[pix];
         return;
     }
     const float u = ((float)x + 0.5f) / (float)c.w, v = ((float)y + 0.5f) / (float)c.h;
-    const float4 n = n_img[pix];
+    const float4 n = normal_at(z_img, x, y, c.w, c.h, z, fl);
+    n_img[pix] = n;
     const float sx = (2.0f * u - 1.0f) * c.tan_half * z, sy = (2.0f * v - 1.0f) * c.tan_half * z, sz = -z;
     float vx = -sx, vy = -sy, vz = -sz;
     const float vl = sqrtf(dot3(vx, vy, vz, vx, vy, vz));
@@ -317,6 +381,8 @@ struct pbf_render {
     unsigned long long *depth = nullptr, *thick64 = nullptr;
     float *zraw = nullptr, *z0 = nullptr, *z1 = nullptr, *thick = nullptr;
     float4 *normal = nullptr, *room = nullptr, *color = nullptr;
+    int* tiles = nullptr;  // number and list of smoothing tiles with fluid
+    int sms = 148;
     const float* zfinal = nullptr;  // the smoothed depth of the last frame
     cudaStream_t last = nullptr;
 };
@@ -326,7 +392,7 @@ namespace {
 int rfail(int code, const char* msg) { return pbf::set_last_error(code, msg); }
 
 void rfree(pbf_render* r) {
-    void* ptrs[] = {r->depth, r->thick64, r->zraw, r->z0, r->z1, r->thick, r->normal, r->room, r->color};
+    void* ptrs[] = {r->depth, r->thick64, r->zraw, r->z0, r->z1, r->thick, r->normal, r->room, r->color, r->tiles};
     for (void* p : ptrs)
         if (p) cudaFree(p);
 }
@@ -349,26 +415,31 @@ int render_points(pbf_render* r, const float* pos, int n, int stride, const pbf_
         return rfail(PBF_ERR_INVALID, "smooth_iterations must lie in [0, 1000]");
     if (!(cam->radius > 0.0f) || !(cam->point_coeff > 0.0f)) return rfail(PBF_ERR_INVALID, "radius and point_coeff must be positive");
     const Cam c = make_cam(*cam, r->w, r->h);
-    const size_t m = (size_t)r->w * r->h;
-    const int b1 = (int)((m + 255) / 256);
-    k_clear<<<b1, 256, 0, st>>>(r->depth, r->thick64, m);
-    if (n > 0) {
-        k_splat<false><<<(n + 255) / 256, 256, 0, st>>>(c, pos, n, stride, r->depth, r->thick64);
-        k_splat<true><<<(n + 255) / 256, 256, 0, st>>>(c, pos, n, stride, r->depth, r->thick64);
-    }
-    k_resolve<<<b1, 256, 0, st>>>(r->depth, r->thick64, r->z0, r->zraw, r->thick, m);
     const dim3 g2((r->w + 255) / 256, r->h);
+    k_room<<<g2, 256, 0, st>>>(c, r->room, r->depth, r->thick64, r->tiles);
+    if (n > 0) k_splat<<<(n + 255) / 256, 256, 0, st>>>(c, pos, n, stride, r->depth, r->thick64);
+    const dim3 gs((r->w + SMOOTH_X - 1) / SMOOTH_X, (r->h + SMOOTH_Y - 1) / SMOOTH_Y);
+    k_resolve<<<gs, 256, 0, st>>>(r->depth, r->thick64, r->z0, r->z1, r->zraw, r->thick, r->w, r->h, r->tiles);
     const float Fy = cam->proj[0], Fx = cam->proj[5];  // the reference's names: Fy = P[0][0], Fx = P[1][1]
+    Flow f{};
+    f.Cx = 2.0f / ((float)r->w * Fx);
+    f.Cy = 2.0f / ((float)r->h * Fy);
+    f.Cx2 = f.Cx * f.Cx;
+    f.Cy2 = f.Cy * f.Cy;
+    f.CxCy = f.Cx * f.Cy;
+    f.Cx2Cy2 = f.Cx2 * f.Cy2;
+    const unsigned resident = (unsigned)r->sms * (2048 / SMOOTH_THREADS);
+    const unsigned blocks = gs.x * gs.y < resident ? gs.x * gs.y : resident;
     float* a = r->z0;
     float* b = r->z1;
-    for (int it = 0; it < cam->smooth_iterations; ++it) {
-        k_smooth<<<g2, 256, 0, st>>>(a, b, r->w, r->h, Fx, Fy);
+    for (int it = 0; it < cam->smooth_iterations; it += SMOOTH_STEPS) {
+        const int left = cam->smooth_iterations - it;
+        k_smooth<<<blocks, SMOOTH_THREADS, 0, st>>>(a, b, r->w, r->h, left < SMOOTH_STEPS ? left : SMOOTH_STEPS, f,
+                                                    r->tiles, (int)gs.x);
         float* t = a; a = b; b = t;
     }
     r->zfinal = a;
-    k_normals<<<g2, 256, 0, st>>>(a, r->normal, r->w, r->h, Fx, Fy);
-    k_room<<<g2, 256, 0, st>>>(c, r->room);
-    k_shade<<<g2, 256, 0, st>>>(c, a, r->thick, r->normal, r->room, r->color);
+    k_shade<<<g2, 256, 0, st>>>(c, f, a, r->thick, r->normal, r->room, r->color);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return rfail(PBF_ERR_CUDA, cudaGetErrorString(e));
     r->last = st;
@@ -398,6 +469,12 @@ int pbf_render_create(int width, int height, pbf_render** out) {
     e = e ? e : cudaMalloc((void**)&r->normal, m * 16);
     e = e ? e : cudaMalloc((void**)&r->room, m * 16);
     e = e ? e : cudaMalloc((void**)&r->color, m * 16);
+    const size_t tiles = (size_t)((width + pbf::SMOOTH_X - 1) / pbf::SMOOTH_X) *
+                         ((height + pbf::SMOOTH_Y - 1) / pbf::SMOOTH_Y);
+    e = e ? e : cudaMalloc((void**)&r->tiles, (tiles + 1) * sizeof(int));
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&r->sms, cudaDevAttrMultiProcessorCount, dev);
+    if (r->sms <= 0) r->sms = 148;
     if (e != cudaSuccess) {
         rfree(r);
         delete r;
