@@ -724,7 +724,7 @@ int create_common(const pbf_solver_parameter* para, int nscenes, const pbf_scene
             return rc;                     \
         }                                  \
     } while (0)
-    AL(s->Sx, n); AL(s->Sv, n); AL(s->Px, n); AL(s->Pv, n); AL(s->Pxold, n); AL(s->Q, n); AL(s->omega, n); AL(s->vw, n);
+    AL(s->Sx, n); AL(s->Sv, n); AL(s->Px, n + 1); AL(s->Pv, n); AL(s->Pxold, n); AL(s->Q, n); AL(s->omega, n); AL(s->vw, n);
     AL(s->Sperm, n); AL(s->Pperm, n); AL(s->cell, n); AL(s->ticket, n); AL(s->tmp, n); AL(s->cell_sorted, n);
     AL(s->ncnt, n);
     AL(s->nbr, (size_t)ext->max_neighbors * s->stride);
