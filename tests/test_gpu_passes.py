@@ -1,0 +1,81 @@
+"""The neighbour passes at the sizes where their variants change, bit for bit
+against the oracle: eight threads per particle up to 9,472 particles (148 SMs x 4
+blocks x 16), the search with eight threads up to 45,056, and the layout for a
+device that is not full up to 113,664 threads (148 SMs x 3 blocks x 256), a particle
+taking one, two or four threads with one or two, four and eight pair lanes. Also
+the searched lists where rows leave the grid, for cells from h/3 to 3h/2, and
+s_corr exponents other than four, which have kernels of their own."""
+import numpy as np
+import pytest
+
+from pbf_b200 import autotune, scenes
+
+from test_gpu_parity import assert_substep_bitexact, make_pair
+
+pytestmark = pytest.mark.gpu
+
+
+def block_of(n, iters=2):
+    """n particles of a dam break large enough to hold them."""
+    side = int(np.ceil(n ** (1.0 / 3.0)))
+    sc = scenes.dam_break(side, (int(1.3 * side) + 4, side + 4, side + 4), stable=True, iterations=iters)
+    sc.pos, sc.vel = sc.pos[:n].copy(), sc.vel[:n].copy()
+    sc.para.nParticles = n
+    return sc
+
+
+@pytest.mark.parametrize("n,lanes,cell", [(9472, 2, 0.5), (9473, 2, 0.5), (9472, 1, 1.0), (9473, 1, 1.0),
+                                          (9473, 4, 0.5), (9473, 8, 0.5), (45056, 2, 0.5), (45057, 2, 1.0),
+                                          (56833, 4, 0.5), (28417, 8, 0.5), (113664, 2, 0.5), (113665, 2, 0.5),
+                                          (113665, 1, 1.0), (113664, 1, 0.5)])
+def test_variant_boundaries_bitexact(n, lanes, cell):
+    sc = block_of(n)
+    s, orc = make_pair(sc, pair_lanes=lanes, cell_scale=cell,
+                       grid_dims=autotune.dims_for_scale(sc.ext_overrides["grid_dims"], cell))
+    s.step(1)
+    orc.substep()
+    assert_substep_bitexact(s, orc)
+    s.close()
+    orc.close()
+
+
+@pytest.mark.parametrize("exponent", [1.0, 3.0, 3.5])
+@pytest.mark.parametrize("n", [1200, 12000])
+def test_scorr_exponents_bitexact(n, exponent):
+    """Whole exponents are repeated products; 3.5 goes through powf, whose last bit
+    is not the host's, so its corrections are compared within 1e-6 of their scale."""
+    sc = block_of(n)
+    sc.para.n = exponent
+    s, orc = make_pair(sc)
+    s.step(1)
+    orc.substep()
+    if exponent == 3.5:
+        want = orc.get("dp")
+        assert np.abs(s.fetch("dp")[:, :3] - want).max() <= 1e-6 * np.abs(want).max()
+    else:
+        assert_substep_bitexact(s, orc)
+
+
+@pytest.mark.parametrize("cell", [1.0 / 3.0, 0.5, 0.7, 1.0, 1.5])
+@pytest.mark.parametrize("n", [2100, 46000])
+def test_search_around_the_grid_bitexact(cell, n):
+    """Particles in and around a grid smaller than their box, on every side and far
+    away, with clumps beyond the neighbour cap."""
+    rng = np.random.RandomState(5)
+    sc = scenes.dam_break(4, (60, 60, 60), stable=True, iterations=1)
+    side = 0.05 * n ** (1.0 / 3.0)
+    pos = rng.uniform(0.0, side + 0.8, size=(n, 3))
+    pos[: n // 7] = 0.5 * side + rng.uniform(0.0, 0.25, size=(n // 7, 3))
+    pos[-3:] = [[5.9, 0.3, 0.3], [0.3, 5.9, 0.3], [0.3, 0.3, 5.9]]
+    sc.pos, sc.vel = pos.astype(np.float32), np.zeros((n, 3), np.float32)
+    sc.para.nParticles = n
+    sc.grid_space = [0.25, 0.2, 0.15, 6.0, 6.0, 6.0]
+    dims = [int(np.ceil((side + 0.3) / (0.1 * cell)))] * 3
+    s, orc = make_pair(sc, cell_scale=cell, grid_dims=dims)
+    s.step(1)
+    orc.substep()
+    cnt = orc.get("ncnt")
+    assert (cnt == 63).any() and (orc.get("cell") < 0).any()
+    assert_substep_bitexact(s, orc)
+    s.close()
+    orc.close()
