@@ -84,13 +84,33 @@ template <typename T> __device__ __forceinline__ T3<T> cross3v(const T3<T>& a, c
             vfma(a.x, b.y, vmul(vmul(a.y, b.x), m1))};
 }
 
-// xyz (or .w) of V gathered float4s as one packet
-__device__ __forceinline__ T3<float> pack3(const float4 (&a)[1]) { return {a[0].x, a[0].y, a[0].z}; }
-__device__ __forceinline__ T3<float2> pack3(const float4 (&a)[2]) {
-    return {make_float2(a[0].x, a[1].x), make_float2(a[0].y, a[1].y), make_float2(a[0].z, a[1].z)};
-}
+// .w of V gathered float4s as one packet
 __device__ __forceinline__ float packw(const float4 (&a)[1]) { return a[0].w; }
 __device__ __forceinline__ float2 packw(const float4 (&a)[2]) { return make_float2(a[0].w, a[1].w); }
+
+// a - b_v for the xyz of V gathered float4s: one scalar subtraction per component,
+// which leaves the V results side by side (packing the gathered registers first
+// takes more instructions than it saves)
+__device__ __forceinline__ T3<float> diff3(const f3& a, const float4 (&b)[1]) {
+    return {a.x - b[0].x, a.y - b[0].y, a.z - b[0].z};
+}
+__device__ __forceinline__ T3<float2> diff3(const f3& a, const float4 (&b)[2]) {
+    return {make_float2(a.x - b[0].x, a.x - b[1].x), make_float2(a.y - b[0].y, a.y - b[1].y),
+            make_float2(a.z - b[0].z, a.z - b[1].z)};
+}
+// b_v - a
+__device__ __forceinline__ T3<float> rdiff3(const float4 (&b)[1], const f3& a) {
+    return {b[0].x - a.x, b[0].y - a.y, b[0].z - a.z};
+}
+__device__ __forceinline__ T3<float2> rdiff3(const float4 (&b)[2], const f3& a) {
+    return {make_float2(b[0].x - a.x, b[1].x - a.x), make_float2(b[0].y - a.y, b[1].y - a.y),
+            make_float2(b[0].z - a.z, b[1].z - a.z)};
+}
+// a + w_v
+__device__ __forceinline__ float addw(float a, const float4 (&b)[1]) { return a + b[0].w; }
+__device__ __forceinline__ float2 addw(float a, const float4 (&b)[2]) {
+    return make_float2(a + b[0].w, a + b[1].w);
+}
 
 template <int V> using vec_t = typename std::conditional<V == 1, float, float2>::type;
 
@@ -105,15 +125,18 @@ template <int V> using vec_t = typename std::conditional<V == 1, float, float2>:
 // rounded |r|^2 exceeds h^2, and c (+0)^3 = +0). A padding entry is the particle
 // itself (r = +0, |r| below rmin), which the gradient's cutoff already drops;
 // only its density weight needs `valid`.
-template <typename T, bool NEED_W>
-__device__ __forceinline__ void pair_terms(const KParams& p, const f3& xk, const T3<T>& xj, unsigned valid, T3<T>& r,
-                                           T& w, T3<T>& g) {
+template <typename T, bool NEED_W, int V>
+__device__ __forceinline__ void pair_terms(const KParams& p, const f3& xk, const float4 (&xj)[V], unsigned valid,
+                                           T3<T>& r, T& w, T3<T>& g) {
     const T m1 = bc<T>(-1.0f);
-    r = {vfma(xj.x, m1, bc<T>(xk.x)), vfma(xj.y, m1, bc<T>(xk.y)), vfma(xj.z, m1, bc<T>(xk.z))};
+    r = diff3(xk, xj);
     const T r2 = vfma(r.z, r.z, vfma(r.y, r.y, vmul(r.x, r.x)));
     if (NEED_W) {
         const T t = vmax(vfma(r2, m1, bc<T>(p.h2)), 0.0f);
-        w = keep_only(vmul(bc<T>(p.poly6_c), vmul(vmul(t, t), t)), valid);
+        // c t^3 as fma(c, t^3, +0), the same value (c t^3 is never -0): the density
+        // sum adds w, and a packed product whose only use is an addition may be fused
+        // into it by the code generator
+        w = keep_only(vfma(bc<T>(p.poly6_c), vmul(vmul(t, t), t), bc<T>(0.0f)), valid);
     }
     const T ny = vrsqrt_neg(vmax(r2, 1e-30f));
     const T nrl = vmul(r2, ny);               // -|r| for the cutoff
@@ -132,10 +155,12 @@ __device__ __forceinline__ float vpow(float q, const KParams& p) { return powf(q
 __device__ __forceinline__ float2 vpow(float2 q, const KParams& p) {
     return make_float2(powf(q.x, p.n_exp), powf(q.y, p.n_exp));
 }
-template <typename T> __device__ __forceinline__ T dp_weight(const KParams& p, float li, T lj, T w) {
+// N4: the usual n = 4, ((q q) q) q, as a constant, so that the pair loop has no
+// branch and the pairs of a batch overlap.
+template <bool N4, typename T> __device__ __forceinline__ T dp_weight(const KParams& p, T lij, T w) {
     const T q = vmul(w, bc<T>(p.inv_wdq));
     T pw;
-    if (p.n_int == 4) {  // the usual n = 4 without a loop: ((q q) q) q
+    if (N4) {
         pw = vmul(vmul(vmul(q, q), q), q);
     } else if (p.n_int > 0) {
         pw = q;
@@ -143,7 +168,7 @@ template <typename T> __device__ __forceinline__ T dp_weight(const KParams& p, f
     } else {
         pw = vpow(q, p);
     }
-    return vfma(vmul(bc<T>(p.nk), pw), bc<T>(p.scorr_scale), vadd(bc<T>(li), lj));
+    return vfma(vmul(bc<T>(p.nk), pw), bc<T>(p.scorr_scale), lij);
 }
 
 // ---- teams -------------------------------------------------------------------
@@ -191,18 +216,61 @@ __device__ __forceinline__ void load_idx(const KParams& p, const int* __restrict
         }
 }
 
-// bit v: entry q + v exists (the callers have q < cnt, so bit 0 is always set)
+// bit v: entry q + v exists
 template <int V> __device__ __forceinline__ unsigned valid_bits(int q, int cnt) {
-    return V == 1 ? 1u : (q + 1 < cnt ? 3u : 1u);
+    return (q < cnt ? 1u : 0u) | (V == 2 && q + 1 < cnt ? 2u : 0u);
+}
+
+// How a pass's inner loop is laid out. A batch of E entries per thread has its
+// gathers issued together and no branch inside: the entries past the end of a list
+// are the particle itself and add zeros, and the pairs of a batch overlap (a test
+// per entry kept them apart: a step then took the whole latency of its arithmetic;
+// 1 M particles, lambda: 81.6 us with the test, 68.9 without; 32,768 particles: 8.1
+// and 6.2).
+//   full device: four entries in the one-array passes, two in the two-array ones,
+//     which then keep their next indices in registers at four blocks per SM (1 M
+//     particles: curl 107 -> 102 us, vorticity 129 -> 118); the correction fits
+//     five blocks (84.8 -> 71.6), lambda is faster at four (69 against 71.5);
+//   ROOMY, all blocks resident at three per SM: four entries everywhere and
+//     registers for it (32,768 particles: lambda 6.0 -> 5.9 us, correction 6.6 ->
+//     5.8, curl 10.4 -> 6.7, vorticity 11 -> 8.3).
+constexpr int ROOMY_BLOCKS = 3;
+
+// body(xj, vj, valid) for the neighbours of slot k that thread t of its team
+// takes, gathered from NA arrays through the list of slots, E entries per batch; the
+// next batch's indices load while a batch computes.
+template <int L, int V, int E, int NA, typename F>
+__device__ __forceinline__ void for_list(const KParams& p, const int* __restrict__ nbr, int k, int t, int cnt,
+                                         const float4* __restrict__ a, const float4* __restrict__ b, F&& body) {
+    constexpr int P = L * V, B = E / V;
+    int jj[B][V];
+    load_idx<V, P, B>(p, nbr, k, V * t, cnt, jj);
+    for (int q0 = V * t; q0 < cnt; q0 += P * B) {
+        float4 xj[B][V], vj[B][V];
+#pragma unroll
+        for (int u = 0; u < B; ++u)
+#pragma unroll
+            for (int c = 0; c < V; ++c) {
+                xj[u][c] = a[jj[u][c]];
+                if (NA == 2) vj[u][c] = b[jj[u][c]];
+            }
+        load_idx<V, P, B>(p, nbr, k, q0 + P * B, cnt, jj);
+#pragma unroll
+        for (int u = 0; u < B; ++u) {
+            const int q = q0 + u * P;
+            body(xj[u], vj[u], valid_bits<V>(q, cnt));
+        }
+    }
 }
 
 // Block-wide max and sum of a per-thread error, folded into one slot with a
 // single pair of atomics per block (max as ordered double bits, value >= 0).
-__device__ __forceinline__ void block_error_reduce(float e, unsigned long long* max_bits, double* sum) {
+__device__ __forceinline__ void block_error_reduce(float e, double esum, unsigned long long* max_bits, double* sum) {
     __shared__ float s_max[32];
-    __shared__ float s_sum[32];
+    __shared__ double s_sum[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float m = e, s = e;
+    float m = e;
+    double s = esum;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -213,16 +281,12 @@ __device__ __forceinline__ void block_error_reduce(float e, unsigned long long* 
     if (threadIdx.x == 0) {
         const int nw = (blockDim.x + 31) >> 5;
         double dsum = 0.0;
-        for (int w = 0; w < nw; ++w) { m = fmaxf(m, s_max[w]); dsum += (double)s_sum[w]; }
+        for (int w = 0; w < nw; ++w) { m = fmaxf(m, s_max[w]); dsum += s_sum[w]; }
         atomicMax(max_bits, (unsigned long long)__double_as_longlong((double)m));
         atomicAdd(sum, dsum);
     }
     __syncthreads();  // a persistent block's next tile writes s_max / s_sum again
 }
-
-// Neighbour entries per thread and batch: four in every pass (V entries per
-// packed instruction, 4 / V instructions' worth of gathers issued together).
-template <int V> __host__ __device__ constexpr int batches() { return 4 / V; }
 
 // ---------------------------------------------------------------------------
 // a9: density, constraint and lambda (calculateLambda cu:156-180), with the
@@ -248,69 +312,77 @@ __device__ __forceinline__ float lambda_tail(const KParams& p, int k, const f3& 
     return __fdiv_rn(-C, gms + p.eps);
 }
 
+// The sums of one pair of the lambda pass.
+template <typename T> struct LambdaSums {
+    T rho, gm;
+    T3<T> gs;
+};
+template <typename T> __device__ __forceinline__ LambdaSums<T> lambda_zero() {
+    return {bc<T>(0.0f), bc<T>(0.0f), zero3<T>()};
+}
+template <typename T, int V>
+__device__ __forceinline__ void lambda_pair(const KParams& p, const f3& xk, const float4 (&xj)[V], unsigned valid,
+                                            LambdaSums<T>& s) {
+    T3<T> r, g;
+    T w;
+    pair_terms<T, true>(p, xk, xj, valid, r, w, g);
+    s.rho = vadd(s.rho, w);
+    s.gs = add3(s.gs, g);
+    s.gm = vfma(g.x, g.x, s.gm);
+    s.gm = vfma(g.y, g.y, s.gm);
+    s.gm = vfma(g.z, g.z, s.gm);
+}
+// The team's sums combined and slot k's lambda written; returns the density
+// error on the team's first thread, 0 on the others.
 template <bool DEBUG, int L, int V>
-__device__ __forceinline__ void lambda_tile(const KParams& p, int vb, const float4* __restrict__ x,
-                                            const int* __restrict__ nbr, const int* __restrict__ ncnt,
-                                            float4* __restrict__ xl, float* __restrict__ rho_out, const IterCtl& ctl) {
-    using T = vec_t<V>;
-    constexpr int P = L * V, B = batches<V>();
-    const Team<L> tm = team_of<L>(vb);
-    const int k = tm.k;
+__device__ __forceinline__ float lambda_store(const KParams& p, const Team<L>& tm, const f3& xk,
+                                              const LambdaSums<vec_t<V>>& s, float4* __restrict__ xl,
+                                              float* __restrict__ rho_out, const IterCtl& ctl) {
+    float rhos = team_sum<L>(fold(s.rho), tm.mask);
+    const float gms = team_sum<L>(fold(s.gm), tm.mask);
+    const f3 g3 = team_sum3<L>(fold3(s.gs), tm.mask);
     float err = 0.0f;
-    if (k < p.n) {
-        const f3 xk = make3(x[k]);
-        const int cnt = ncnt[k];
-        T rho = bc<T>(0.0f), gm = bc<T>(0.0f);
-        T3<T> gs = zero3<T>();
-        int jj[B][V];
-        load_idx<V, P, B>(p, nbr, k, V * tm.t, cnt, jj);
-        for (int q0 = V * tm.t; q0 < cnt; q0 += P * B) {
-            float4 xj[B][V];
-#pragma unroll
-            for (int u = 0; u < B; ++u)
-#pragma unroll
-                for (int v = 0; v < V; ++v) xj[u][v] = x[jj[u][v]];
-            // the next batch's indices load while this batch computes
-            load_idx<V, P, B>(p, nbr, k, q0 + P * B, cnt, jj);
-#pragma unroll
-            for (int u = 0; u < B; ++u) {
-                const int q = q0 + u * P;
-                if (q >= cnt) break;
-                T3<T> r, g;
-                T w;
-                pair_terms<T, true>(p, xk, pack3(xj[u]), valid_bits<V>(q, cnt), r, w, g);
-                rho = vadd(rho, w);
-                gs = add3(gs, g);
-                gm = vfma(g.x, g.x, gm);
-                gm = vfma(g.y, g.y, gm);
-                gm = vfma(g.z, g.z, gm);
-            }
-        }
-        float rhos = team_sum<L>(fold(rho), tm.mask);
-        const float gms = team_sum<L>(fold(gm), tm.mask);
-        const f3 g3 = team_sum3<L>(fold3(gs), tm.mask);
-        if (tm.t == 0) {
-            const float lam = lambda_tail(p, k, xk, rhos, gms, g3, err);
-            xl[k] = make_float4(xk.x, xk.y, xk.z, lam);
-            if (ctl.lam_acc) ctl.lam_acc[k] += lam;
-            if (DEBUG) rho_out[k] = rhos;
-        }
+    if (tm.t == 0) {
+        const int k = tm.k;
+        const float lam = lambda_tail(p, k, xk, rhos, gms, g3, err);
+        xl[k] = make_float4(xk.x, xk.y, xk.z, lam);
+        if (ctl.lam_acc) ctl.lam_acc[k] += lam;
+        if (DEBUG) rho_out[k] = rhos;
     }
-    if (ctl.max_bits) {
-        const int sl = ctl.cur_slot();
-        block_error_reduce(err, ctl.max_bits + sl, ctl.sum + sl);
-    }
+    return err;
+}
+template <bool DEBUG, int L, int V>
+__device__ __forceinline__ float lambda_list(const KParams& p, const Team<L>& tm, const float4* __restrict__ x,
+                                             const int* __restrict__ nbr, const int* __restrict__ ncnt,
+                                             float4* __restrict__ xl, float* __restrict__ rho_out,
+                                             const IterCtl& ctl) {
+    using T = vec_t<V>;
+    const f3 xk = make3(x[tm.k]);
+    LambdaSums<T> s = lambda_zero<T>();
+    for_list<L, V, 4, 1>(p, nbr, tm.k, tm.t, ncnt[tm.k], x, x,
+                            [&](const float4(&xj)[V], const float4(&)[V], unsigned valid) {
+                                lambda_pair<T, V>(p, xk, xj, valid, s);
+                            });
+    return lambda_store<DEBUG, L, V>(p, tm, xk, s, xl, rho_out, ctl);
 }
 
 // nvb tiles of blockDim.x slots' teams; the grid strides over them (a grid of
 // nvb blocks is the ordinary one-block-per-tile launch)
-template <bool DEBUG, int L, int V>
-__global__ void __launch_bounds__(256, V == 1 ? 6 : 4) k_lambda(KParams p, int nvb, const float4* __restrict__ x,
+template <bool DEBUG, bool ROOMY, int L, int V>
+__global__ void __launch_bounds__(256, ROOMY ? ROOMY_BLOCKS : 4) k_lambda(KParams p, int nvb, const float4* __restrict__ x,
                                                                 const int* __restrict__ nbr,
                                                                 const int* __restrict__ ncnt, float4* __restrict__ xl,
                                                                 float* __restrict__ rho_out, IterCtl ctl) {
     if (ctl.done && *ctl.done) return;
-    for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) lambda_tile<DEBUG, L, V>(p, vb, x, nbr, ncnt, xl, rho_out, ctl);
+    for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
+        const Team<L> tm = team_of<L>(vb);
+        float err = 0.0f;
+        if (tm.k < p.n) err = lambda_list<DEBUG, L, V>(p, tm, x, nbr, ncnt, xl, rho_out, ctl);
+        if (ctl.max_bits) {
+            const int sl = ctl.cur_slot();
+            block_error_reduce(err, err, ctl.max_bits + sl, ctl.sum + sl);
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -339,7 +411,7 @@ __device__ __forceinline__ bool features_one(const KParams& p, const Team<L>& tm
                                              float4* __restrict__ xl, float* __restrict__ feat,
                                              float* __restrict__ lam_acc, float (&f)[12], float& lam) {
     using T = vec_t<V>;
-    constexpr int P = L * V, B = batches<V>();
+    constexpr int P = L * V, B = 4 / V;
     const int k = tm.k;
     if (k >= p.n) return false;  // uniform over the team
     const f3 xk = make3(x[k]);
@@ -364,18 +436,16 @@ __device__ __forceinline__ bool features_one(const KParams& p, const Team<L>& tm
 #pragma unroll
         for (int u = 0; u < B; ++u) {
             const int q = q0 + u * P;
-            if (q >= cnt) break;
             const unsigned valid = valid_bits<V>(q, cnt);
             T3<T> r, g;
             T w;
-            pair_terms<T, true>(p, xk, pack3(xj[u]), valid, r, w, g);
+            pair_terms<T, true>(p, xk, xj[u], valid, r, w, g);
             rho = vadd(rho, w);
             gs = add3(gs, g);
             gm = vfma(g.x, g.x, gm);
             gm = vfma(g.y, g.y, gm);
             gm = vfma(g.z, g.z, gm);
-            const T3<T> vv = pack3(vj[u]);
-            const T3<T> vji = {vsub(vv.x, bc<T>(vk.x)), vsub(vv.y, bc<T>(vk.y)), vsub(vv.z, bc<T>(vk.z))};
+            const T3<T> vji = rdiff3(vj[u], vk);
             div = vfma(vji.x, g.x, div);
             div = vfma(vji.y, g.y, div);
             div = vfma(vji.z, g.z, div);
@@ -611,77 +681,22 @@ __global__ void __launch_bounds__(256, 3) k_features_warm(KParams p, int nvb, co
 // and on the last iteration v = (x - x_old) / dt
 // (calculateOffset cu:182-199, updatePosition cu:15-22)
 // ---------------------------------------------------------------------------
-template <bool DEBUG, int L, int V>
-__device__ __forceinline__ void dp_tile(const KParams& p, int vb, const float4* __restrict__ xl,
-                                        const int* __restrict__ nbr, const int* __restrict__ ncnt,
-                                        const float4* __restrict__ xold, float4* __restrict__ xout,
-                                        float4* __restrict__ vout, float4* __restrict__ dp_out);
-
-template <bool DEBUG, int L, int V>
-__global__ void __launch_bounds__(256, V == 1 ? 6 : 4) k_dp(KParams p, int nvb, const float4* __restrict__ xl,
-                                                            const int* __restrict__ nbr, const int* __restrict__ ncnt,
-                                                            const float4* __restrict__ xold, float4* __restrict__ xout,
-                                                            float4* __restrict__ vout, float4* __restrict__ dp_out,
-                                                            IterCtl ctl) {
-    if (ctl.done) {
-        if (*ctl.done) return;
-        // the lambda pass just measured the positions this pass would correct;
-        // when they are within tolerance the loop ends here
-        const int sl = ctl.cur_slot();
-        if (sl >= ctl.min_slot && __longlong_as_double((long long)ctl.max_bits[sl]) <= ctl.tol) {
-            if (blockIdx.x == 0 && threadIdx.x == 0) {
-                *ctl.done = 1;
-                *ctl.conv_slot = sl;
-            }
-            return;
-        }
-        if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(ctl.iters, 1);
-    }
-    for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x)
-        dp_tile<DEBUG, L, V>(p, vb, xl, nbr, ncnt, xold, xout, vout, dp_out);
+template <bool N4, typename T, int V>
+__device__ __forceinline__ void dp_pair(const KParams& p, const f3& xk, float lk, const float4 (&xj)[V],
+                                        unsigned valid, T3<T>& a) {
+    T3<T> r, g;
+    T w;
+    pair_terms<T, true>(p, xk, xj, valid, r, w, g);
+    const T s = dp_weight<N4>(p, addw(lk, xj), w);
+    a = {vfma(s, g.x, a.x), vfma(s, g.y, a.y), vfma(s, g.z, a.z)};
 }
-
-template <bool DEBUG, int L, int V>
-__device__ __forceinline__ void dp_tile(const KParams& p, int vb, const float4* __restrict__ xl,
-                                        const int* __restrict__ nbr, const int* __restrict__ ncnt,
-                                        const float4* __restrict__ xold, float4* __restrict__ xout,
-                                        float4* __restrict__ vout, float4* __restrict__ dp_out) {
-    using T = vec_t<V>;
-    constexpr int P = L * V, B = batches<V>();
-    const Team<L> tm = team_of<L>(vb);
-    const int k = tm.k;
-    if (k >= p.n) return;  // uniform over the team
-    const float4 xk4 = xl[k];
-    const f3 xk = make3(xk4);
-    const float lk = xk4.w;
-    const int cnt = ncnt[k];
-    T3<T> a = zero3<T>();
-    // index prefetch one batch ahead (packed form only: the scalar form has no
-    // registers left for it within 40)
-    constexpr bool PF = V == 2;
-    int jj[B][V];
-    if (PF) load_idx<V, P, B>(p, nbr, k, V * tm.t, cnt, jj);
-    for (int q0 = V * tm.t; q0 < cnt; q0 += P * B) {
-        if (!PF) load_idx<V, P, B>(p, nbr, k, q0, cnt, jj);
-        float4 xj[B][V];
-#pragma unroll
-        for (int u = 0; u < B; ++u)
-#pragma unroll
-            for (int c = 0; c < V; ++c) xj[u][c] = xl[jj[u][c]];
-        if (PF) load_idx<V, P, B>(p, nbr, k, q0 + P * B, cnt, jj);
-#pragma unroll
-        for (int u = 0; u < B; ++u) {
-            const int q = q0 + u * P;
-            if (q >= cnt) break;
-            T3<T> r, g;
-            T w;
-            pair_terms<T, true>(p, xk, pack3(xj[u]), valid_bits<V>(q, cnt), r, w, g);
-            const T s = dp_weight(p, lk, packw(xj[u]), w);
-            a = {vfma(s, g.x, a.x), vfma(s, g.y, a.y), vfma(s, g.z, a.z)};
-        }
-    }
-    f3 as = team_sum3<L>(fold3(a), tm.mask);
-    if (tm.t != 0) return;
+struct DpOut {
+    const float4* xold;
+    float4 *xout, *vout, *dp_out;
+};
+// Particle k moved by its summed correction.
+template <bool DEBUG>
+__device__ __forceinline__ void dp_apply(const KParams& p, int k, const f3& xk, float lk, f3 as, const DpOut& o) {
     if (p.flags & FLAG_WALL_DENSITY) {
         f3 gw;
         wall_term(p, scene_of(p, k), xk, gw);
@@ -692,13 +707,63 @@ __device__ __forceinline__ void dp_tile(const KParams& p, int vb, const float4* 
     const f3 dp = {__fdiv_rn(as.x, p.rho0), __fdiv_rn(as.y, p.rho0), __fdiv_rn(as.z, p.rho0)};
     f3 xn = {xk.x + dp.x, xk.y + dp.y, xk.z + dp.z};
     bound_particle(p, scene_of(p, k), xn);
-    xout[k] = make_float4(xn.x, xn.y, xn.z, 0.0f);
-    if (vout) {
-        const float4 xo = xold[k];
-        vout[k] = make_float4(__fdiv_rn(xn.x - xo.x, p.dt), __fdiv_rn(xn.y - xo.y, p.dt),
-                              __fdiv_rn(xn.z - xo.z, p.dt), 0.0f);
+    o.xout[k] = make_float4(xn.x, xn.y, xn.z, 0.0f);
+    if (o.vout) {
+        const float4 xo = o.xold[k];
+        o.vout[k] = make_float4(__fdiv_rn(xn.x - xo.x, p.dt), __fdiv_rn(xn.y - xo.y, p.dt),
+                                __fdiv_rn(xn.z - xo.z, p.dt), 0.0f);
     }
-    if (DEBUG) dp_out[k] = make_float4(dp.x, dp.y, dp.z, 0.0f);
+    if (DEBUG) o.dp_out[k] = make_float4(dp.x, dp.y, dp.z, 0.0f);
+}
+template <bool DEBUG, int L, int V>
+__device__ __forceinline__ void dp_store(const KParams& p, const Team<L>& tm, const f3& xk, float lk,
+                                         const T3<vec_t<V>>& a, const DpOut& o) {
+    const f3 as = team_sum3<L>(fold3(a), tm.mask);
+    if (tm.t == 0) dp_apply<DEBUG>(p, tm.k, xk, lk, as, o);
+}
+template <bool DEBUG, bool N4, int L, int V>
+__device__ __forceinline__ void dp_list(const KParams& p, const Team<L>& tm, const float4* __restrict__ xl,
+                                        const int* __restrict__ nbr, const int* __restrict__ ncnt, const DpOut& o) {
+    using T = vec_t<V>;
+    const float4 xk4 = xl[tm.k];
+    const f3 xk = make3(xk4);
+    T3<T> a = zero3<T>();
+    for_list<L, V, 4, 1>(p, nbr, tm.k, tm.t, ncnt[tm.k], xl, xl,
+                              [&](const float4(&xj)[V], const float4(&)[V], unsigned valid) {
+                                  dp_pair<N4, T, V>(p, xk, xk4.w, xj, valid, a);
+                              });
+    dp_store<DEBUG, L, V>(p, tm, xk, xk4.w, a, o);
+}
+
+// Adaptive loop: true when this correction is not to be applied (the loop ended
+// before, or ends here because the positions it would correct are within
+// tolerance).
+__device__ __forceinline__ bool dp_skip(const IterCtl& ctl) {
+    if (!ctl.done) return false;
+    if (*ctl.done) return true;
+    // the lambda pass just measured the positions this pass would correct;
+    // when they are within tolerance the loop ends here
+    const int sl = ctl.cur_slot();
+    if (sl >= ctl.min_slot && __longlong_as_double((long long)ctl.max_bits[sl]) <= ctl.tol) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            *ctl.done = 1;
+            *ctl.conv_slot = sl;
+        }
+        return true;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(ctl.iters, 1);
+    return false;
+}
+
+template <bool DEBUG, bool N4, bool ROOMY, int L, int V>
+__global__ void __launch_bounds__(256, ROOMY ? ROOMY_BLOCKS : L == 1 && (N4 || V == 1) ? 5 : 4) k_dp(KParams p, int nvb, const float4* __restrict__ xl,
+                                                            const int* __restrict__ nbr, const int* __restrict__ ncnt,
+                                                            DpOut o, IterCtl ctl) {
+    if (dp_skip(ctl)) return;
+    for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
+        const Team<L> tm = team_of<L>(vb);
+        if (tm.k < p.n) dp_list<DEBUG, N4, L, V>(p, tm, xl, nbr, ncnt, o);  // uniform over the team
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -706,59 +771,51 @@ __device__ __forceinline__ void dp_tile(const KParams& p, int vb, const float4* 
 // writes (w_i, |w_i|) and (v_i, |w_i|): the vorticity pass then gathers two
 // float4s per neighbour (x_j and v_j with |w_j|) instead of three
 // ---------------------------------------------------------------------------
+template <typename T, int V>
+__device__ __forceinline__ void curl_pair(const KParams& p, const f3& xk, const f3& vk, const float4 (&xj)[V],
+                                          const float4 (&vj)[V], unsigned valid, T3<T>& wsum) {
+    T3<T> r, g;
+    T w;
+    pair_terms<T, false>(p, xk, xj, valid, r, w, g);
+    const T3<T> vji = rdiff3(vj, vk);
+    wsum = add3(wsum, cross3v(vji, g));
+}
+__device__ __forceinline__ void curl_apply(int k, const f3& vk, const f3& w3, float4* __restrict__ omega,
+                                           float4* __restrict__ vw) {
+    const float wl = __fsqrt_rn(dot_fma(w3, w3));
+    omega[k] = make_float4(w3.x, w3.y, w3.z, wl);
+    vw[k] = make_float4(vk.x, vk.y, vk.z, wl);
+}
 template <int L, int V>
-__device__ __forceinline__ void curl_tile(const KParams& p, int vb, const float4* __restrict__ x,
+__device__ __forceinline__ void curl_store(const Team<L>& tm, const f3& vk, const T3<vec_t<V>>& wsum,
+                                           float4* __restrict__ omega, float4* __restrict__ vw) {
+    const f3 w3 = team_sum3<L>(fold3(wsum), tm.mask);
+    if (tm.t == 0) curl_apply(tm.k, vk, w3, omega, vw);
+}
+template <bool ROOMY, int L, int V>
+__device__ __forceinline__ void curl_list(const KParams& p, const Team<L>& tm, const float4* __restrict__ x,
                                           const float4* __restrict__ v, const int* __restrict__ nbr,
                                           const int* __restrict__ ncnt, float4* __restrict__ omega,
                                           float4* __restrict__ vw) {
     using T = vec_t<V>;
-    constexpr int P = L * V, B = batches<V>();
-    const Team<L> tm = team_of<L>(vb);
-    const int k = tm.k;
-    if (k >= p.n) return;  // uniform over the team
-    const f3 xk = make3(x[k]);
-    const f3 vk = make3(v[k]);
-    const int cnt = ncnt[k];
+    const f3 xk = make3(x[tm.k]), vk = make3(v[tm.k]);
     T3<T> wsum = zero3<T>();
-    int jj[B][V];
-    load_idx<V, P, B>(p, nbr, k, V * tm.t, cnt, jj);
-    for (int q0 = V * tm.t; q0 < cnt; q0 += P * B) {
-        float4 xj[B][V], vj[B][V];
-#pragma unroll
-        for (int u = 0; u < B; ++u)
-#pragma unroll
-            for (int c = 0; c < V; ++c) {
-                xj[u][c] = x[jj[u][c]];
-                vj[u][c] = v[jj[u][c]];
-            }
-        // the next batch's indices load while this batch computes
-        load_idx<V, P, B>(p, nbr, k, q0 + P * B, cnt, jj);
-#pragma unroll
-        for (int u = 0; u < B; ++u) {
-            const int q = q0 + u * P;
-            if (q >= cnt) break;
-            T3<T> r, g;
-            T w;
-            pair_terms<T, false>(p, xk, pack3(xj[u]), valid_bits<V>(q, cnt), r, w, g);
-            const T3<T> vv = pack3(vj[u]);
-            const T3<T> vji = {vsub(vv.x, bc<T>(vk.x)), vsub(vv.y, bc<T>(vk.y)), vsub(vv.z, bc<T>(vk.z))};
-            wsum = add3(wsum, cross3v(vji, g));
-        }
-    }
-    const f3 w3 = team_sum3<L>(fold3(wsum), tm.mask);
-    if (tm.t == 0) {
-        const float wl = __fsqrt_rn(dot_fma(w3, w3));
-        omega[k] = make_float4(w3.x, w3.y, w3.z, wl);
-        vw[k] = make_float4(vk.x, vk.y, vk.z, wl);
-    }
+    for_list<L, V, ROOMY ? 4 : 2, 2>(p, nbr, tm.k, tm.t, ncnt[tm.k], x, v,
+                            [&](const float4(&xj)[V], const float4(&vj)[V], unsigned valid) {
+                                curl_pair<T, V>(p, xk, vk, xj, vj, valid, wsum);
+                            });
+    curl_store<L, V>(tm, vk, wsum, omega, vw);
 }
 
-template <int L, int V>
-__global__ void __launch_bounds__(256) k_curl(KParams p, int nvb, const float4* __restrict__ x,
+template <bool ROOMY, int L, int V>
+__global__ void __launch_bounds__(256, ROOMY ? ROOMY_BLOCKS : 4) k_curl(KParams p, int nvb, const float4* __restrict__ x,
                                               const float4* __restrict__ v, const int* __restrict__ nbr,
                                               const int* __restrict__ ncnt, float4* __restrict__ omega,
                                               float4* __restrict__ vw) {
-    for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) curl_tile<L, V>(p, vb, x, v, nbr, ncnt, omega, vw);
+    for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
+        const Team<L> tm = team_of<L>(vb);
+        if (tm.k < p.n) curl_list<ROOMY, L, V>(p, tm, x, v, nbr, ncnt, omega, vw);  // uniform over the team
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -769,97 +826,316 @@ __global__ void __launch_bounds__(256) k_curl(KParams p, int nvb, const float4* 
 // a2: prediction, wall clamp, cell key and its histogram), which therefore needs
 // no pass of its own.
 // ---------------------------------------------------------------------------
-// One particle (team tm); returns its next cell key on the team's first thread
-// and -1 on the others.
-template <bool DEBUG, int L, int V>
-__device__ __forceinline__ int vort_one(const KParams& p, const Team<L>& tm, int k, const float4* __restrict__ x,
-                                        const float4* __restrict__ vw, const float4* __restrict__ omega,
-                                        const int* __restrict__ nbr, const int* __restrict__ ncnt,
-                                        float4* __restrict__ xout, float4* __restrict__ vout,
-                                        const int* __restrict__ perm_in, int* __restrict__ perm_out,
-                                        float4* __restrict__ vort_out, float4* __restrict__ visc_out,
-                                        int* __restrict__ err) {
-    using T = vec_t<V>;
-    constexpr int P = L * V, B = batches<V>();  // two 16-byte gathers per entry
-    const f3 xk = make3(x[k]);
-    const f3 vk = make3(vw[k]);
-    const int cnt = ncnt[k];
-    T3<T> pv = zero3<T>(), eta = zero3<T>();
-    // (no index prefetch here: the three gathers per entry leave no registers
-    // for it within 64)
-    for (int q0 = V * tm.t; q0 < cnt; q0 += P * B) {
-        int jj[B][V];
-        load_idx<V, P, B>(p, nbr, k, q0, cnt, jj);
-        float4 xj[B][V], vj[B][V];
-#pragma unroll
-        for (int u = 0; u < B; ++u)
-#pragma unroll
-            for (int c = 0; c < V; ++c) {
-                xj[u][c] = x[jj[u][c]];
-                vj[u][c] = vw[jj[u][c]];
-            }
-#pragma unroll
-        for (int u = 0; u < B; ++u) {
-            const int q = q0 + u * P;
-            if (q >= cnt) break;
-            T3<T> r, g;
-            T w;
-            pair_terms<T, true>(p, xk, pack3(xj[u]), valid_bits<V>(q, cnt), r, w, g);
-            const T3<T> vv = pack3(vj[u]);
-            const T3<T> vji = {vsub(vv.x, bc<T>(vk.x)), vsub(vv.y, bc<T>(vk.y)), vsub(vv.z, bc<T>(vk.z))};
-            pv = {vfma(vji.x, w, pv.x), vfma(vji.y, w, pv.y), vfma(vji.z, w, pv.z)};
-            const T wl = packw(vj[u]);  // |w_j| (k_curl)
-            eta = {vfma(wl, g.x, eta.x), vfma(wl, g.y, eta.y), vfma(wl, g.z, eta.z)};
-        }
-    }
-    const f3 pvs = team_sum3<L>(fold3(pv), tm.mask);
-    f3 etas = team_sum3<L>(fold3(eta), tm.mask);
-    if (tm.t != 0) return -1;
+struct VortIO {
+    const float4* omega;
+    float4 *xout, *vout;
+    const int* perm_in;
+    int* perm_out;
+    float4 *vort_out, *visc_out;
+    int *cell, *ticket, *hist, *err;
+};
+template <typename T> struct VortSums {
+    T3<T> pv, eta;
+};
+template <typename T, int V>
+__device__ __forceinline__ void vort_pair(const KParams& p, const f3& xk, const f3& vk, const float4 (&xj)[V],
+                                          const float4 (&vj)[V], unsigned valid, VortSums<T>& s) {
+    T3<T> r, g;
+    T w;
+    pair_terms<T, true>(p, xk, xj, valid, r, w, g);
+    const T3<T> vji = rdiff3(vj, vk);
+    s.pv = {vfma(vji.x, w, s.pv.x), vfma(vji.y, w, s.pv.y), vfma(vji.z, w, s.pv.z)};
+    const T wl = packw(vj);  // |w_j| (k_curl)
+    s.eta = {vfma(wl, g.x, s.eta.x), vfma(wl, g.y, s.eta.y), vfma(wl, g.z, s.eta.z)};
+}
+// Particle k from its sums; returns its next cell key.
+template <bool DEBUG>
+__device__ __forceinline__ int vort_apply(const KParams& p, int k, const f3& xk, const f3& vk, const f3& pvs, f3 etas,
+                                          const VortIO& o) {
     const float el = __fsqrt_rn(dot_fma(etas, etas));
     if ((double)el > 1e-3) etas = {__fdiv_rn(etas.x, el), __fdiv_rn(etas.y, el), __fdiv_rn(etas.z, el)};
-    const f3 cr = cross3(etas, make3(omega[k]));
+    const f3 cr = cross3(etas, make3(o.omega[k]));
     const f3 fv = {p.vort_eps * cr.x, p.vort_eps * cr.y, p.vort_eps * cr.z};
     const f3 vs = {p.visc_c * pvs.x, p.visc_c * pvs.y, p.visc_c * pvs.z};
     const f3 t = {p.dt * fv.x + vs.x, p.dt * fv.y + vs.y, p.dt * fv.z + vs.z};
     f3 vn = {vk.x + t.x, vk.y + t.y, vk.z + t.z};
-    xout[k] = make_float4(xk.x, xk.y, xk.z, 0.0f);
-    vout[k] = make_float4(vn.x, vn.y, vn.z, 0.0f);
-    perm_out[k] = perm_in[k];
+    o.xout[k] = make_float4(xk.x, xk.y, xk.z, 0.0f);
+    o.vout[k] = make_float4(vn.x, vn.y, vn.z, 0.0f);
+    o.perm_out[k] = o.perm_in[k];
     if (DEBUG) {
-        vort_out[k] = make_float4(fv.x, fv.y, fv.z, 0.0f);
-        visc_out[k] = make_float4(vs.x, vs.y, vs.z, 0.0f);
+        o.vort_out[k] = make_float4(fv.x, fv.y, fv.z, 0.0f);
+        o.visc_out[k] = make_float4(vs.x, vs.y, vs.z, 0.0f);
     }
     // the next substep's prediction and cell key (as k_hash computes them from
     // the state just written)
     const SceneView sc = scene_of(p, k);
     f3 xq = xk;
     predict(p, sc, xq, vn);
-    if (!(isfinite(xq.x) && isfinite(xq.y) && isfinite(xq.z))) atomicOr(err, DEVERR_NONFINITE);
+    if (!(isfinite(xq.x) && isfinite(xq.y) && isfinite(xq.z))) atomicOr(o.err, DEVERR_NONFINITE);
     return cell_key(p, sc, xq);
 }
-
+// the same from the team's sums: the key on its first thread, -1 on the others
 template <bool DEBUG, int L, int V>
-__global__ void __launch_bounds__(256, 4) k_vort(KParams p, int nvb, const float4* __restrict__ x,
-                                              const float4* __restrict__ vw, const float4* __restrict__ omega,
-                                              const int* __restrict__ nbr, const int* __restrict__ ncnt,
-                                              float4* __restrict__ xout, float4* __restrict__ vout,
-                                              const int* __restrict__ perm_in, int* __restrict__ perm_out,
-                                              float4* __restrict__ vort_out, float4* __restrict__ visc_out,
-                                              int* __restrict__ cell, int* __restrict__ ticket, int* __restrict__ hist,
-                                              int* __restrict__ err) {
+__device__ __forceinline__ int vort_store(const KParams& p, const Team<L>& tm, const f3& xk, const f3& vk,
+                                          const VortSums<vec_t<V>>& s, const VortIO& o) {
+    const f3 pvs = team_sum3<L>(fold3(s.pv), tm.mask);
+    const f3 etas = team_sum3<L>(fold3(s.eta), tm.mask);
+    return tm.t == 0 ? vort_apply<DEBUG>(p, tm.k, xk, vk, pvs, etas, o) : -1;
+}
+// the next substep's histogram (every lane of the warp takes part)
+__device__ __forceinline__ void vort_hash(int k, int key, const VortIO& o) {
+    const int tk = warp_histogram(key, o.hist);
+    if (key >= 0) {
+        o.cell[k] = key;
+        o.ticket[k] = tk;
+    }
+}
+template <bool DEBUG, bool ROOMY, int L, int V>
+__device__ __forceinline__ int vort_list(const KParams& p, const Team<L>& tm, const float4* __restrict__ x,
+                                         const float4* __restrict__ vw, const int* __restrict__ nbr,
+                                         const int* __restrict__ ncnt, const VortIO& o) {
+    using T = vec_t<V>;
+    const f3 xk = make3(x[tm.k]), vk = make3(vw[tm.k]);
+    VortSums<T> s = {zero3<T>(), zero3<T>()};
+    for_list<L, V, ROOMY ? 4 : 2, 2>(p, nbr, tm.k, tm.t, ncnt[tm.k], x, vw,
+                             [&](const float4(&xj)[V], const float4(&vj)[V], unsigned valid) {
+                                 vort_pair<T, V>(p, xk, vk, xj, vj, valid, s);
+                             });
+    return vort_store<DEBUG, L, V>(p, tm, xk, vk, s, o);
+}
+
+template <bool DEBUG, bool ROOMY, int L, int V>
+__global__ void __launch_bounds__(256, ROOMY ? ROOMY_BLOCKS : 4) k_vort(KParams p, int nvb, const float4* __restrict__ x,
+                                                 const float4* __restrict__ vw, const int* __restrict__ nbr,
+                                                 const int* __restrict__ ncnt, VortIO o) {
     for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
         const Team<L> tm = team_of<L>(vb);
-        const int k = tm.k;
         int key = -1;
-        if (k < p.n)  // uniform over the team
-            key = vort_one<DEBUG, L, V>(p, tm, k, x, vw, omega, nbr, ncnt, xout, vout, perm_in, perm_out, vort_out,
-                                        visc_out, err);
-        // the next substep's histogram (every lane of the warp takes part)
-        const int tk = warp_histogram(key, hist);
-        if (key >= 0) {
-            cell[k] = key;
-            ticket[k] = tk;
+        if (tm.k < p.n) key = vort_list<DEBUG, ROOMY, L, V>(p, tm, x, vw, nbr, ncnt, o);  // uniform over the team
+        vort_hash(tm.k, key, o);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Small scenes. A thread per particle evaluates its 33 pairs one step after the
+// other, and a pass over a few thousand particles takes that chain whatever their
+// number. Here WIDE = 8 threads share a particle whatever the pair lanes: each takes
+// every eighth entry and leaves what its pairs contribute in shared memory; the
+// sums, whose order the pair lanes define, are then run one chain per thread (lane p
+// of quantity q adds entries p, p + P, ...), the lanes combined as by the butterfly.
+// The values are those of the other kernels bit for bit. 4,096 particles: lambda
+// 5.4 us -> 4.7, correction 5.4 -> 4.6, curl 6.0 -> 3.9, vorticity 8.6 -> 6.1 (four
+// threads per particle were slower than either: 5.9, 5.9, 5.9, 7.9).
+// ---------------------------------------------------------------------------
+constexpr int WIDE = 8;            // threads per particle
+constexpr int WIDE_THREADS = 128;  // per block: 16 particles
+constexpr int WIDE_ENTRIES = 5;    // per thread in flight (a list holds about 33)
+
+// A team of WIDE threads: its particle and its slice of the block's shared memory:
+// `rows` entries of NV float4, padded so that teams of a warp start on different
+// banks.
+struct WideTeam {
+    int k, t;      // slot, thread of the team
+    float4* s;     // the entries' values
+    float* out;    // lane sums, [quantity][8]
+    float* out0;   // those of the block's first team
+};
+template <int NV> __host__ __device__ constexpr int wide_stride(int rows) { return rows * NV + 2; }  // in float4
+__host__ __device__ inline int wide_rows(int max_nbr) { return (max_nbr + 7) & ~7; }
+template <int NV> static int wide_smem(int max_nbr) {
+    return WIDE_THREADS / WIDE * (wide_stride<NV>(wide_rows(max_nbr)) * 16 + 64 * 4);
+}
+
+template <int NV> __device__ __forceinline__ WideTeam wide_team(int max_nbr) {
+    extern __shared__ float4 s_wide[];
+    constexpr int TEAMS = WIDE_THREADS / WIDE;
+    const int team = threadIdx.x / WIDE, stride = wide_stride<NV>(wide_rows(max_nbr));
+    WideTeam w;
+    w.k = blockIdx.x * TEAMS + team;
+    w.t = threadIdx.x & (WIDE - 1);
+    w.s = s_wide + team * stride;
+    w.out0 = reinterpret_cast<float*>(s_wide + TEAMS * stride);
+    w.out = w.out0 + team * 64;
+    return w;
+}
+
+// eval(xj, vj, dst) for every entry of the team's list that this thread takes: dst
+// receives the entry's NV float4.
+template <int NV, int NA, typename F>
+__device__ __forceinline__ void wide_pairs(const KParams& p, const WideTeam& w, int cnt, const int* __restrict__ nbr,
+                                           const float4* __restrict__ a, const float4* __restrict__ b, F&& eval) {
+    constexpr int U = WIDE_ENTRIES;
+    for (int q0 = w.t; q0 < cnt; q0 += WIDE * U) {
+        int j[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int q = q0 + WIDE * u;
+            j[u] = q < cnt ? nbr[(size_t)q * p.stride + w.k] : -1;
         }
+        float4 xj[U][1], vj[U][1];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (j[u] >= 0) {
+                xj[u][0] = a[j[u]];
+                if (NA == 2) vj[u][0] = b[j[u]];
+            }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (j[u] >= 0) eval(xj[u], vj[u], w.s + (q0 + WIDE * u) * NV);
+    }
+    __syncwarp();
+}
+
+// Quantity q of pair lane `lane` summed by add(q, acc, values of the entry), chains
+// dealt to the team's threads; NQ quantities. Ends with a block barrier: the
+// particles' epilogues then run on the block's first threads, one each, instead of
+// on one thread of every team.
+template <int NV, int NQ, typename F>
+__device__ __forceinline__ void wide_sums(const WideTeam& w, int cnt, int P, F&& add) {
+    for (int c = w.t; c < NQ * P; c += WIDE) {
+        const int q = c / P, lane = c - q * P;
+        float acc = 0.0f;
+        const float4* e = w.s + lane * NV;
+#pragma unroll 4
+        for (int i = lane; i < cnt; i += P, e += P * NV) acc = add(q, acc, reinterpret_cast<const float*>(e));
+        w.out[q * 8 + lane] = acc;
+    }
+    __syncthreads();
+}
+// the butterfly over P lane sums
+__device__ __forceinline__ float wide_total(const float* s, int P) {
+    float v = s[0];
+    if (P >= 2) v = s[0] + s[1];
+    if (P >= 4) v = v + (s[2] + s[3]);
+    if (P >= 8) v = v + ((s[4] + s[5]) + (s[6] + s[7]));
+    return v;
+}
+__device__ __forceinline__ f3 wide_total3(const float* s, int P) {
+    return {wide_total(s, P), wide_total(s + 8, P), wide_total(s + 16, P)};
+}
+// the particle whose epilogue this thread runs, -1 for none, and its sums
+__device__ __forceinline__ int wide_mine(const KParams& p, const WideTeam& w, const float*& sums) {
+    constexpr int TEAMS = WIDE_THREADS / WIDE;
+    const int k = blockIdx.x * TEAMS + threadIdx.x;
+    sums = w.out0 + threadIdx.x * 64;
+    return threadIdx.x < TEAMS && k < p.n ? k : -1;
+}
+
+template <bool DEBUG>
+__global__ void __launch_bounds__(WIDE_THREADS) k_lambda_wide(KParams p, const float4* __restrict__ x,
+                                                              const int* __restrict__ nbr,
+                                                              const int* __restrict__ ncnt, float4* __restrict__ xl,
+                                                              float* __restrict__ rho_out, IterCtl ctl) {
+    if (ctl.done && *ctl.done) return;
+    const WideTeam w = wide_team<1>(p.max_nbr);
+    const bool on = w.k < p.n;
+    const int cnt = on ? ncnt[w.k] : 0;
+    const f3 xk = on ? make3(x[w.k]) : f3{0.0f, 0.0f, 0.0f};
+    wide_pairs<1, 1>(p, w, cnt, nbr, x, x, [&](const float4(&xj)[1], const float4(&)[1], float4* dst) {
+        T3<float> r, g;
+        float wt;
+        pair_terms<float, true>(p, xk, xj, 1u, r, wt, g);
+        *dst = make_float4(g.x, g.y, g.z, wt);
+    });
+    // gradient sums, density, sum of squared gradients
+    wide_sums<1, 5>(w, cnt, p.lanes, [&](int q, float acc, const float* v) {
+        if (q < 4) return acc + v[q];
+        acc = __fmaf_rn(v[0], v[0], acc);
+        acc = __fmaf_rn(v[1], v[1], acc);
+        return __fmaf_rn(v[2], v[2], acc);
+    });
+    float err = 0.0f;
+    const float* s;
+    const int k = wide_mine(p, w, s);
+    if (k >= 0) {
+        const f3 q = make3(x[k]);
+        float rhos = wide_total(s + 24, p.lanes);
+        const float lam = lambda_tail(p, k, q, rhos, wide_total(s + 32, p.lanes), wide_total3(s, p.lanes), err);
+        xl[k] = make_float4(q.x, q.y, q.z, lam);
+        if (ctl.lam_acc) ctl.lam_acc[k] += lam;
+        if (DEBUG) rho_out[k] = rhos;
+    }
+    if (ctl.max_bits) {
+        const int sl = ctl.cur_slot();
+        block_error_reduce(err, err, ctl.max_bits + sl, ctl.sum + sl);
+    }
+}
+
+template <bool DEBUG, bool N4>
+__global__ void __launch_bounds__(WIDE_THREADS) k_dp_wide(KParams p, const float4* __restrict__ xl,
+                                                          const int* __restrict__ nbr, const int* __restrict__ ncnt,
+                                                          DpOut o, IterCtl ctl) {
+    if (dp_skip(ctl)) return;
+    const WideTeam w = wide_team<1>(p.max_nbr);
+    const bool on = w.k < p.n;
+    const int cnt = on ? ncnt[w.k] : 0;
+    const float4 xk4 = on ? xl[w.k] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const f3 xk = make3(xk4);
+    wide_pairs<1, 1>(p, w, cnt, nbr, xl, xl, [&](const float4(&xj)[1], const float4(&)[1], float4* dst) {
+        T3<float> r, g;
+        float wt;
+        pair_terms<float, true>(p, xk, xj, 1u, r, wt, g);
+        *dst = make_float4(g.x, g.y, g.z, dp_weight<N4>(p, addw(xk4.w, xj), wt));
+    });
+    wide_sums<1, 3>(w, cnt, p.lanes, [&](int q, float acc, const float* v) { return __fmaf_rn(v[3], v[q], acc); });
+    const float* s;
+    const int k = wide_mine(p, w, s);
+    if (k >= 0) {
+        const float4 q = xl[k];
+        dp_apply<DEBUG>(p, k, make3(q), q.w, wide_total3(s, p.lanes), o);
+    }
+}
+
+__global__ void __launch_bounds__(WIDE_THREADS) k_curl_wide(KParams p, const float4* __restrict__ x,
+                                                            const float4* __restrict__ v, const int* __restrict__ nbr,
+                                                            const int* __restrict__ ncnt, float4* __restrict__ omega,
+                                                            float4* __restrict__ vw) {
+    const WideTeam w = wide_team<1>(p.max_nbr);
+    const bool on = w.k < p.n;
+    const int cnt = on ? ncnt[w.k] : 0;
+    const f3 xk = on ? make3(x[w.k]) : f3{0.0f, 0.0f, 0.0f}, vk = on ? make3(v[w.k]) : f3{0.0f, 0.0f, 0.0f};
+    wide_pairs<1, 2>(p, w, cnt, nbr, x, v, [&](const float4(&xj)[1], const float4(&vj)[1], float4* dst) {
+        T3<float> r, g;
+        float wt;
+        pair_terms<float, false>(p, xk, xj, 1u, r, wt, g);
+        const T3<float> c = cross3v(rdiff3(vj, vk), g);
+        *dst = make_float4(c.x, c.y, c.z, 0.0f);
+    });
+    wide_sums<1, 3>(w, cnt, p.lanes, [&](int q, float acc, const float* s) { return acc + s[q]; });
+    const float* s;
+    const int k = wide_mine(p, w, s);
+    if (k >= 0) curl_apply(k, make3(v[k]), wide_total3(s, p.lanes), omega, vw);
+}
+
+template <bool DEBUG>
+__global__ void __launch_bounds__(WIDE_THREADS) k_vort_wide(KParams p, const float4* __restrict__ x,
+                                                            const float4* __restrict__ vw,
+                                                            const int* __restrict__ nbr, const int* __restrict__ ncnt,
+                                                            VortIO o) {
+    const WideTeam w = wide_team<2>(p.max_nbr);
+    const bool on = w.k < p.n;
+    const int cnt = on ? ncnt[w.k] : 0;
+    const f3 xk = on ? make3(x[w.k]) : f3{0.0f, 0.0f, 0.0f}, vk = on ? make3(vw[w.k]) : f3{0.0f, 0.0f, 0.0f};
+    wide_pairs<2, 2>(p, w, cnt, nbr, x, vw, [&](const float4(&xj)[1], const float4(&vj)[1], float4* dst) {
+        T3<float> r, g;
+        float wt;
+        pair_terms<float, true>(p, xk, xj, 1u, r, wt, g);
+        const T3<float> d = rdiff3(vj, vk);
+        dst[0] = make_float4(d.x, d.y, d.z, wt);
+        dst[1] = make_float4(g.x, g.y, g.z, packw(vj));
+    });
+    // sum of (v_j - v_i) W, then of |w_j| grad W
+    wide_sums<2, 6>(w, cnt, p.lanes, [&](int q, float acc, const float* s) {
+        return q < 3 ? __fmaf_rn(s[q], s[3], acc) : __fmaf_rn(s[7], s[q + 1], acc);
+    });
+    if (threadIdx.x < 32) {  // the 16 particles: all on the first warp
+        const float* s;
+        const int k = wide_mine(p, w, s);
+        int key = -1;
+        if (k >= 0)
+            key = vort_apply<DEBUG>(p, k, make3(x[k]), make3(vw[k]), wide_total3(s, p.lanes),
+                                    wide_total3(s + 24, p.lanes), o);
+        vort_hash(k, key, o);
     }
 }
 
@@ -869,23 +1145,40 @@ __global__ void __launch_bounds__(256, 4) k_vort(KParams p, int nvb, const float
 // blocks for n particles with L threads each
 static inline int team_blocks(int n, int L, int bs) { return (int)(((long long)n * L + bs - 1) / bs); }
 
+static int sm_count() {
+    static int sms = 0;
+    if (!sms) {
+        int dev = 0, v = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+        sms = v > 0 ? v : 1;
+    }
+    return sms;
+}
 // Grid of a neighbour pass over nvb tiles: nvb blocks, or with p.persistent the
 // blocks that are resident at once (SMs x blocks per SM at this block size), each
 // striding over the tiles.
 template <typename K> static int pass_grid(const KParams& p, K kernel, int nvb) {
     if (!p.persistent) return nvb;
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (sms <= 0) sms = 1;
-    }
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, p.block, 0) != cudaSuccess || per_sm <= 0)
         per_sm = 1;
-    const long long g = (long long)per_sm * sms;
+    const long long g = (long long)per_sm * sm_count();
     return (int)(g < nvb ? g : nvb);
+}
+// All blocks of a pass with L threads per particle resident at ROOMY_BLOCKS x 256
+// threads per SM.
+static bool roomy(const KParams& p, int L) { return (long long)p.n * L <= (long long)sm_count() * ROOMY_BLOCKS * 256; }
+
+using Yes = std::true_type;
+using No = std::false_type;
+// Calls f with the flags as compile-time constants.
+template <typename F> static void with_flag(bool a, F&& f) {
+    if (a) f(Yes{});
+    else f(No{});
+}
+template <typename F> static void with_flags(bool a, bool b, F&& f) {
+    with_flag(a, [&](auto x) { with_flag(b, [&](auto y) { f(x, y); }); });
 }
 
 // Calls f with (L, V) of pair_lanes as compile-time constants.
@@ -901,27 +1194,57 @@ template <typename F> void with_lanes(int lanes, F&& f) {
     }
 }
 
+// The wide kernels run scenes of up to four of their blocks per SM, with one or two
+// pair lanes: substeps of 4,096 particles take 69 us with them and 78 without, of
+// 13,824 the same, and beyond that the flat kernels fill the device with less work
+// (four and eight lanes already spread a particle over two and four threads).
+static bool wide(const KParams& p) {
+    return !p.persistent && p.lanes <= 2 && p.n <= sm_count() * 4 * (WIDE_THREADS / WIDE);
+}
+template <int NV, typename K, typename... A>
+static void launch_wide(const KParams& p, K kernel, cudaStream_t st, A... args) {
+    const int smem = wide_smem<NV>(p.max_nbr);  // at most 69 KB (127 entries of two float4)
+    if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const int per = WIDE_THREADS / WIDE;
+    kernel<<<(p.n + per - 1) / per, WIDE_THREADS, smem, st>>>(p, args...);
+}
+
 void launch_lambda(const KParams& p, bool debug, const float4* x, const int* nbr, const int* ncnt, float4* xl,
-                   float* rho, const IterCtl& ctl, cudaStream_t st) {
+                  float* rho, const IterCtl& ctl, cudaStream_t st) {
+    if (wide(p)) {
+        with_flag(debug, [&](auto d) {
+            launch_wide<1>(p, k_lambda_wide<decltype(d)::value>, st, x, nbr, ncnt, xl, rho, ctl);
+        });
+        return;
+    }
     with_lanes(p.lanes, [&](auto c) {
         constexpr int L = decltype(c)::L, V = decltype(c)::V;
         const int b = team_blocks(p.n, L, p.block);
-        if (debug) k_lambda<true, L, V><<<pass_grid(p, k_lambda<true, L, V>, b), p.block, 0, st>>>(p, b, x, nbr, ncnt, xl, rho, ctl);
-        else k_lambda<false, L, V><<<pass_grid(p, k_lambda<false, L, V>, b), p.block, 0, st>>>(p, b, x, nbr, ncnt, xl, rho, ctl);
+        with_flags(debug, roomy(p, L), [&](auto d, auto r) {
+            auto* k = k_lambda<decltype(d)::value, decltype(r)::value, L, V>;
+            k<<<pass_grid(p, k, b), p.block, 0, st>>>(p, b, x, nbr, ncnt, xl, rho, ctl);
+        });
     });
 }
 
 void launch_dp(const KParams& p, bool debug, const float4* xl, const int* nbr, const int* ncnt, const float4* xold,
                float4* xout, float4* vout, float4* dp, const IterCtl& ctl, cudaStream_t st) {
+    const DpOut o{xold, xout, vout, dp};
+    if (wide(p)) {
+        with_flags(debug, p.n_int == 4, [&](auto d, auto n4) {
+            launch_wide<1>(p, k_dp_wide<decltype(d)::value, decltype(n4)::value>, st, xl, nbr, ncnt, o, ctl);
+        });
+        return;
+    }
     with_lanes(p.lanes, [&](auto c) {
         constexpr int L = decltype(c)::L, V = decltype(c)::V;
         const int b = team_blocks(p.n, L, p.block);
-        if (debug)
-            k_dp<true, L, V><<<pass_grid(p, k_dp<true, L, V>, b), p.block, 0, st>>>(p, b, xl, nbr, ncnt, xold, xout,
-                                                                                     vout, dp, ctl);
-        else
-            k_dp<false, L, V><<<pass_grid(p, k_dp<false, L, V>, b), p.block, 0, st>>>(p, b, xl, nbr, ncnt, xold, xout,
-                                                                                       vout, dp, ctl);
+        with_flags(debug, p.n_int == 4, [&](auto d, auto n4) {
+            with_flag(roomy(p, L), [&](auto r) {
+                auto* k = k_dp<decltype(d)::value, decltype(n4)::value, decltype(r)::value, L, V>;
+                k<<<pass_grid(p, k, b), p.block, 0, st>>>(p, b, xl, nbr, ncnt, o, ctl);
+            });
+        });
     });
 }
 
@@ -966,26 +1289,36 @@ int launch_features_warm(const KParams& p, const float4* x, const float4* v, con
 }
 
 void launch_curl(const KParams& p, const float4* x, const float4* v, const int* nbr, const int* ncnt, float4* omega,
-                 float4* vw, cudaStream_t st) {
+                float4* vw, cudaStream_t st) {
+    if (wide(p)) {
+        launch_wide<1>(p, k_curl_wide, st, x, v, nbr, ncnt, omega, vw);
+        return;
+    }
     with_lanes(p.lanes, [&](auto c) {
         constexpr int L = decltype(c)::L, V = decltype(c)::V;
         const int b = team_blocks(p.n, L, p.block);
-        k_curl<L, V><<<pass_grid(p, k_curl<L, V>, b), p.block, 0, st>>>(p, b, x, v, nbr, ncnt, omega, vw);
+        with_flag(roomy(p, L), [&](auto r) {
+            auto* k = k_curl<decltype(r)::value, L, V>;
+            k<<<pass_grid(p, k, b), p.block, 0, st>>>(p, b, x, v, nbr, ncnt, omega, vw);
+        });
     });
 }
 
 void launch_vort(const KParams& p, bool debug, const float4* x, const float4* vw, const float4* omega, const int* nbr,
-                 const int* ncnt, float4* xout, float4* vout, const int* perm_in, int* perm_out, float4* vort,
-                 float4* visc, int* cell, int* ticket, int* hist, int* err, cudaStream_t st) {
+                const int* ncnt, float4* xout, float4* vout, const int* perm_in, int* perm_out, float4* vort,
+                float4* visc, int* cell, int* ticket, int* hist, int* err, cudaStream_t st) {
+    const VortIO o{omega, xout, vout, perm_in, perm_out, vort, visc, cell, ticket, hist, err};
+    if (wide(p)) {
+        with_flag(debug, [&](auto d) { launch_wide<2>(p, k_vort_wide<decltype(d)::value>, st, x, vw, nbr, ncnt, o); });
+        return;
+    }
     with_lanes(p.lanes, [&](auto c) {
         constexpr int L = decltype(c)::L, V = decltype(c)::V;
         const int b = team_blocks(p.n, L, p.block);
-        if (debug)
-            k_vort<true, L, V><<<pass_grid(p, k_vort<true, L, V>, b), p.block, 0, st>>>(
-                p, b, x, vw, omega, nbr, ncnt, xout, vout, perm_in, perm_out, vort, visc, cell, ticket, hist, err);
-        else
-            k_vort<false, L, V><<<pass_grid(p, k_vort<false, L, V>, b), p.block, 0, st>>>(
-                p, b, x, vw, omega, nbr, ncnt, xout, vout, perm_in, perm_out, vort, visc, cell, ticket, hist, err);
+        with_flags(debug, roomy(p, L), [&](auto d, auto r) {
+            auto* k = k_vort<decltype(d)::value, decltype(r)::value, L, V>;
+            k<<<pass_grid(p, k, b), p.block, 0, st>>>(p, b, x, vw, nbr, ncnt, o);
+        });
     });
 }
 
