@@ -67,6 +67,8 @@ namespace {
 constexpr int kMaxIter = 64;
 constexpr int kSlots = kMaxIter + 2;
 
+constexpr int kMaxPad = 16;  // largest KParams::pad
+
 struct DevStats {
     unsigned long long max_bits[kSlots];
     double sum[kSlots];
@@ -200,6 +202,9 @@ KParams make_kparams(const pbf_solver& s) {
     k.persistent = e.persistent;
     k.max_nbr = e.max_neighbors;
     k.stride = s.stride;
+    // four entries per thread and batch, one, two or four threads per particle
+    k.pad = k.lanes <= 2 ? 4 : k.lanes == 4 ? 8 : kMaxPad;
+    k.pad_slot = s.capacity;
     k.cell_order = e.cell_order;
     k.flags = e.flags;
     k.poly6_c64 = 315.0 / (64.0 * M_PI * std::pow((double)p.h, 9));
@@ -724,10 +729,12 @@ int create_common(const pbf_solver_parameter* para, int nscenes, const pbf_scene
             return rc;                     \
         }                                  \
     } while (0)
-    AL(s->Sx, n); AL(s->Sv, n); AL(s->Px, n + 1); AL(s->Pv, n); AL(s->Pxold, n); AL(s->Q, n); AL(s->omega, n); AL(s->vw, n);
+    AL(s->Sx, n); AL(s->Sv, n); AL(s->Px, n + 1); AL(s->Pv, n + 1); AL(s->Pxold, n); AL(s->Q, n + 1); AL(s->omega, n); AL(s->vw, n + 1);
     AL(s->Sperm, n); AL(s->Pperm, n); AL(s->cell, n); AL(s->ticket, n); AL(s->tmp, n); AL(s->cell_sorted, n);
     AL(s->ncnt, n);
-    AL(s->nbr, (size_t)ext->max_neighbors * s->stride);
+    // (rows for the longest list padded to whole batches; slot n of the gathered arrays
+    // is the padding slot)
+    AL(s->nbr, (size_t)((ext->max_neighbors + kMaxPad - 1) / kMaxPad * kMaxPad) * s->stride);
     AL(s->cell_start, (size_t)s->nkeys + 1);
     AL(s->lam_acc, n); AL(s->lam_prev_sorted, n); AL(s->lam0, n);
     AL(s->feat, n * (size_t)MLP_IN);
@@ -768,6 +775,12 @@ int create_common(const pbf_solver_parameter* para, int nscenes, const pbf_scene
     if (e == cudaSuccess) e = cudaMemset(s->dstats, 0, sizeof(DevStats));
     if (e == cudaSuccess) e = cudaMemset(s->lam_acc, 0, sizeof(float) * n);
     if (e == cudaSuccess) e = cudaMemset(s->lam0, 0, sizeof(float) * n);
+    if (e == cudaSuccess) {
+        launch_fill_pad(s->Px + n, s->Q + n, s->Pv + n, s->vw + n, nullptr);
+        e = cudaGetLastError();
+    }
+    // a caller's non-blocking stream must find the set-up done
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->cap_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->body_stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) {

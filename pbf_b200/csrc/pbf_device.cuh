@@ -57,6 +57,10 @@ struct SceneView {
     int pcount;
 };
 
+// Where the padding slot lies: farther than h from every particle, with a squared
+// distance that is still finite. Its velocity, lambda and vorticity are zero.
+constexpr float PAD_POSITION = 1e18f;
+
 struct KParams {
     // kernel constants, all computed on the host (pbf_capi.cu: make_kparams)
     float h, h2, cell, inv_cell, poly6_c, spiky_c, inv_wdq, nk, scorr_scale, n_exp;
@@ -72,6 +76,8 @@ struct KParams {
     int block;      // threads per block of the neighbour passes
     int lanes;      // pair lanes per particle of the neighbour passes (1, 2, 4, 8)
     int max_nbr;    // neighbour cap (reference MAX_NEIGHBOR = 63)
+    int pad;        // lists are padded to a multiple of this (a batch of every thread of a team)
+    int pad_slot;   // with this slot of the position, velocity and lambda arrays (PAD_POSITION)
     int stride;     // neighbour list stride (slot-major layout: nbr[q * stride + k])
     int cell_order; // 0 ascending, 1 descending within a cell
     int n_int;      // s_corr exponent when a small integer, else 0

@@ -537,6 +537,7 @@ __device__ __forceinline__ void neighbors_one(const KParams& p, int k, const flo
         }
     }
     ncnt[k] = c;
+    for (; c % p.pad != 0; ++c) list[(size_t)c * p.stride] = p.pad_slot;
 }
 
 // nvb tiles of blockDim.x slots; the grid strides over them (a grid of nvb
@@ -653,7 +654,12 @@ __global__ void __launch_bounds__(SEARCH_WIDE_THREADS) k_neighbors_wide(KParams 
                 }
         }
     }
-    if (on && t == SEARCH_WIDE - 1) ncnt[k] = min(incl, cap);
+    const int total = min(__shfl_sync(0xffffffffu, incl, SEARCH_WIDE - 1, SEARCH_WIDE), cap);
+    if (on) {
+        if (t == 0) ncnt[k] = total;
+        const int end = (total + p.pad - 1) / p.pad * p.pad;
+        for (int q = total + t; q < end; q += SEARCH_WIDE) nbr[(size_t)q * p.stride + k] = p.pad_slot;
+    }
 }
 
 // Copies features and total lambda of the given slots (training rows).
@@ -836,6 +842,11 @@ __global__ void __launch_bounds__(256) k_to_aos(int n, const float4* __restrict_
         out2[3 * o + 1] = r.y;
         out2[3 * o + 2] = r.z;
     }
+}
+
+__global__ void k_fill_pad(float4* x, float4* q, float4* v, float4* vw) {
+    *x = *q = make_float4(PAD_POSITION, PAD_POSITION, PAD_POSITION, 0.0f);
+    *v = *vw = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 }
 
 __global__ void k_copy4(int n, const float4* __restrict__ a, float4* __restrict__ b) {
@@ -1072,6 +1083,10 @@ void launch_sorted_state(int n, const float4* x, const float4* v, const int* per
                          cudaStream_t st) {
     k_sorted_state<<<blocks_for(n, 256), 256, 0, st>>>(n, x, v, perm, cell_sorted, cell_start, pos, vel, ids, key,
                                                        rank);
+}
+
+void launch_fill_pad(float4* x, float4* q, float4* v, float4* vw, cudaStream_t st) {
+    k_fill_pad<<<1, 1, 0, st>>>(x, q, v, vw);
 }
 
 void launch_copy4(int n, const float4* a, float4* b, cudaStream_t st) {

@@ -73,6 +73,9 @@ void launch_upload(const KParams& p, const float* pos, const float* vel, float4*
 // Slot order to original order: a to out and (when out2 is not null) a2 to out2.
 void launch_to_aos(int n, const float4* a, const float4* a2, const int* perm, float* out, float* out2, int* err,
                    cudaStream_t st);
+// The padding slot's position (x, and q with lambda 0) and velocity (v, and vw with
+// vorticity 0).
+void launch_fill_pad(float4* x, float4* q, float4* v, float4* vw, cudaStream_t st);
 void launch_copy4(int n, const float4* a, float4* b, cudaStream_t st);
 void launch_sorted_state(int n, const float4* x, const float4* v, const int* perm, const int* cell_sorted,
                          const int* cell_start, float* pos, float* vel, int* ids, int* key, int* rank,

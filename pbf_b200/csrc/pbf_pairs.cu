@@ -19,9 +19,11 @@
 // ((s0 + s1) + (s2 + s3)) + ... on every lane. pair_lanes = P selects
 // (L, V): 1 = (1, 1), 2 = (1, 2), 4 = (2, 2), 8 = (4, 2).
 //
-// A padding component (an entry past the end of the list) contributes +0 to
-// every sum, which leaves the sum unchanged: no accumulator is ever -0 (they
-// start at +0, and in round-to-nearest x + (-x) = +0 and +0 + (-0) = +0).
+// The search pads every list to whole batches with the padding slot (KParams::pad_slot,
+// a position no particle comes near). A padding entry contributes +0 or -0 to every
+// sum, which leaves the sum unchanged: no accumulator is ever -0 (they start at +0,
+// and in round-to-nearest x + (-x) = +0 and +0 + (-0) = +0). So no entry is tested
+// for the end of its list.
 #include "pbf_kernels.h"
 #include "pbf_mlp.h"
 #include "pbf_mlp_dev.cuh"
@@ -32,16 +34,20 @@
 
 namespace pbf {
 
-// bit v set: component v greater than / less than s
-__device__ __forceinline__ unsigned gt_mask(float a, float s) { return a > s ? 1u : 0u; }
-__device__ __forceinline__ unsigned gt_mask(float2 a, float s) { return (a.x > s ? 1u : 0u) | (a.y > s ? 2u : 0u); }
-__device__ __forceinline__ unsigned lt_mask(float a, float s) { return a < s ? 1u : 0u; }
-__device__ __forceinline__ unsigned lt_mask(float2 a, float s) { return (a.x < s ? 1u : 0u) | (a.y < s ? 2u : 0u); }
-// components whose bit in keep is clear become +0
-__device__ __forceinline__ float keep_only(float a, unsigned keep) { return (keep & 1u) ? a : 0.0f; }
-__device__ __forceinline__ float2 keep_only(float2 a, unsigned keep) {
-    return make_float2((keep & 1u) ? a.x : 0.0f, (keep & 2u) ? a.y : 0.0f);
-}
+// one truth value per component, and the components where it holds (+0 elsewhere)
+struct bool2v {
+    bool x, y;
+};
+__device__ __forceinline__ float keep_only(float a, bool k) { return k ? a : 0.0f; }
+__device__ __forceinline__ float2 keep_only(float2 a, bool2v k) { return make_float2(k.x ? a.x : 0.0f, k.y ? a.y : 0.0f); }
+// lo <= a <= hi
+__device__ __forceinline__ bool within(float a, float lo, float hi) { return !(a < lo) && !(a > hi); }
+__device__ __forceinline__ bool2v within(float2 a, float lo, float hi) { return {within(a.x, lo, hi), within(a.y, lo, hi)}; }
+__device__ __forceinline__ bool below(float a, float s, bool valid) { return a < s && valid; }
+__device__ __forceinline__ bool2v below(float2 a, float s, bool2v valid) { return {a.x < s && valid.x, a.y < s && valid.y}; }
+// which components are entries of a list with `left` of them left
+__device__ __forceinline__ bool entries_left(float, int left) { return left > 0; }
+__device__ __forceinline__ bool2v entries_left(float2, int left) { return {left > 0, left > 1}; }
 // the first butterfly step: the two lanes of a thread
 __device__ __forceinline__ float fold(float a) { return a; }
 __device__ __forceinline__ float fold(float2 a) { return a.x + a.y; }
@@ -116,18 +122,18 @@ template <int V> using vec_t = typename std::conditional<V == 1, float, float2>:
 
 // r = x_k - x_j, |r|^2 = fma(z, z, fma(y, y, x*x)), Wpoly6 (when NEED_W) and the
 // spiky gradient of V pairs, exactly as w_poly6 / grad_spiky (pbf_device.cuh)
-// evaluate one pair; components outside `valid` give w = +0 and g = +0 or -0.
+// evaluate one pair.
 // Every difference a - b is fma(b, -1, a), which rounds the same exact value
 // once (signed zeros included), and the rsqrt comes negated (ny = -y), so no
 // operand needs a negation of its own: h - |r| = fma(|r|^2, ny, h), |r| > h is
 // |r|^2 ny < -h, and ((c d) d) y = ((-c d) d) ny. The poly6 cutoff |r|^2 > h^2
 // is max(h^2 - |r|^2, +0) (the difference is negative exactly when the same
-// rounded |r|^2 exceeds h^2, and c (+0)^3 = +0). A padding entry is the particle
-// itself (r = +0, |r| below rmin), which the gradient's cutoff already drops;
-// only its density weight needs `valid`.
+// rounded |r|^2 exceeds h^2, and c (+0)^3 = +0). A padding entry is the padding
+// slot, far from every particle: its weight is c (+0)^3 and the cutoff drops its
+// gradient, so it gives w = +0 and g = +0 or -0.
 template <typename T, bool NEED_W, int V>
-__device__ __forceinline__ void pair_terms(const KParams& p, const f3& xk, const float4 (&xj)[V], unsigned valid,
-                                           T3<T>& r, T& w, T3<T>& g) {
+__device__ __forceinline__ void pair_terms(const KParams& p, const f3& xk, const float4 (&xj)[V], T3<T>& r, T& w,
+                                           T3<T>& g) {
     const T m1 = bc<T>(-1.0f);
     r = diff3(xk, xj);
     const T r2 = vfma(r.z, r.z, vfma(r.y, r.y, vmul(r.x, r.x)));
@@ -136,16 +142,15 @@ __device__ __forceinline__ void pair_terms(const KParams& p, const f3& xk, const
         // c t^3 as fma(c, t^3, +0), the same value (c t^3 is never -0): the density
         // sum adds w, and a packed product whose only use is an addition may be fused
         // into it by the code generator
-        w = keep_only(vfma(bc<T>(p.poly6_c), vmul(vmul(t, t), t), bc<T>(0.0f)), valid);
+        w = vfma(bc<T>(p.poly6_c), vmul(vmul(t, t), t), bc<T>(0.0f));
     }
     const T ny = vrsqrt_neg(vmax(r2, 1e-30f));
     const T nrl = vmul(r2, ny);               // -|r| for the cutoff
     const T d = vfma(r2, ny, bc<T>(p.h));      // h - |r|
     const T s = vmul(vmul(vmul(bc<T>(-p.spiky_c), d), d), ny);
-    const unsigned keep = ~(lt_mask(nrl, -p.h) | gt_mask(nrl, -p.rmin));
     // the mask on the magnitude: a dropped pair gives a gradient of +0 or -0,
     // which leaves every sum it enters unchanged (no accumulator is ever -0)
-    const T sk = keep_only(s, keep);
+    const T sk = keep_only(s, within(nrl, -p.h, -p.rmin));
     g = {vmul(sk, r.x), vmul(sk, r.y), vmul(sk, r.z)};
 }
 
@@ -201,30 +206,20 @@ template <int L> __device__ __forceinline__ f3 team_sum3(f3 v, unsigned mask) {
     return {team_sum<L>(v.x, mask), team_sum<L>(v.y, mask), team_sum<L>(v.z, mask)};
 }
 
-// Entries q0 + u P + v (u < B, v < V) of slot k's list; slot k itself past the
-// end (its data is then masked). All index loads of a batch are issued before
-// the gathers that depend on them.
+// Entries q0 + u P + v (u < B, v < V) of slot k's (padded) list. All index loads of
+// a batch are issued before the gathers that depend on them.
 template <int V, int P, int B>
-__device__ __forceinline__ void load_idx(const KParams& p, const int* __restrict__ nbr, int k, int q0, int cnt,
+__device__ __forceinline__ void load_idx(const KParams& p, const int* __restrict__ nbr, int k, int q0,
                                          int (&jj)[B][V]) {
 #pragma unroll
     for (int u = 0; u < B; ++u)
 #pragma unroll
-        for (int v = 0; v < V; ++v) {
-            const int q = q0 + u * P + v;
-            jj[u][v] = q < cnt ? nbr[(size_t)q * p.stride + k] : k;
-        }
-}
-
-// bit v: entry q + v exists
-template <int V> __device__ __forceinline__ unsigned valid_bits(int q, int cnt) {
-    return (q < cnt ? 1u : 0u) | (V == 2 && q + 1 < cnt ? 2u : 0u);
+        for (int v = 0; v < V; ++v) jj[u][v] = nbr[(size_t)(q0 + u * P + v) * p.stride + k];
 }
 
 // How a pass's inner loop is laid out. A batch of E entries per thread has its
-// gathers issued together and no branch inside: the entries past the end of a list
-// are the particle itself and add zeros, and the pairs of a batch overlap (a test
-// per entry kept them apart: a step then took the whole latency of its arithmetic;
+// gathers issued together and no branch inside, so the pairs of a batch overlap (a
+// test per entry for the end of the list kept them apart: a step then took the whole latency of its arithmetic;
 // 1 M particles, lambda: 81.6 us with the test, 68.9 without; 32,768 particles: 8.1
 // and 6.2).
 //   full device: four entries in the one-array passes, two in the two-array ones,
@@ -236,7 +231,7 @@ template <int V> __device__ __forceinline__ unsigned valid_bits(int q, int cnt) 
 //     5.8, curl 10.4 -> 6.7, vorticity 11 -> 8.3).
 constexpr int ROOMY_BLOCKS = 3;
 
-// body(xj, vj, valid) for the neighbours of slot k that thread t of its team
+// body(xj, vj) for the neighbours of slot k that thread t of its team
 // takes, gathered from NA arrays through the list of slots, E entries per batch; the
 // next batch's indices load while a batch computes.
 template <int L, int V, int E, int NA, typename F>
@@ -244,8 +239,9 @@ __device__ __forceinline__ void for_list(const KParams& p, const int* __restrict
                                          const float4* __restrict__ a, const float4* __restrict__ b, F&& body) {
     constexpr int P = L * V, B = E / V;
     int jj[B][V];
-    load_idx<V, P, B>(p, nbr, k, V * t, cnt, jj);
-    for (int q0 = V * t; q0 < cnt; q0 += P * B) {
+    if (cnt > 0) load_idx<V, P, B>(p, nbr, k, V * t, jj);
+    // (every thread of a team runs the same batches: the lists are padded for it)
+    for (int q0 = 0; q0 < cnt; q0 += P * B) {
         float4 xj[B][V], vj[B][V];
 #pragma unroll
         for (int u = 0; u < B; ++u)
@@ -254,12 +250,9 @@ __device__ __forceinline__ void for_list(const KParams& p, const int* __restrict
                 xj[u][c] = a[jj[u][c]];
                 if (NA == 2) vj[u][c] = b[jj[u][c]];
             }
-        load_idx<V, P, B>(p, nbr, k, q0 + P * B, cnt, jj);
+        if (q0 + P * B < cnt) load_idx<V, P, B>(p, nbr, k, q0 + P * B + V * t, jj);
 #pragma unroll
-        for (int u = 0; u < B; ++u) {
-            const int q = q0 + u * P;
-            body(xj[u], vj[u], valid_bits<V>(q, cnt));
-        }
+        for (int u = 0; u < B; ++u) body(xj[u], vj[u]);
     }
 }
 
@@ -321,11 +314,11 @@ template <typename T> __device__ __forceinline__ LambdaSums<T> lambda_zero() {
     return {bc<T>(0.0f), bc<T>(0.0f), zero3<T>()};
 }
 template <typename T, int V>
-__device__ __forceinline__ void lambda_pair(const KParams& p, const f3& xk, const float4 (&xj)[V], unsigned valid,
+__device__ __forceinline__ void lambda_pair(const KParams& p, const f3& xk, const float4 (&xj)[V],
                                             LambdaSums<T>& s) {
     T3<T> r, g;
     T w;
-    pair_terms<T, true>(p, xk, xj, valid, r, w, g);
+    pair_terms<T, true>(p, xk, xj, r, w, g);
     s.rho = vadd(s.rho, w);
     s.gs = add3(s.gs, g);
     s.gm = vfma(g.x, g.x, s.gm);
@@ -360,8 +353,8 @@ __device__ __forceinline__ float lambda_list(const KParams& p, const Team<L>& tm
     const f3 xk = make3(x[tm.k]);
     LambdaSums<T> s = lambda_zero<T>();
     for_list<L, V, 4, 1>(p, nbr, tm.k, tm.t, ncnt[tm.k], x, x,
-                            [&](const float4(&xj)[V], const float4(&)[V], unsigned valid) {
-                                lambda_pair<T, V>(p, xk, xj, valid, s);
+                            [&](const float4(&xj)[V], const float4(&)[V]) {
+                                lambda_pair<T, V>(p, xk, xj, s);
                             });
     return lambda_store<DEBUG, L, V>(p, tm, xk, s, xl, rho_out, ctl);
 }
@@ -421,8 +414,8 @@ __device__ __forceinline__ bool features_one(const KParams& p, const Team<L>& tm
     T3<T> gs = zero3<T>(), rs = zero3<T>();
     const float q2 = 0.25f * p.h2;
     int jj[B][V];
-    load_idx<V, P, B>(p, nbr, k, V * tm.t, cnt, jj);
-    for (int q0 = V * tm.t; q0 < cnt; q0 += P * B) {
+    if (cnt > 0) load_idx<V, P, B>(p, nbr, k, V * tm.t, jj);
+    for (int q0 = 0; q0 < cnt; q0 += P * B) {
         float4 xj[B][V], vj[B][V];
 #pragma unroll
         for (int u = 0; u < B; ++u)
@@ -432,14 +425,13 @@ __device__ __forceinline__ bool features_one(const KParams& p, const Team<L>& tm
                 vj[u][c] = v[jj[u][c]];
             }
         // the next batch's indices load while this batch computes
-        load_idx<V, P, B>(p, nbr, k, q0 + P * B, cnt, jj);
+        if (q0 + P * B < cnt) load_idx<V, P, B>(p, nbr, k, q0 + P * B + V * tm.t, jj);
 #pragma unroll
         for (int u = 0; u < B; ++u) {
-            const int q = q0 + u * P;
-            const unsigned valid = valid_bits<V>(q, cnt);
+            const auto valid = entries_left(T{}, cnt - (q0 + u * P + V * tm.t));
             T3<T> r, g;
             T w;
-            pair_terms<T, true>(p, xk, xj[u], valid, r, w, g);
+            pair_terms<T, true>(p, xk, xj[u], r, w, g);
             rho = vadd(rho, w);
             gs = add3(gs, g);
             gm = vfma(g.x, g.x, gm);
@@ -450,7 +442,7 @@ __device__ __forceinline__ bool features_one(const KParams& p, const Team<L>& tm
             div = vfma(vji.y, g.y, div);
             div = vfma(vji.z, g.z, div);
             const T r2 = vfma(r.z, r.z, vfma(r.y, r.y, vmul(r.x, r.x)));
-            close = vadd(close, keep_only(bc<T>(1.0f), valid & lt_mask(r2, q2)));
+            close = vadd(close, keep_only(bc<T>(1.0f), below(r2, q2, valid)));
             rs = add3(rs, T3<T>{keep_only(r.x, valid), keep_only(r.y, valid), keep_only(r.z, valid)});
             dv2 = vadd(dv2, keep_only(vfma(vji.z, vji.z, vfma(vji.y, vji.y, vmul(vji.x, vji.x))), valid));
         }
@@ -683,10 +675,10 @@ __global__ void __launch_bounds__(256, 3) k_features_warm(KParams p, int nvb, co
 // ---------------------------------------------------------------------------
 template <bool N4, typename T, int V>
 __device__ __forceinline__ void dp_pair(const KParams& p, const f3& xk, float lk, const float4 (&xj)[V],
-                                        unsigned valid, T3<T>& a) {
+                                        T3<T>& a) {
     T3<T> r, g;
     T w;
-    pair_terms<T, true>(p, xk, xj, valid, r, w, g);
+    pair_terms<T, true>(p, xk, xj, r, w, g);
     const T s = dp_weight<N4>(p, addw(lk, xj), w);
     a = {vfma(s, g.x, a.x), vfma(s, g.y, a.y), vfma(s, g.z, a.z)};
 }
@@ -729,8 +721,8 @@ __device__ __forceinline__ void dp_list(const KParams& p, const Team<L>& tm, con
     const f3 xk = make3(xk4);
     T3<T> a = zero3<T>();
     for_list<L, V, 4, 1>(p, nbr, tm.k, tm.t, ncnt[tm.k], xl, xl,
-                              [&](const float4(&xj)[V], const float4(&)[V], unsigned valid) {
-                                  dp_pair<N4, T, V>(p, xk, xk4.w, xj, valid, a);
+                              [&](const float4(&xj)[V], const float4(&)[V]) {
+                                  dp_pair<N4, T, V>(p, xk, xk4.w, xj, a);
                               });
     dp_store<DEBUG, L, V>(p, tm, xk, xk4.w, a, o);
 }
@@ -773,10 +765,10 @@ __global__ void __launch_bounds__(256, ROOMY ? ROOMY_BLOCKS : L == 1 && (N4 || V
 // ---------------------------------------------------------------------------
 template <typename T, int V>
 __device__ __forceinline__ void curl_pair(const KParams& p, const f3& xk, const f3& vk, const float4 (&xj)[V],
-                                          const float4 (&vj)[V], unsigned valid, T3<T>& wsum) {
+                                          const float4 (&vj)[V], T3<T>& wsum) {
     T3<T> r, g;
     T w;
-    pair_terms<T, false>(p, xk, xj, valid, r, w, g);
+    pair_terms<T, false>(p, xk, xj, r, w, g);
     const T3<T> vji = rdiff3(vj, vk);
     wsum = add3(wsum, cross3v(vji, g));
 }
@@ -801,8 +793,8 @@ __device__ __forceinline__ void curl_list(const KParams& p, const Team<L>& tm, c
     const f3 xk = make3(x[tm.k]), vk = make3(v[tm.k]);
     T3<T> wsum = zero3<T>();
     for_list<L, V, ROOMY ? 4 : 2, 2>(p, nbr, tm.k, tm.t, ncnt[tm.k], x, v,
-                            [&](const float4(&xj)[V], const float4(&vj)[V], unsigned valid) {
-                                curl_pair<T, V>(p, xk, vk, xj, vj, valid, wsum);
+                            [&](const float4(&xj)[V], const float4(&vj)[V]) {
+                                curl_pair<T, V>(p, xk, vk, xj, vj, wsum);
                             });
     curl_store<L, V>(tm, vk, wsum, omega, vw);
 }
@@ -839,10 +831,10 @@ template <typename T> struct VortSums {
 };
 template <typename T, int V>
 __device__ __forceinline__ void vort_pair(const KParams& p, const f3& xk, const f3& vk, const float4 (&xj)[V],
-                                          const float4 (&vj)[V], unsigned valid, VortSums<T>& s) {
+                                          const float4 (&vj)[V], VortSums<T>& s) {
     T3<T> r, g;
     T w;
-    pair_terms<T, true>(p, xk, xj, valid, r, w, g);
+    pair_terms<T, true>(p, xk, xj, r, w, g);
     const T3<T> vji = rdiff3(vj, vk);
     s.pv = {vfma(vji.x, w, s.pv.x), vfma(vji.y, w, s.pv.y), vfma(vji.z, w, s.pv.z)};
     const T wl = packw(vj);  // |w_j| (k_curl)
@@ -898,8 +890,8 @@ __device__ __forceinline__ int vort_list(const KParams& p, const Team<L>& tm, co
     const f3 xk = make3(x[tm.k]), vk = make3(vw[tm.k]);
     VortSums<T> s = {zero3<T>(), zero3<T>()};
     for_list<L, V, ROOMY ? 4 : 2, 2>(p, nbr, tm.k, tm.t, ncnt[tm.k], x, vw,
-                             [&](const float4(&xj)[V], const float4(&vj)[V], unsigned valid) {
-                                 vort_pair<T, V>(p, xk, vk, xj, vj, valid, s);
+                             [&](const float4(&xj)[V], const float4(&vj)[V]) {
+                                 vort_pair<T, V>(p, xk, vk, xj, vj, s);
                              });
     return vort_store<DEBUG, L, V>(p, tm, xk, vk, s, o);
 }
@@ -1034,7 +1026,7 @@ __global__ void __launch_bounds__(WIDE_THREADS) k_lambda_wide(KParams p, const f
     wide_pairs<1, 1>(p, w, cnt, nbr, x, x, [&](const float4(&xj)[1], const float4(&)[1], float4* dst) {
         T3<float> r, g;
         float wt;
-        pair_terms<float, true>(p, xk, xj, 1u, r, wt, g);
+        pair_terms<float, true>(p, xk, xj, r, wt, g);
         *dst = make_float4(g.x, g.y, g.z, wt);
     });
     // gradient sums, density, sum of squared gradients
@@ -1074,7 +1066,7 @@ __global__ void __launch_bounds__(WIDE_THREADS) k_dp_wide(KParams p, const float
     wide_pairs<1, 1>(p, w, cnt, nbr, xl, xl, [&](const float4(&xj)[1], const float4(&)[1], float4* dst) {
         T3<float> r, g;
         float wt;
-        pair_terms<float, true>(p, xk, xj, 1u, r, wt, g);
+        pair_terms<float, true>(p, xk, xj, r, wt, g);
         *dst = make_float4(g.x, g.y, g.z, dp_weight<N4>(p, addw(xk4.w, xj), wt));
     });
     wide_sums<1, 3>(w, cnt, p.lanes, [&](int q, float acc, const float* v) { return __fmaf_rn(v[3], v[q], acc); });
@@ -1097,7 +1089,7 @@ __global__ void __launch_bounds__(WIDE_THREADS) k_curl_wide(KParams p, const flo
     wide_pairs<1, 2>(p, w, cnt, nbr, x, v, [&](const float4(&xj)[1], const float4(&vj)[1], float4* dst) {
         T3<float> r, g;
         float wt;
-        pair_terms<float, false>(p, xk, xj, 1u, r, wt, g);
+        pair_terms<float, false>(p, xk, xj, r, wt, g);
         const T3<float> c = cross3v(rdiff3(vj, vk), g);
         *dst = make_float4(c.x, c.y, c.z, 0.0f);
     });
@@ -1119,7 +1111,7 @@ __global__ void __launch_bounds__(WIDE_THREADS) k_vort_wide(KParams p, const flo
     wide_pairs<2, 2>(p, w, cnt, nbr, x, vw, [&](const float4(&xj)[1], const float4(&vj)[1], float4* dst) {
         T3<float> r, g;
         float wt;
-        pair_terms<float, true>(p, xk, xj, 1u, r, wt, g);
+        pair_terms<float, true>(p, xk, xj, r, wt, g);
         const T3<float> d = rdiff3(vj, vk);
         dst[0] = make_float4(d.x, d.y, d.z, wt);
         dst[1] = make_float4(g.x, g.y, g.z, packw(vj));
