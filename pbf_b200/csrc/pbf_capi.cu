@@ -75,7 +75,8 @@ struct DevStats {
     int done;
     int iters;
     int conv_slot;
-    int loop_k;  // passes of the device-side correction loop
+    int loop_k;   // corrections of the device-side loop before the current lambda pass
+    int loop_k1;  // the same plus one, for the current delta-p pass
     // not reset per substep:
     int err;
     int fallback;
@@ -392,10 +393,12 @@ int count_kernel_nodes(cudaGraph_t g, int* out) {
 }
 
 // Appends to the capture on `st` the adaptive correction loop as a graph while
-// node. Each pass runs one correction (lambda, then delta-p, which ends the loop
-// instead when the lambda pass measured an error within tolerance) and the
-// loop-control kernel; passes run for slots first, first + 1, ... < max_it.
-// A converged substep therefore launches no further kernels.
+// node. Each pass runs one correction: lambda, then delta-p, which ends the loop
+// instead when the lambda pass measured an error within tolerance, and which sets
+// the loop's condition; corrections run for slots first, first + 1, ... < max_it. A
+// converged substep therefore launches no further kernels. The passes count for
+// each other: lambda reads loop_k and writes loop_k1, delta-p the other way round,
+// so no block reads a counter that another block of its kernel writes.
 int capture_correction_loop(pbf_solver* s, cudaStream_t st, int first, int min_it, int max_it, float* acc, bool dbg) {
     const KParams& kp = s->kp;
     DevStats* ds = s->dstats;
@@ -419,11 +422,18 @@ int capture_correction_loop(pbf_solver* s, cudaStream_t st, int first, int min_i
     cudaGraph_t body = np.conditional.phGraph_out[0];
     cudaStream_t bs = s->body_stream;
     CK(cudaStreamBeginCaptureToGraph(bs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    const IterCtl c{&ds->done, ds->max_bits, ds->sum, &ds->iters, &ds->conv_slot, (double)s->ext.density_tol,
-                    first, min_it, &ds->loop_k, acc};
+    IterCtl c{&ds->done, ds->max_bits, ds->sum, &ds->iters, &ds->conv_slot, (double)s->ext.density_tol,
+              first, min_it, &ds->loop_k, acc};
+    c.loop_next = &ds->loop_k1;
+    IterCtl d = c;
+    d.slot = first - 1;
+    d.loop_k = &ds->loop_k1;
+    d.loop_next = &ds->loop_k;
+    d.loop_add = 0;
+    d.handle = h;
+    d.max_slot = max_it;
     launch_lambda(kp, dbg, s->Px, s->nbr, s->ncnt, s->Q, s->rho_dbg, c, bs);
-    launch_dp(kp, dbg, s->Q, s->nbr, s->ncnt, s->Pxold, s->Px, nullptr, s->dp_dbg, c, bs);
-    launch_loop_ctl(h, &ds->loop_k, &ds->done, first, max_it, bs);
+    launch_dp(kp, dbg, s->Q, s->nbr, s->ncnt, s->Pxold, s->Px, nullptr, s->dp_dbg, d, bs);
     cudaGraph_t out = nullptr;
     CK(cudaStreamEndCapture(bs, &out));
     return count_kernel_nodes(body, &s->loop_kernel_nodes);
@@ -431,12 +441,15 @@ int capture_correction_loop(pbf_solver* s, cudaStream_t st, int first, int min_i
 
 // Enqueue one substep on `st` (captured into the graph).
 int enqueue_substep(pbf_solver* s, cudaStream_t st) {
-    const KParams& kp = s->kp;
+    KParams kp = s->kp;
     const bool dbg = s->ext.debug != 0;
     const int n = s->n;
     int* err = &s->dstats->err;
     DevStats* ds = s->dstats;
     Prof P{s, st, s->ext.profile != 0};
+    // A chain of kernels only: no event records, copies or conditional nodes between.
+    kp.pdl = !P.on && !dbg && !s->ext.adaptive && !s->ext.measure_error &&
+             !(s->ext.warm_start && s->mlp_w && s->ext.warm_unfused);
     // (the grid hash of this substep's predicted positions -- cell keys, tickets
     // and counts -- was done by the previous substep's vorticity pass, or by the
     // upload or grid build that set the state)
@@ -446,7 +459,7 @@ int enqueue_substep(pbf_solver* s, cudaStream_t st) {
         launch_scan(s->cnt, s->cell_start, s->nkeys, s->scan_ws, (int*)ds, (int)(offsetof(DevStats, err) / sizeof(int)),
                     err, st);
     });
-    P(ST_SCATTER, [&] { launch_scatter(n, s->cell, s->ticket, s->cell_start, s->tmp, err, st); });
+    P(ST_SCATTER, [&] { launch_scatter(kp.pdl, n, s->cell, s->ticket, s->cell_start, s->tmp, err, st); });
     // the substep's total lambda is tracked when features are computed (warm
     // start, or recording features for training)
     const bool warm = s->ext.warm_start && s->mlp_w;
@@ -1053,7 +1066,7 @@ int pbf_build_grid(pbf_solver* s, void* stream) {
     launch_hash(kp, false, s->Sx, s->Sv, s->cell, s->ticket, s->cnt, err, st);
     if (s->hash_dbg) CK(cudaMemcpyAsync(s->hash_dbg, s->cell, sizeof(int) * s->n, cudaMemcpyDeviceToDevice, st));
     launch_scan(s->cnt, s->cell_start, s->nkeys, s->scan_ws, nullptr, 0, err, st);
-    launch_scatter(s->n, s->cell, s->ticket, s->cell_start, s->tmp, err, st);
+    launch_scatter(false, s->n, s->cell, s->ticket, s->cell_start, s->tmp, err, st);
     launch_reorder(kp, false, s->Sx, s->Sv, s->Sperm, s->cell, s->cell_start, s->tmp, s->Px, s->Pv, s->Pxold, s->Pperm,
                    s->cell_sorted, nullptr, nullptr, err, st);
     launch_neighbors(kp, s->Px, s->cell_start, s->nbr, s->ncnt, st);

@@ -81,6 +81,7 @@ struct KParams {
     int stride;     // neighbour list stride (slot-major layout: nbr[q * stride + k])
     int cell_order; // 0 ascending, 1 descending within a cell
     int n_int;      // s_corr exponent when a small integer, else 0
+    int pdl;        // the substep's kernels launch programmatically dependent on one another
     int persistent; // neighbour passes: resident blocks striding over the tiles of slots
     unsigned flags;
     double poly6_c64;  // exact poly6 constant for the FP64 density reduction
@@ -104,6 +105,12 @@ struct IterCtl {
     const int* loop_k;             // pass counter of a device-side loop (graph while node), or null
     float* lam_acc;                // when set, the lambda pass adds its lambda here (the
                                    // substep's total lambda: warm-start feature and target)
+    // device-side loop: the counter the other pass reads receives *loop_k + loop_add;
+    // the dp pass also sets the loop's condition (handle) for slots below max_slot
+    int* loop_next = nullptr;
+    int loop_add = 1;
+    int max_slot = 0;
+    cudaGraphConditionalHandle handle = 0;
     __device__ __forceinline__ int cur_slot() const { return loop_k ? slot + *loop_k : slot; }
 };
 

@@ -17,6 +17,7 @@
 #include <algorithm>
 
 #include "pbf_kernels.h"
+#include "pbf_launch.cuh"
 #include "pbf_packed.cuh"
 
 namespace pbf {
@@ -297,6 +298,7 @@ template <int U>
 __global__ void __launch_bounds__(256) k_scatter(int n, const int* __restrict__ cell, const int* __restrict__ ticket,
                                                  const int* __restrict__ cell_start, int* __restrict__ tmp,
                                                  int* __restrict__ err) {
+    pdl_wait();
     const long long i0 = (long long)blockIdx.x * blockDim.x * U + threadIdx.x;
     int c[U], t[U];
 #pragma unroll
@@ -326,6 +328,7 @@ __global__ void __launch_bounds__(256, 8) k_reorder(KParams p, const float4* __r
                                                  float4* __restrict__ xold, int* __restrict__ perm_out,
                                                  int* __restrict__ cell_sorted, const float* __restrict__ lam_in,
                                                  float* __restrict__ lam_out, int* __restrict__ err) {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= p.n) return;
     const int c = cell[i];
@@ -546,6 +549,7 @@ template <int RR>
 __global__ void __launch_bounds__(256) k_neighbors(KParams p, int nvb, const float4* __restrict__ x,
                                                    const int* __restrict__ cell_start, int* __restrict__ nbr,
                                                    int* __restrict__ ncnt) {
+    pdl_wait();
     for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x)
         neighbors_one<RR>(p, vb * blockDim.x + threadIdx.x, x, cell_start, nbr, ncnt);
 }
@@ -563,6 +567,7 @@ __global__ void __launch_bounds__(SEARCH_WIDE_THREADS) k_neighbors_wide(KParams 
                                                                         const int* __restrict__ cell_start,
                                                                         int* __restrict__ nbr,
                                                                         int* __restrict__ ncnt) {
+    pdl_wait();
     constexpr int W = 2 * RR + 1, ROWS = W * W, MR = (ROWS + SEARCH_WIDE - 1) / SEARCH_WIDE;
     const int t = threadIdx.x & (SEARCH_WIDE - 1);
     const int team = (blockIdx.x * SEARCH_WIDE_THREADS + threadIdx.x) / SEARCH_WIDE;
@@ -685,16 +690,6 @@ __global__ void k_count_fallback(const int* __restrict__ iters, int first, int c
     const int used = first + *iters;
     if (used > configured) *fallback += 1;
     *total += used;
-}
-
-// Control of the device-side correction loop (a graph while node whose body is
-// one lambda pass and one delta-p pass, then this kernel): counts the pass and
-// keeps the loop running while the error is above tolerance and slots are left.
-__global__ void k_loop_ctl(cudaGraphConditionalHandle h, int* __restrict__ loop_k, const int* __restrict__ done,
-                           int first, int max_it) {
-    const int k = *loop_k + 1;
-    *loop_k = k;
-    cudaGraphSetConditional(h, (*done == 0 && first + k < max_it) ? 1u : 0u);
 }
 
 // v = (x - x_old) / dt as its own pass (adaptive iteration counts)
@@ -994,10 +989,12 @@ void launch_scan_silent_tile(const int* in, int* out, int m, void* ws, int* err,
     launch_scan_cleared<false>(const_cast<int*>(in), out, m, ws, err, nullptr, st, silent_tile, spin_limit);
 }
 
-void launch_scatter(int n, const int* cell, const int* ticket, const int* cell_start, int* tmp, int* err,
+void launch_scatter(bool pdl, int n, const int* cell, const int* ticket, const int* cell_start, int* tmp, int* err,
                     cudaStream_t st) {
-    if (n >= (1 << 20)) k_scatter<4><<<blocks_for(n, 256 * 4), 256, 0, st>>>(n, cell, ticket, cell_start, tmp, err);
-    else k_scatter<1><<<blocks_for(n, 256), 256, 0, st>>>(n, cell, ticket, cell_start, tmp, err);
+    if (n >= (1 << 20))
+        launch(pdl, k_scatter<4>, blocks_for(n, 256 * 4), 256, 0, st, n, cell, ticket, cell_start, tmp, err);
+    else
+        launch(pdl, k_scatter<1>, blocks_for(n, 256), 256, 0, st, n, cell, ticket, cell_start, tmp, err);
 }
 
 void launch_reorder(const KParams& p, bool predict_on, const float4* x, const float4* v, const int* perm,
@@ -1005,10 +1002,10 @@ void launch_reorder(const KParams& p, bool predict_on, const float4* x, const fl
                     int* perm_out, int* cell_sorted, const float* lam_in, float* lam_out, int* err, cudaStream_t st) {
     const int b = blocks_for(p.n, 256);
     if (predict_on)
-        k_reorder<true><<<b, 256, 0, st>>>(p, x, v, perm, cell, cell_start, tmp, xp, vp, xold, perm_out, cell_sorted,
+        launch(p.pdl, k_reorder<true>, b, 256, 0, st, p, x, v, perm, cell, cell_start, tmp, xp, vp, xold, perm_out, cell_sorted,
                                            lam_in, lam_out, err);
     else
-        k_reorder<false><<<b, 256, 0, st>>>(p, x, v, perm, cell, cell_start, tmp, xp, vp, xold, perm_out, cell_sorted,
+        launch(p.pdl, k_reorder<false>, b, 256, 0, st, p, x, v, perm, cell, cell_start, tmp, xp, vp, xold, perm_out, cell_sorted,
                                             lam_in, lam_out, err);
 }
 
@@ -1032,14 +1029,14 @@ constexpr int SEARCH_WIDE_MAX_N = 45056;
 void launch_neighbors(const KParams& p, const float4* x, const int* cell_start, int* nbr, int* ncnt, cudaStream_t st) {
     if (p.n <= SEARCH_WIDE_MAX_N && !p.persistent && p.radius <= 2) {
         const int b = blocks_for(p.n, SEARCH_WIDE_THREADS / SEARCH_WIDE);
-        if (p.radius == 1) k_neighbors_wide<1><<<b, SEARCH_WIDE_THREADS, 0, st>>>(p, x, cell_start, nbr, ncnt);
-        else k_neighbors_wide<2><<<b, SEARCH_WIDE_THREADS, 0, st>>>(p, x, cell_start, nbr, ncnt);
+        if (p.radius == 1) launch(p.pdl, k_neighbors_wide<1>, b, SEARCH_WIDE_THREADS, 0, st, p, x, cell_start, nbr, ncnt);
+        else launch(p.pdl, k_neighbors_wide<2>, b, SEARCH_WIDE_THREADS, 0, st, p, x, cell_start, nbr, ncnt);
         return;
     }
     const int b = blocks_for(p.n, p.block);
-    if (p.radius == 1) k_neighbors<1><<<resident_grid(p, k_neighbors<1>, b), p.block, 0, st>>>(p, b, x, cell_start, nbr, ncnt);
-    else if (p.radius == 2) k_neighbors<2><<<resident_grid(p, k_neighbors<2>, b), p.block, 0, st>>>(p, b, x, cell_start, nbr, ncnt);
-    else k_neighbors<0><<<resident_grid(p, k_neighbors<0>, b), p.block, 0, st>>>(p, b, x, cell_start, nbr, ncnt);
+    if (p.radius == 1) launch(p.pdl, k_neighbors<1>, resident_grid(p, k_neighbors<1>, b), p.block, 0, st, p, b, x, cell_start, nbr, ncnt);
+    else if (p.radius == 2) launch(p.pdl, k_neighbors<2>, resident_grid(p, k_neighbors<2>, b), p.block, 0, st, p, b, x, cell_start, nbr, ncnt);
+    else launch(p.pdl, k_neighbors<0>, resident_grid(p, k_neighbors<0>, b), p.block, 0, st, p, b, x, cell_start, nbr, ncnt);
 }
 
 void launch_gather_rows(const int* slots, int count, int n, const float* feat, const float* lam_acc, float* out_feat,
@@ -1052,11 +1049,6 @@ void launch_gather_rows(const int* slots, int count, int n, const float* feat, c
 void launch_count_fallback(const int* iters, int first, int configured, int* fallback, long long* total,
                            cudaStream_t st) {
     k_count_fallback<<<1, 1, 0, st>>>(iters, first, configured, fallback, total);
-}
-
-void launch_loop_ctl(cudaGraphConditionalHandle h, int* loop_k, const int* done, int first, int max_it,
-                     cudaStream_t st) {
-    k_loop_ctl<<<1, 1, 0, st>>>(h, loop_k, done, first, max_it);
 }
 
 void launch_velocity(const KParams& p, const float4* x, const float4* xold, float4* v, cudaStream_t st) {

@@ -29,7 +29,8 @@ void launch_scan_const(const int* in, int* out, int m, void* ws, size_t clear_by
 // look-back gives up after spin_limit polls (input left unchanged)
 void launch_scan_silent_tile(const int* in, int* out, int m, void* status_ws, int* err, int silent_tile,
                              long long spin_limit, cudaStream_t st);
-void launch_scatter(int n, const int* cell, const int* ticket, const int* cell_start, int* tmp, int* err,
+// (pdl here and KParams::pdl: programmatic dependent launch on the kernel before)
+void launch_scatter(bool pdl, int n, const int* cell, const int* ticket, const int* cell_start, int* tmp, int* err,
                     cudaStream_t st);
 void launch_reorder(const KParams& p, bool predict_on, const float4* x, const float4* v, const int* perm,
                     const int* cell, const int* cell_start, const int* tmp, float4* xp, float4* vp, float4* xold,
@@ -51,8 +52,6 @@ void launch_gather_rows(const int* slots, int count, int n, const float* feat, c
                         float* out_target, int* err, cudaStream_t st);
 void launch_count_fallback(const int* iters, int first, int configured, int* fallback, long long* total,
                            cudaStream_t st);
-void launch_loop_ctl(cudaGraphConditionalHandle h, int* loop_k, const int* done, int first, int max_it,
-                     cudaStream_t st);
 void launch_velocity(const KParams& p, const float4* x, const float4* xold, float4* v, cudaStream_t st);
 // Curl: omega = (w, |w|) and vw = (v, |w|) per particle.
 void launch_curl(const KParams& p, const float4* x, const float4* v, const int* nbr, const int* ncnt, float4* omega,

@@ -13,6 +13,7 @@
 #include <stdint.h>
 
 #include "pbf_device.cuh"
+#include "pbf_launch.cuh"
 #include "pbf_mlp.h"
 #include "pbf_packed.cuh"
 #include "pbf_tc.cuh"
@@ -264,11 +265,6 @@ __global__ void __launch_bounds__(128, 1) k_mlp_fwd(FwdIO io) {
 // per layer and direction (activations stored 2 bytes at a time, one launch per
 // gradient sum), see the measured time at k_mlp_reduce.
 // ---------------------------------------------------------------------------
-// Programmatic dependent launch: let the next kernel of the stream start its
-// prologue; wait until the kernels before are complete and their writes visible.
-__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 struct TrainIO {
     const uint16_t* w;    // bf16 weights
     const float* b;       // biases and constants
@@ -708,23 +704,6 @@ void mlp_trainer_destroy(MlpTrainer* t) {
     delete t;
 }
 
-// Launch with programmatic stream serialisation (the kernel calls pdl_wait before
-// it reads what the kernels before it wrote).
-template <typename... P, typename... A>
-static int launch_pdl(void (*k)(P...), int grid, int block, int smem, cudaStream_t st, A... args) {
-    cudaLaunchConfig_t c{};
-    c.gridDim = dim3(grid);
-    c.blockDim = dim3(block);
-    c.dynamicSmemBytes = smem;
-    c.stream = st;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    c.attrs = &at;
-    c.numAttrs = 1;
-    return cudaLaunchKernelEx(&c, k, P(args)...) == cudaSuccess ? 0 : -1;
-}
-
 // The tiles' gradient partials of a batch; the caller sums them.
 static int launch_train(MlpTrainer* t, const float* feat, const float* target, int B, cudaStream_t st) {
     if (B <= 0 || B > t->cap) return -1;
@@ -734,14 +713,14 @@ static int launch_train(MlpTrainer* t, const float* feat, const float* target, i
     const int tiles = (B + TILE - 1) / TILE;
     const int grid = tiles < sm_count() ? tiles : sm_count();
     const TrainIO io{t->w16, t->b32, feat, target, t->part, B, 1.0f / (float)B, t->err};
-    return launch_pdl(k_mlp_train, grid, TR_THREADS, TR_SMEM, st, io);
+    return launch(true, k_mlp_train, grid, TR_THREADS, TR_SMEM, st, io);
 }
 
 constexpr int REDUCE_BLOCKS = (MLP_NUM_WEIGHTS + MLP_NUM_TRAINED_BIASES + 1 + 63) / 64;
 
 int mlp_gradients(MlpTrainer* t, const float* feat, const float* target, int B, cudaStream_t st) {
     if (launch_train(t, feat, target, B, st)) return -1;
-    return launch_pdl(k_mlp_reduce<false>, REDUCE_BLOCKS, 64, 0, st, t->part, (B + TILE - 1) / TILE, t->gw, t->gb,
+    return launch(true, k_mlp_reduce<false>, REDUCE_BLOCKS, 64, 0, st, t->part, (B + TILE - 1) / TILE, t->gw, t->gb,
                       t->loss, AdamIO{});
 }
 
@@ -751,7 +730,7 @@ int mlp_train_step(MlpTrainer* t, const float* feat, const float* target, int B,
     t->step += 1;
     const AdamIO a{t->w32, t->b32, t->mw, t->mb, t->vw, t->vb, t->w16, lr, beta1, beta2, eps,
                    1.0f - powf(beta1, (float)t->step), 1.0f - powf(beta2, (float)t->step)};
-    return launch_pdl(k_mlp_reduce<true>, REDUCE_BLOCKS, 64, 0, st, t->part, (B + TILE - 1) / TILE, t->gw, t->gb,
+    return launch(true, k_mlp_reduce<true>, REDUCE_BLOCKS, 64, 0, st, t->part, (B + TILE - 1) / TILE, t->gw, t->gb,
                       t->loss, a);
 }
 

@@ -27,6 +27,7 @@
 #include "pbf_kernels.h"
 #include "pbf_mlp.h"
 #include "pbf_mlp_dev.cuh"
+#include "pbf_launch.cuh"
 #include "pbf_packed.cuh"
 
 #include <algorithm>
@@ -359,6 +360,13 @@ __device__ __forceinline__ float lambda_list(const KParams& p, const Team<L>& tm
     return lambda_store<DEBUG, L, V>(p, tm, xk, s, xl, rho_out, ctl);
 }
 
+// Adaptive loop: true when it has ended. In the device-side loop it also hands the
+// delta-p pass its counter.
+__device__ __forceinline__ bool lambda_skip(const IterCtl& ctl) {
+    if (ctl.loop_next && blockIdx.x == 0 && threadIdx.x == 0) *ctl.loop_next = *ctl.loop_k + ctl.loop_add;
+    return ctl.done && *ctl.done;
+}
+
 // nvb tiles of blockDim.x slots' teams; the grid strides over them (a grid of
 // nvb blocks is the ordinary one-block-per-tile launch)
 template <bool DEBUG, bool ROOMY, int L, int V>
@@ -366,7 +374,8 @@ __global__ void __launch_bounds__(256, ROOMY ? ROOMY_BLOCKS : 4) k_lambda(KParam
                                                                 const int* __restrict__ nbr,
                                                                 const int* __restrict__ ncnt, float4* __restrict__ xl,
                                                                 float* __restrict__ rho_out, IterCtl ctl) {
-    if (ctl.done && *ctl.done) return;
+    pdl_wait();
+    if (lambda_skip(ctl)) return;
     for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
         const Team<L> tm = team_of<L>(vb);
         float err = 0.0f;
@@ -503,6 +512,7 @@ __global__ void __launch_bounds__(256) k_features(KParams p, int nvb, const floa
                                                   const int* __restrict__ ncnt, const float* __restrict__ lam_prev,
                                                   float4* __restrict__ xl, float* __restrict__ feat,
                                                   float* __restrict__ lam_acc) {
+    pdl_wait();
     for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
         float f[12], lam;
         features_one<L, V>(p, team_of<L>(vb), x, v, nbr, ncnt, lam_prev, xl, feat, lam_acc, f, lam);
@@ -548,6 +558,7 @@ __global__ void __launch_bounds__(256, 3) k_features_warm(KParams p, int nvb, co
                                                           const float* __restrict__ lam_prev,
                                                           float4* __restrict__ xl, float* __restrict__ feat,
                                                           float* __restrict__ lam_acc, WarmIO io) {
+    pdl_wait();
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint64_t mbar;
     __shared__ uint32_t tmem_slot;
@@ -732,25 +743,31 @@ __device__ __forceinline__ void dp_list(const KParams& p, const Team<L>& tm, con
 // tolerance).
 __device__ __forceinline__ bool dp_skip(const IterCtl& ctl) {
     if (!ctl.done) return false;
-    if (*ctl.done) return true;
+    const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
     // the lambda pass just measured the positions this pass would correct;
     // when they are within tolerance the loop ends here
     const int sl = ctl.cur_slot();
-    if (sl >= ctl.min_slot && __longlong_as_double((long long)ctl.max_bits[sl]) <= ctl.tol) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
+    const bool over = *ctl.done != 0;
+    const bool met = !over && sl >= ctl.min_slot && __longlong_as_double((long long)ctl.max_bits[sl]) <= ctl.tol;
+    if (lead) {
+        if (met) {
             *ctl.done = 1;
             *ctl.conv_slot = sl;
         }
-        return true;
+        if (!over && !met) atomicAdd(ctl.iters, 1);
+        if (ctl.loop_next) {
+            *ctl.loop_next = *ctl.loop_k + ctl.loop_add;
+            cudaGraphSetConditional(ctl.handle, !over && !met && sl + 1 < ctl.max_slot ? 1u : 0u);
+        }
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(ctl.iters, 1);
-    return false;
+    return over || met;
 }
 
 template <bool DEBUG, bool N4, bool ROOMY, int L, int V>
 __global__ void __launch_bounds__(256, ROOMY ? ROOMY_BLOCKS : L == 1 && (N4 || V == 1) ? 5 : 4) k_dp(KParams p, int nvb, const float4* __restrict__ xl,
                                                             const int* __restrict__ nbr, const int* __restrict__ ncnt,
                                                             DpOut o, IterCtl ctl) {
+    pdl_wait();
     if (dp_skip(ctl)) return;
     for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
         const Team<L> tm = team_of<L>(vb);
@@ -804,6 +821,7 @@ __global__ void __launch_bounds__(256, ROOMY ? ROOMY_BLOCKS : 4) k_curl(KParams 
                                               const float4* __restrict__ v, const int* __restrict__ nbr,
                                               const int* __restrict__ ncnt, float4* __restrict__ omega,
                                               float4* __restrict__ vw) {
+    pdl_wait();
     for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
         const Team<L> tm = team_of<L>(vb);
         if (tm.k < p.n) curl_list<ROOMY, L, V>(p, tm, x, v, nbr, ncnt, omega, vw);  // uniform over the team
@@ -900,6 +918,7 @@ template <bool DEBUG, bool ROOMY, int L, int V>
 __global__ void __launch_bounds__(256, ROOMY ? ROOMY_BLOCKS : 4) k_vort(KParams p, int nvb, const float4* __restrict__ x,
                                                  const float4* __restrict__ vw, const int* __restrict__ nbr,
                                                  const int* __restrict__ ncnt, VortIO o) {
+    pdl_wait();
     for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
         const Team<L> tm = team_of<L>(vb);
         int key = -1;
@@ -1018,7 +1037,8 @@ __global__ void __launch_bounds__(WIDE_THREADS) k_lambda_wide(KParams p, const f
                                                               const int* __restrict__ nbr,
                                                               const int* __restrict__ ncnt, float4* __restrict__ xl,
                                                               float* __restrict__ rho_out, IterCtl ctl) {
-    if (ctl.done && *ctl.done) return;
+    pdl_wait();
+    if (lambda_skip(ctl)) return;
     const WideTeam w = wide_team<1>(p.max_nbr);
     const bool on = w.k < p.n;
     const int cnt = on ? ncnt[w.k] : 0;
@@ -1057,6 +1077,7 @@ template <bool DEBUG, bool N4>
 __global__ void __launch_bounds__(WIDE_THREADS) k_dp_wide(KParams p, const float4* __restrict__ xl,
                                                           const int* __restrict__ nbr, const int* __restrict__ ncnt,
                                                           DpOut o, IterCtl ctl) {
+    pdl_wait();
     if (dp_skip(ctl)) return;
     const WideTeam w = wide_team<1>(p.max_nbr);
     const bool on = w.k < p.n;
@@ -1082,6 +1103,7 @@ __global__ void __launch_bounds__(WIDE_THREADS) k_curl_wide(KParams p, const flo
                                                             const float4* __restrict__ v, const int* __restrict__ nbr,
                                                             const int* __restrict__ ncnt, float4* __restrict__ omega,
                                                             float4* __restrict__ vw) {
+    pdl_wait();
     const WideTeam w = wide_team<1>(p.max_nbr);
     const bool on = w.k < p.n;
     const int cnt = on ? ncnt[w.k] : 0;
@@ -1104,6 +1126,7 @@ __global__ void __launch_bounds__(WIDE_THREADS) k_vort_wide(KParams p, const flo
                                                             const float4* __restrict__ vw,
                                                             const int* __restrict__ nbr, const int* __restrict__ ncnt,
                                                             VortIO o) {
+    pdl_wait();
     const WideTeam w = wide_team<2>(p.max_nbr);
     const bool on = w.k < p.n;
     const int cnt = on ? ncnt[w.k] : 0;
@@ -1198,7 +1221,7 @@ static void launch_wide(const KParams& p, K kernel, cudaStream_t st, A... args) 
     const int smem = wide_smem<NV>(p.max_nbr);  // at most 69 KB (127 entries of two float4)
     if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     const int per = WIDE_THREADS / WIDE;
-    kernel<<<(p.n + per - 1) / per, WIDE_THREADS, smem, st>>>(p, args...);
+    launch(p.pdl, kernel, (p.n + per - 1) / per, WIDE_THREADS, smem, st, p, args...);
 }
 
 void launch_lambda(const KParams& p, bool debug, const float4* x, const int* nbr, const int* ncnt, float4* xl,
@@ -1214,7 +1237,7 @@ void launch_lambda(const KParams& p, bool debug, const float4* x, const int* nbr
         const int b = team_blocks(p.n, L, p.block);
         with_flags(debug, roomy(p, L), [&](auto d, auto r) {
             auto* k = k_lambda<decltype(d)::value, decltype(r)::value, L, V>;
-            k<<<pass_grid(p, k, b), p.block, 0, st>>>(p, b, x, nbr, ncnt, xl, rho, ctl);
+            launch(p.pdl, k, pass_grid(p, k, b), p.block, 0, st, p, b, x, nbr, ncnt, xl, rho, ctl);
         });
     });
 }
@@ -1234,7 +1257,7 @@ void launch_dp(const KParams& p, bool debug, const float4* xl, const int* nbr, c
         with_flags(debug, p.n_int == 4, [&](auto d, auto n4) {
             with_flag(roomy(p, L), [&](auto r) {
                 auto* k = k_dp<decltype(d)::value, decltype(n4)::value, decltype(r)::value, L, V>;
-                k<<<pass_grid(p, k, b), p.block, 0, st>>>(p, b, xl, nbr, ncnt, o, ctl);
+                launch(p.pdl, k, pass_grid(p, k, b), p.block, 0, st, p, b, xl, nbr, ncnt, o, ctl);
             });
         });
     });
@@ -1245,7 +1268,7 @@ void launch_features(const KParams& p, const float4* x, const float4* v, const i
     with_lanes(p.lanes, [&](auto c) {
         constexpr int L = decltype(c)::L, V = decltype(c)::V;
         const int b = team_blocks(p.n, L, p.block);
-        k_features<L, V><<<pass_grid(p, k_features<L, V>, b), p.block, 0, st>>>(p, b, x, v, nbr, ncnt, lam_prev, xl,
+        launch(p.pdl, k_features<L, V>, pass_grid(p, k_features<L, V>, b), p.block, 0, st, p, b, x, v, nbr, ncnt, lam_prev, xl,
                                                                                  feat, lam_acc);
     });
 }
@@ -1275,7 +1298,7 @@ int launch_features_warm(const KParams& p, const float4* x, const float4* v, con
             grid = (int)std::min<long long>((long long)per_sm * sms, nvb);
         }
         const WarmIO io{w, b, lam0, clamp, floor, err};
-        k_features_warm<L, V><<<grid, p.block, smem, st>>>(p, nvb, x, v, nbr, ncnt, lam_prev, xl, feat, lam_acc, io);
+        launch(p.pdl, k_features_warm<L, V>, grid, p.block, smem, st, p, nvb, x, v, nbr, ncnt, lam_prev, xl, feat, lam_acc, io);
     });
     return rc;
 }
@@ -1291,7 +1314,7 @@ void launch_curl(const KParams& p, const float4* x, const float4* v, const int* 
         const int b = team_blocks(p.n, L, p.block);
         with_flag(roomy(p, L), [&](auto r) {
             auto* k = k_curl<decltype(r)::value, L, V>;
-            k<<<pass_grid(p, k, b), p.block, 0, st>>>(p, b, x, v, nbr, ncnt, omega, vw);
+            launch(p.pdl, k, pass_grid(p, k, b), p.block, 0, st, p, b, x, v, nbr, ncnt, omega, vw);
         });
     });
 }
@@ -1309,7 +1332,7 @@ void launch_vort(const KParams& p, bool debug, const float4* x, const float4* vw
         const int b = team_blocks(p.n, L, p.block);
         with_flags(debug, roomy(p, L), [&](auto d, auto r) {
             auto* k = k_vort<decltype(d)::value, decltype(r)::value, L, V>;
-            k<<<pass_grid(p, k, b), p.block, 0, st>>>(p, b, x, vw, nbr, ncnt, o);
+            launch(p.pdl, k, pass_grid(p, k, b), p.block, 0, st, p, b, x, vw, nbr, ncnt, o);
         });
     });
 }
