@@ -93,8 +93,9 @@ typedef struct pbf_ext_params {
                             persistent launch: the blocks resident at once stride over all
                             scenes' tiles of slots (default 0: one block per tile). Same results */
     int warm_unfused;    /* 1: the warm start's feature pass and network as two launches with the
-                            features through HBM (default 0: one fused launch, the features go
-                            from the feature pass to the tensor cores through shared memory).
+                            features in FP32 through HBM (default 0: one fused launch in small
+                            scenes, the features going to the tensor cores through shared
+                            memory, two with packed BF16 rows between them in large ones).
                             Same results; kept for measurement */
     int warm_floor;      /* 1: with warm_clamp > 0, lambda0 is also at least as strong as the plain
                             lambda of its pass (between it and warm_clamp times it), so the first

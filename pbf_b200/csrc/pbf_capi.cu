@@ -485,7 +485,8 @@ int enqueue_substep(pbf_solver* s, cudaStream_t st) {
             P(ST_LAMBDA, [&] {
                 rc = launch_features_warm(kp, s->Px, s->Pv, s->nbr, s->ncnt, s->lam_prev_sorted, s->Q,
                                           s->ext.record_features ? s->feat : nullptr, s->lam_acc, s->mlp_w, s->mlp_b,
-                                          s->lam0, s->ext.warm_clamp, s->ext.warm_floor, err, st);
+                                          s->lam0, s->ext.warm_clamp, s->ext.warm_floor, reinterpret_cast<uint4*>(s->omega),
+                                          reinterpret_cast<uint4*>(s->vw), err, st);
             });
             if (rc) return fail(PBF_ERR_CUDA, "fused warm-start pass: launch configuration failed");
         } else {

@@ -43,11 +43,13 @@ void launch_dp(const KParams& p, bool debug, const float4* xl, const int* nbr, c
 void launch_features(const KParams& p, const float4* x, const float4* v, const int* nbr, const int* ncnt,
                      const float* lam_prev, float4* xl, float* feat, float* lam_acc, cudaStream_t st);
 // The first lambda pass of a warm-started substep fused with the network on the
-// tensor cores: writes xl = (x, lambda0), lam_acc = lam0 = lambda0 (feat only
-// when not null). Returns nonzero when the launch could not be configured.
+// tensor cores, in one launch or two by size: writes xl = (x, lambda0), lam_acc =
+// lam0 = lambda0 (feat only when not null); row_lo and row_hi, n entries each, are
+// scratch. Returns nonzero when the launch could not be configured.
 int launch_features_warm(const KParams& p, const float4* x, const float4* v, const int* nbr, const int* ncnt,
                          const float* lam_prev, float4* xl, float* feat, float* lam_acc, const uint16_t* w,
-                         const float* b, float* lam0, float clamp, int floor, int* err, cudaStream_t st);
+                         const float* b, float* lam0, float clamp, int floor, uint4* row_lo, uint4* row_hi, int* err,
+                         cudaStream_t st);
 void launch_gather_rows(const int* slots, int count, int n, const float* feat, const float* lam_acc, float* out_feat,
                         float* out_target, int* err, cudaStream_t st);
 void launch_count_fallback(const int* iters, int first, int configured, int* fallback, long long* total,

@@ -413,7 +413,7 @@ __device__ __forceinline__ bool features_one(const KParams& p, const Team<L>& tm
                                              float4* __restrict__ xl, float* __restrict__ feat,
                                              float* __restrict__ lam_acc, float (&f)[12], float& lam) {
     using T = vec_t<V>;
-    constexpr int P = L * V, B = 4 / V;
+    constexpr int P = L * V, B = 2 / V;
     const int k = tm.k;
     if (k >= p.n) return false;  // uniform over the team
     const f3 xk = make3(x[k]);
@@ -506,16 +506,42 @@ __device__ __forceinline__ bool features_one(const KParams& p, const Team<L>& tm
     return true;
 }
 
-template <int L, int V>
-__global__ void __launch_bounds__(256) k_features(KParams p, int nvb, const float4* __restrict__ x,
+// The network's input row of a particle: its normalised features as BF16, padded
+// from 12 to 16 with zeros. norm: the network's biases and constants.
+__device__ __forceinline__ void pack_row(const float (&f)[12], const float* norm, uint32_t (&pk)[8]) {
+    float xf[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) xf[i] = 0.0f;
+#pragma unroll
+    for (int i = 0; i < MLP_IN; ++i) xf[i] = (f[i] - norm[FMEAN_OFF + i]) * norm[FISTD_OFF + i];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        pk[i] = (uint32_t)bf16_bits(xf[2 * i]) | ((uint32_t)bf16_bits(xf[2 * i + 1]) << 16);
+}
+
+// ROWS: also writes the particle's network input, entries 0-7 to row_lo and 8-15
+// to row_hi, for k_warm_rows. Two
+// entries per batch and four blocks per SM, as the two-array passes: 34.7 us at
+// 262,144 particles; two entries without the bound 42.6, four entries 36.2 at three
+// blocks and 45.0 without a bound.
+template <bool ROWS, int L, int V>
+__global__ void __launch_bounds__(256, 4) k_features(KParams p, int nvb, const float4* __restrict__ x,
                                                   const float4* __restrict__ v, const int* __restrict__ nbr,
                                                   const int* __restrict__ ncnt, const float* __restrict__ lam_prev,
                                                   float4* __restrict__ xl, float* __restrict__ feat,
-                                                  float* __restrict__ lam_acc) {
+                                                  float* __restrict__ lam_acc, const float* __restrict__ norm,
+                                                  uint4* __restrict__ row_lo, uint4* __restrict__ row_hi) {
     pdl_wait();
     for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
+        const Team<L> tm = team_of<L>(vb);
         float f[12], lam;
-        features_one<L, V>(p, team_of<L>(vb), x, v, nbr, ncnt, lam_prev, xl, feat, lam_acc, f, lam);
+        const bool have = features_one<L, V>(p, tm, x, v, nbr, ncnt, lam_prev, xl, feat, lam_acc, f, lam);
+        if (ROWS && have) {
+            uint32_t pk[8];
+            pack_row(f, norm, pk);
+            row_lo[tm.k] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+            row_hi[tm.k] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+        }
     }
 }
 
@@ -532,7 +558,9 @@ __global__ void __launch_bounds__(256) k_features(KParams p, int nvb, const floa
 // of the second half of a 256-thread block the second tile's columns. While
 // one block waits on its MMAs the SM runs the other resident blocks' gathers.
 // The arithmetic is k_mlp_fwd's (same operands, MMA shapes and epilogue), so
-// lambda0 is the unfused path's bit for bit.
+// lambda0 is the unfused path's bit for bit. The blocks' shared memory leaves the
+// gathers 70 KB of L1: large scenes run the same two halves as k_features and
+// k_warm_rows instead.
 // ---------------------------------------------------------------------------
 struct WarmIO {
     const uint16_t* w;  // BF16 weights (W1 [64][16], W2, W3 [64][64], w4 [64])
@@ -551,6 +579,99 @@ constexpr int FW_X_TILE = 128 * 16 * 2;
 constexpr int FW_H_TILE = 128 * 64 * 2;
 __host__ __device__ constexpr int warm_smem_bytes(int tiles) { return FW_SX + tiles * (FW_X_TILE + FW_H_TILE); }
 
+// Stages the weights, biases and the barrier, allocates `cols` TMEM columns and
+// returns their base. Called by every thread of the block.
+__device__ __forceinline__ uint32_t warm_setup(const WarmIO& io, uint8_t* smem, uint64_t* mbar, uint32_t* tmem_slot,
+                                               float* sb, float* sw4, uint32_t cols) {
+    const int t = threadIdx.x;
+    if (t < 32) tmem_alloc(tmem_slot, cols);
+    if (t == 0) mbar_init(mbar, 1);
+    stage_weight(smem + FW_SW1, io.w + W1_OFF, 64, 16);
+    stage_weight(smem + FW_SW2, io.w + W2_OFF, 64, 64);
+    stage_weight(smem + FW_SW3, io.w + W3_OFF, 64, 64);
+    for (int i = t; i < MLP_NUM_BIASES; i += blockDim.x) sb[i] = io.b[i];
+    if (t < 64) sw4[t] = bf16_val(io.w[W4_OFF + t]);
+    fence_before_sync();
+    __syncthreads();
+    fence_after_sync();
+    return *tmem_slot;
+}
+
+// The three hidden layers and the read-out for the rows of `tiles` 128-row tiles:
+// layer l reads X (l = 0, tile j at sX + j x_stride) or H and writes H (l < 2).
+// Thread t has row t of the block and returns its output in y. synced() runs after
+// the barrier that makes the block's X visible. False on an expired wait.
+template <typename F>
+__device__ __forceinline__ bool warm_layers(const WarmIO& io, const uint8_t* smem, const uint8_t* sX, int x_stride,
+                                            uint8_t* sH, int tiles, uint32_t tbase, uint64_t* mbar, uint32_t& phase,
+                                            const float* sb, const float* sw4, float& y, F&& synced) {
+    const int t = threadIdx.x, warp = t >> 5;
+    const bool ep_warp = (warp >> 2) < tiles;  // this warp's TMEM quarter holds rows of a tile
+    const uint32_t lane_base = tmem_addr(tbase, 32 * (warp & 3), 64 * (warp >> 2));
+    uint8_t* my_h = sH + (warp >> 2) * FW_H_TILE;
+    y = sb[B4_OFF];
+#pragma unroll 1
+    for (int l = 0; l < 3; ++l) {
+        sync_for_mma();
+        if (l == 0) synced();
+        if (t == 0) {
+            for (int j = 0; j < tiles; ++j) {
+                if (l == 0) gemm_issue(tbase + 64 * j, sX + j * x_stride, smem + FW_SW1, 64, 16, 0);
+                else gemm_issue(tbase + 64 * j, sH + j * FW_H_TILE, smem + (l == 1 ? FW_SW2 : FW_SW3), 64, 64, 0);
+            }
+            commit(mbar);
+        }
+        if (!wait_mma(mbar, phase, io.err)) return false;
+        if (ep_warp) {
+            const float* bias = sb + (l == 0 ? B1_OFF : l == 1 ? B2_OFF : B3_OFF);
+#pragma unroll 1
+            for (int c = 0; c < 4; ++c) {
+                float vv[16];
+                tmem_ld16(lane_base + 16 * c, vv);
+                tmem_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 16; i += 4) {
+                    const float4 bi = *reinterpret_cast<const float4*>(bias + 16 * c + i);
+                    const float2 h0 = gelu2(vadd(make_float2(vv[i], vv[i + 1]), make_float2(bi.x, bi.y)));
+                    const float2 h1 = gelu2(vadd(make_float2(vv[i + 2], vv[i + 3]), make_float2(bi.z, bi.w)));
+                    vv[i] = h0.x;
+                    vv[i + 1] = h0.y;
+                    vv[i + 2] = h1.x;
+                    vv[i + 3] = h1.y;
+                }
+                if (l < 2) {
+                    put_row64(my_h, t & 127, vv, 16 * c);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 16; i += 4) {
+                        const float4 w = *reinterpret_cast<const float4*>(sw4 + 16 * c + i);
+                        y = __fmaf_rn(vv[i], w.x, y);
+                        y = __fmaf_rn(vv[i + 1], w.y, y);
+                        y = __fmaf_rn(vv[i + 2], w.z, y);
+                        y = __fmaf_rn(vv[i + 3], w.w, y);
+                    }
+                }
+            }
+        }
+    }
+    return true;
+}
+
+// Slot k's lambda0 from the network's output y: the trust region around the plain
+// lambda of this pass has its sign and at most clamp times its magnitude.
+__device__ __forceinline__ void warm_store(const WarmIO& io, const float* sb, int k, float y, float lam_plain,
+                                           float4* __restrict__ xl, float* __restrict__ lam_acc) {
+    float l0 = y * sb[OSCALE_OFF];
+    if (io.clamp > 0.0f) {
+        const float a = io.clamp * lam_plain;
+        const float f0 = io.floor ? lam_plain : 0.0f;  // the weak end of the interval
+        l0 = fminf(fmaxf(l0, fminf(a, f0)), fmaxf(a, f0));
+    }
+    reinterpret_cast<float*>(xl)[4 * (size_t)k + 3] = l0;
+    lam_acc[k] = l0;
+    io.lam0[k] = l0;
+}
+
 template <int L, int V>
 __global__ void __launch_bounds__(256, 3) k_features_warm(KParams p, int nvb, const float4* __restrict__ x,
                                                           const float4* __restrict__ v, const int* __restrict__ nbr,
@@ -562,32 +683,19 @@ __global__ void __launch_bounds__(256, 3) k_features_warm(KParams p, int nvb, co
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint64_t mbar;
     __shared__ uint32_t tmem_slot;
-    __shared__ float sb[MLP_NUM_BIASES];
-    __shared__ float sw4[64];
+    __shared__ __align__(16) float sb[MLP_NUM_BIASES];
+    __shared__ __align__(16) float sw4[64];
     __shared__ float s_lam[256];
-    const int t = threadIdx.x, warp = t >> 5;
+    const int t = threadIdx.x;
     const int R = blockDim.x / L;            // particles per tile of slots: rows
     const int tiles = (R + 127) >> 7;        // 128-row MMA tiles
     const uint32_t cols = tiles > 1 ? 128u : 64u;
     uint8_t* sX = smem + FW_SX;
     uint8_t* sH = sX + tiles * FW_X_TILE;
-    if (warp == 0) tmem_alloc(&tmem_slot, cols);
-    if (t == 0) mbar_init(&mbar, 1);
-    stage_weight(smem + FW_SW1, io.w + W1_OFF, 64, 16);
-    stage_weight(smem + FW_SW2, io.w + W2_OFF, 64, 64);
-    stage_weight(smem + FW_SW3, io.w + W3_OFF, 64, 64);
-    for (int i = t; i < MLP_NUM_BIASES; i += blockDim.x) sb[i] = io.b[i];
-    if (t < 64) sw4[t] = bf16_val(io.w[W4_OFF + t]);
     // rows of the last tile past R stay zero
     for (int i = t; i < tiles * FW_X_TILE / 16; i += blockDim.x)
         reinterpret_cast<uint4*>(sX)[i] = make_uint4(0u, 0u, 0u, 0u);
-    fence_before_sync();
-    __syncthreads();
-    fence_after_sync();
-    const uint32_t tbase = tmem_slot;
-    const bool ep_warp = (warp >> 2) < tiles;  // this warp's TMEM quarter holds rows of a tile
-    const uint32_t lane_base = tmem_addr(tbase, 32 * (warp & 3), 64 * (warp >> 2));
-    uint8_t* my_h = sH + (warp >> 2) * FW_H_TILE;
+    const uint32_t tbase = warm_setup(io, smem, &mbar, &tmem_slot, sb, sw4, cols);
     uint32_t phase = 0;
     bool alive = true;
     for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
@@ -596,87 +704,75 @@ __global__ void __launch_bounds__(256, 3) k_features_warm(KParams p, int nvb, co
         const bool have = features_one<L, V>(p, tm, x, v, nbr, ncnt, lam_prev, xl, feat, lam_acc, f, lam);
         if (tm.t == 0) {
             const int row = t / L;
-            float xf[16];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) xf[i] = 0.0f;
-            if (have) {
-#pragma unroll
-                for (int i = 0; i < MLP_IN; ++i) xf[i] = (f[i] - sb[FMEAN_OFF + i]) * sb[FISTD_OFF + i];
-            }
-            uint32_t pk[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                pk[i] = (uint32_t)bf16_bits(xf[2 * i]) | ((uint32_t)bf16_bits(xf[2 * i + 1]) << 16);
+            uint32_t pk[8] = {};
+            if (have) pack_row(f, sb, pk);
             uint8_t* xt = sX + (row >> 7) * FW_X_TILE;
             *reinterpret_cast<uint4*>(xt + kmajor_offset(row & 127, 0, 128)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
             *reinterpret_cast<uint4*>(xt + kmajor_offset(row & 127, 8, 128)) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
             s_lam[row] = lam;
         }
         if (!alive) continue;  // an expired wait: no more tensor-core work (the error bit is set)
-        // three hidden layers; layer l reads X (l = 0) or H and writes H (l < 2)
-        float y = sb[B4_OFF];
-        // row t's plain lambda, read after the first barrier (its team leader
+        // row t's plain lambda is read after the first barrier (its team leader
         // wrote it) and before the second (after which that leader may write
         // the next tile's)
-        float lam_plain = 0.0f;
-#pragma unroll 1
-        for (int l = 0; l < 3; ++l) {
-            sync_for_mma();
-            if (l == 0 && t < R) lam_plain = s_lam[t];
-            if (t == 0) {
-                for (int j = 0; j < tiles; ++j) {
-                    if (l == 0) gemm_issue(tbase + 64 * j, sX + j * FW_X_TILE, smem + FW_SW1, 64, 16, 0);
-                    else gemm_issue(tbase + 64 * j, sH + j * FW_H_TILE, smem + (l == 1 ? FW_SW2 : FW_SW3), 64, 64, 0);
-                }
-                commit(&mbar);
-            }
-            if (!wait_mma(&mbar, phase, io.err)) {
-                alive = false;
-                break;
-            }
-            if (ep_warp) {
-                const float* bias = sb + (l == 0 ? B1_OFF : l == 1 ? B2_OFF : B3_OFF);
-#pragma unroll 1
-                for (int c = 0; c < 4; ++c) {
-                    float vv[16];
-                    tmem_ld16(lane_base + 16 * c, vv);
-                    tmem_wait_ld();
-#pragma unroll
-                    for (int i = 0; i < 16; i += 2) {
-                        const float2 hh =
-                            gelu2(vadd(make_float2(vv[i], vv[i + 1]),
-                                       make_float2(bias[16 * c + i], bias[16 * c + i + 1])));
-                        vv[i] = hh.x;
-                        vv[i + 1] = hh.y;
-                    }
-                    if (l < 2) {
-                        put_row64(my_h, t & 127, vv, 16 * c);
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) y = __fmaf_rn(vv[i], sw4[16 * c + i], y);
-                    }
-                }
-            }
-        }
+        float y, lam_plain = 0.0f;
+        alive = warm_layers(io, smem, sX, FW_X_TILE, sH, tiles, tbase, &mbar, phase, sb, sw4, y, [&] {
+            if (t < R) lam_plain = s_lam[t];
+        });
         if (!alive) continue;
         const int k = vb * R + t;
-        if (t < R && k < p.n) {
-            float l0 = y * sb[OSCALE_OFF];
-            if (io.clamp > 0.0f) {
-                // trust region around the plain lambda of this pass: same sign,
-                // at most clamp times its magnitude
-                const float a = io.clamp * lam_plain;
-                const float f0 = io.floor ? lam_plain : 0.0f;  // the weak end of the interval
-                l0 = fminf(fmaxf(l0, fminf(a, f0)), fmaxf(a, f0));
-            }
-            reinterpret_cast<float*>(xl)[4 * (size_t)k + 3] = l0;
-            lam_acc[k] = l0;
-            io.lam0[k] = l0;
-        }
+        if (t < R && k < p.n) warm_store(io, sb, k, y, lam_plain, xl, lam_acc);
     }
     fence_before_sync();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tbase, cols);
+    if (t < 32) tmem_dealloc(tbase, cols);
+}
+
+// The network over rows that k_features wrote: 256 rows (two tiles) per step, X in
+// the first 4 KB of each tile's H (layer 0 has read it before its epilogue writes
+// there), the next step's rows loaded during this one's layers. 50 KB and 128 TMEM
+// columns: four blocks per SM. Bound by the GELU epilogues' instructions (2,000 per
+// row; 57 % of the issue slots, 43 % of the MUFU's): 262,144 rows take 27.2 us, 28.6
+// with one bias per shared load and no early loads, 29.3 in blocks of one tile.
+constexpr int WR_SMEM = FW_SX + 2 * FW_H_TILE;
+constexpr int WR_BLOCKS = 4;
+__global__ void __launch_bounds__(256, WR_BLOCKS) k_warm_rows(int n, const uint4* __restrict__ row_lo,
+                                                              const uint4* __restrict__ row_hi,
+                                                              float4* __restrict__ xl, float* __restrict__ lam_acc,
+                                                              WarmIO io) {
+    pdl_wait();
+    extern __shared__ __align__(1024) uint8_t smem[];
+    __shared__ uint64_t mbar;
+    __shared__ uint32_t tmem_slot;
+    __shared__ __align__(16) float sb[MLP_NUM_BIASES];
+    __shared__ __align__(16) float sw4[64];
+    const int t = threadIdx.x;
+    uint8_t* sH = smem + FW_SX;
+    uint8_t* xt = sH + (t >> 7) * FW_H_TILE;
+    const uint32_t tbase = warm_setup(io, smem, &mbar, &tmem_slot, sb, sw4, 128u);
+    uint32_t phase = 0;
+    uint4 lo = make_uint4(0u, 0u, 0u, 0u), hi = lo;
+    float next_plain = 0.0f;
+    const auto load = [&](int k) {
+        if (k < n) {
+            lo = row_lo[k];
+            hi = row_hi[k];
+            next_plain = lam_acc[k];
+        }
+    };
+    load(blockIdx.x * 256 + t);
+    for (int k = blockIdx.x * 256 + t; k - t < n; k += gridDim.x * 256) {
+        const float lam_plain = next_plain;
+        *reinterpret_cast<uint4*>(xt + kmajor_offset(t & 127, 0, 128)) = lo;
+        *reinterpret_cast<uint4*>(xt + kmajor_offset(t & 127, 8, 128)) = hi;
+        load(k + (int)gridDim.x * 256);
+        float y;
+        if (!warm_layers(io, smem, sH, FW_H_TILE, sH, 2, tbase, &mbar, phase, sb, sw4, y, [] {})) break;
+        if (k < n) warm_store(io, sb, k, y, lam_plain, xl, lam_acc);
+    }
+    fence_before_sync();
+    __syncthreads();
+    if (t < 32) tmem_dealloc(tbase, 128u);
 }
 
 // ---------------------------------------------------------------------------
@@ -1268,15 +1364,37 @@ void launch_features(const KParams& p, const float4* x, const float4* v, const i
     with_lanes(p.lanes, [&](auto c) {
         constexpr int L = decltype(c)::L, V = decltype(c)::V;
         const int b = team_blocks(p.n, L, p.block);
-        launch(p.pdl, k_features<L, V>, pass_grid(p, k_features<L, V>, b), p.block, 0, st, p, b, x, v, nbr, ncnt, lam_prev, xl,
-                                                                                 feat, lam_acc);
+        const auto k = k_features<false, L, V>;
+        launch(p.pdl, k, pass_grid(p, k, b), p.block, 0, st, p, b, x, v, nbr, ncnt, lam_prev, xl, feat, lam_acc,
+               (const float*)nullptr, (uint4*)nullptr, (uint4*)nullptr);
     });
 }
 
 int launch_features_warm(const KParams& p, const float4* x, const float4* v, const int* nbr, const int* ncnt,
                          const float* lam_prev, float4* xl, float* feat, float* lam_acc, const uint16_t* w,
-                         const float* b, float* lam0, float clamp, int floor, int* err, cudaStream_t st) {
+                         const float* b, float* lam0, float clamp, int floor, uint4* row_lo, uint4* row_hi, int* err,
+                         cudaStream_t st) {
     int rc = 0;
+    const WarmIO io{w, b, lam0, clamp, floor, err};
+    // In two launches above two blocks of 256 particles per SM: the gathers then have
+    // the L1 and the warps that the fused pass gives to the network's tiles (262,144
+    // particles: 34.7 + 27.2 us against 75.6; frames at 64,000 / 85,184 / 884,736
+    // particles: 219 / 258 / 1,593 us against 216 / 261 / 1,635). Below, one launch
+    // less is worth more (4,096: 128 us fused against 133).
+    if (p.n > 2 * 256 * sm_count()) {
+        if (cudaFuncSetAttribute(k_warm_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, WR_SMEM) != cudaSuccess)
+            return -1;
+        with_lanes(p.lanes, [&](auto c) {
+            constexpr int L = decltype(c)::L, V = decltype(c)::V;
+            const int nvb = team_blocks(p.n, L, p.block);
+            const auto k = k_features<true, L, V>;
+            launch(p.pdl, k, pass_grid(p, k, nvb), p.block, 0, st, p, nvb, x, v, nbr, ncnt, lam_prev, xl, feat, lam_acc,
+                   b, row_lo, row_hi);
+        });
+        const int steps = (p.n + 255) / 256;
+        return launch(p.pdl, k_warm_rows, std::min(steps, WR_BLOCKS * sm_count()), 256, WR_SMEM, st, p.n,
+                      (const uint4*)row_lo, (const uint4*)row_hi, xl, lam_acc, io);
+    }
     with_lanes(p.lanes, [&](auto c) {
         constexpr int L = decltype(c)::L, V = decltype(c)::V;
         const int rows = p.block / L;
@@ -1297,7 +1415,6 @@ int launch_features_warm(const KParams& p, const float4* x, const float4* v, con
                 per_sm = 1;
             grid = (int)std::min<long long>((long long)per_sm * sms, nvb);
         }
-        const WarmIO io{w, b, lam0, clamp, floor, err};
         launch(p.pdl, k_features_warm<L, V>, grid, p.block, smem, st, p, nvb, x, v, nbr, ncnt, lam_prev, xl, feat, lam_acc, io);
     });
     return rc;

@@ -4,11 +4,14 @@ blocks x 16), the search with eight threads up to 45,056, and the layout for a
 device that is not full up to 113,664 threads (148 SMs x 3 blocks x 256), a particle
 taking one, two or four threads with one or two, four and eight pair lanes. Also
 the searched lists where rows leave the grid, for cells from h/3 to 3h/2, and
-s_corr exponents other than four, which have kernels of their own."""
+s_corr exponents other than four, which have kernels of their own; and the warm
+start's first pass, one launch up to 75,776 particles (148 SMs x 2 x 256) and two
+above."""
 import numpy as np
 import pytest
+import torch
 
-from pbf_b200 import autotune, scenes
+from pbf_b200 import Solver, autotune, learned, scenes
 
 from test_gpu_parity import assert_substep_bitexact, make_pair
 
@@ -79,3 +82,32 @@ def test_search_around_the_grid_bitexact(cell, n):
     assert_substep_bitexact(s, orc)
     s.close()
     orc.close()
+
+
+@pytest.mark.parametrize("n,lanes,block,persistent,record", [(75776, 2, 256, 0, 0), (75777, 2, 256, 0, 1),
+                                                             (75777, 1, 128, 0, 0), (80001, 8, 256, 0, 1),
+                                                             (80001, 4, 64, 1, 0), (160000, 2, 256, 0, 0)])
+def test_warm_pass_in_two_launches_bitexact(n, lanes, block, persistent, record):
+    """lambda0, the total lambda and the state of the first pass with packed rows
+    between its launches against the path with FP32 features, bit for bit."""
+    sc = block_of(n)
+    rng = np.random.RandomState(n)
+    feat = torch.from_numpy(rng.normal(size=(2048, 12)).astype(np.float32)).cuda()
+    target = torch.from_numpy(rng.normal(size=2048).astype(np.float32)).cuda()
+    tr, _ = learned.train(feat, target, epochs=1, batch=1024, lr=2e-3)
+    _, b32, w16 = tr.params()
+    tr.close()
+    runs = []
+    for unfused in (0, 1):
+        s = Solver(sc.para, sc.grid_space, sc.boundary,
+                   sc.ext(warm_start=1, warm_unfused=unfused, pair_lanes=lanes, block_size=block,
+                          persistent=persistent, warm_clamp=0.0, record_features=record))
+        learned.install(s, w16, b32)
+        s.upload(sc.pos, sc.vel)
+        s.step(3)
+        assert s.stats()["error_bits"] == 0
+        runs.append({k: s.fetch(k) for k in ("lambda0", "lambda_total", "x", "v", "curl")})
+        s.close()
+    for k in runs[0]:
+        assert np.array_equal(runs[0][k].view(np.uint32), runs[1][k].view(np.uint32)), k
+    assert np.count_nonzero(runs[0]["lambda0"]) > n // 2
