@@ -743,7 +743,7 @@ int create_common(const pbf_solver_parameter* para, int nscenes, const pbf_scene
             return rc;                     \
         }                                  \
     } while (0)
-    AL(s->Sx, n); AL(s->Sv, n); AL(s->Px, n + 1); AL(s->Pv, n + 1); AL(s->Pxold, n); AL(s->Q, n + 1); AL(s->omega, n); AL(s->vw, n + 1);
+    AL(s->Sx, n); AL(s->Sv, n); AL(s->Px, n + SEARCH_SLACK); AL(s->Pv, n + 1); AL(s->Pxold, n); AL(s->Q, n + 1); AL(s->omega, n); AL(s->vw, n + 1);
     AL(s->Sperm, n); AL(s->Pperm, n); AL(s->cell, n); AL(s->ticket, n); AL(s->tmp, n); AL(s->cell_sorted, n);
     AL(s->ncnt, n);
     // (rows for the longest list padded to whole batches; slot n of the gathered arrays

@@ -376,15 +376,21 @@ __device__ __forceinline__ float cell_from(const KParams& p, float g, int t) {
 }
 
 // Stencil radius RR as a constant (1: cells of h, 2: cells of h/2; 0: any radius,
-// read from p.radius).
+// read from p.radius). Places in a list are 32-bit offsets from its first entry, in
+// units of 32 ints (the stride between entries is a multiple of that).
 //
 // For RR > 0 the pass is bound by instructions (a lane of a warp of 32 walks its
 // own rows, about 20 of 32 lanes are active), so they are what is saved: the
 // distances to the cells beside the particle's own are squared once per particle
-// and a row's range is a few compares; candidates go two per step, a step without
-// branches (predicated stores); the particle itself is left out by splitting its
-// own row's range, and the cap is tested per row. 262,144 particles, cells of h/2:
-// 67.8 us -> 55.8 (47.4 M -> 38.8 M warp instructions); cells of h: 79 -> 72.
+// and a row's range is a few compares; candidates go two or four per step, a step
+// without branches (predicated stores); the particle itself is left out by splitting
+// its own row's range, and the cap is tested per row. 262,144 particles, cells of
+// h/2: 67.8 us -> 52.6 (57.1 with the entries counted and multiplied by the stride,
+// 53.6 with byte offsets); cells of h: 79 -> 64.
+//
+// Candidates per step: rows hold 3-4 in cells of h/2, where four per step only add
+// instructions (64 scenes, 1.3 M particles: 225 us with two, 240 with four), and 10 or more
+// in cells of h (262,144 particles: 76 us with two, 64 with four, 67 with six).
 template <int RR>
 __device__ __forceinline__ void neighbors_one(const KParams& p, int k, const float4* __restrict__ x,
                                               const int* __restrict__ cell_start, int* __restrict__ nbr,
@@ -398,41 +404,72 @@ __device__ __forceinline__ void neighbors_one(const KParams& p, int k, const flo
     const int cap = p.max_nbr;
     const float m = p.h * 1e-3f + 1e-6f * (fabsf(xk.x) + fabsf(xk.y) + fabsf(xk.z));
     const float hm2 = (p.h + m) * (p.h + m);
-    int c = 0;
+    // entry i of the list is i step units after entry 0
+    const unsigned step = (unsigned)p.stride / 32, last = (unsigned)cap * step;
+    unsigned o = 0;  // of the next entry
     int* __restrict__ list = nbr + k;
-    // candidates [s, e) in slot order, two at a time: |r|^2 as dot_fma gives it,
-    // packed. The second of an odd range's last two reads one slot further (the
-    // position arrays are one slot longer than the particles) and is dropped.
+    auto at = [&](unsigned i) { return list + (size_t)i * 32; };
+    const float h2 = p.h2;
+    // candidates [s, e) in slot order, two or four at a time: |r|^2 as dot_fma gives
+    // it, packed. The last step of a range may read slots after it (the position
+    // array has SEARCH_SLACK slots more than there are particles) and drops them.
+    auto r2_pair = [&](const float4& a0, const float4& a1) {
+        const float2 rx = make_float2(xk.x - a0.x, xk.x - a1.x), ry = make_float2(xk.y - a0.y, xk.y - a1.y),
+                     rz = make_float2(xk.z - a0.z, xk.z - a1.z);
+        return vfma(rz, rz, vfma(ry, ry, vmul(rx, rx)));
+    };
     auto scan = [&](int s, int e) {
         const float4* q = x + s;
-        for (int j = s; j < e; j += 2, q += 2) {
-            const float4 a0 = q[0], a1 = q[1];
-            const float2 rx = make_float2(xk.x - a0.x, xk.x - a1.x), ry = make_float2(xk.y - a0.y, xk.y - a1.y),
-                         rz = make_float2(xk.z - a0.z, xk.z - a1.z);
-            const float2 d2 = vfma(rz, rz, vfma(ry, ry, vmul(rx, rx)));
-            if (d2.x <= p.h2) {
-                list[(size_t)((unsigned)c * (unsigned long long)(unsigned)p.stride)] = j;
-                ++c;
+        if constexpr (RR == 1) {
+            for (int j = s; j < e; j += 4, q += 4) {
+                const float4 a0 = q[0], a1 = q[1], a2 = q[2], a3 = q[3];
+                const float2 d01 = r2_pair(a0, a1), d23 = r2_pair(a2, a3);
+                const int left = e - j;
+                if (d01.x <= h2) {
+                    *at(o) = j;
+                    o += step;
+                }
+                if (d01.y <= h2 && left > 1) {
+                    *at(o) = j + 1;
+                    o += step;
+                }
+                if (d23.x <= h2 && left > 2) {
+                    *at(o) = j + 2;
+                    o += step;
+                }
+                if (d23.y <= h2 && left > 3) {
+                    *at(o) = j + 3;
+                    o += step;
+                }
             }
-            if (d2.y <= p.h2 && j + 1 < e) {
-                list[(size_t)((unsigned)c * (unsigned long long)(unsigned)p.stride)] = j + 1;
-                ++c;
+        } else {
+            for (int j = s; j < e; j += 2, q += 2) {
+                const float4 a0 = q[0], a1 = q[1];
+                const float2 d01 = r2_pair(a0, a1);
+                if (d01.x <= h2) {
+                    *at(o) = j;
+                    o += step;
+                }
+                if (d01.y <= h2 && j + 1 < e) {
+                    *at(o) = j + 1;
+                    o += step;
+                }
             }
         }
     };
     // the same near the cap
     auto scan_capped = [&](int s, int e) {
-        for (int j = s; j < e && c < cap; ++j) {
+        for (int j = s; j < e && o < last; ++j) {
             const float4 a0 = x[j];
             const f3 r = {xk.x - a0.x, xk.y - a0.y, xk.z - a0.z};
-            if (dot_fma(r, r) <= p.h2) {
-                list[(size_t)c * p.stride] = j;
-                ++c;
+            if (dot_fma(r, r) <= h2) {
+                *at(o) = j;
+                o += step;
             }
         }
     };
     auto scan_row = [&](int s, int e) {
-        if (c + (e - s) <= cap) scan(s, e);
+        if (o + (unsigned)min(e - s, cap + 1) * step <= last) scan(s, e);
         else scan_capped(s, e);
     };
     if (RR > 0) {
@@ -462,7 +499,7 @@ __device__ __forceinline__ void neighbors_one(const KParams& p, int k, const flo
         // stencil reaches)
         const bool in_x = d[0] >= 0 && d[0] < nx;
         const int x0 = max(d[0] - RR, 0), x1 = min(d[0] + RR, nx - 1);
-        for (int dz = -RR; dz <= RR && c < cap && x0 <= x1; ++dz) {
+        for (int dz = -RR; dz <= RR && o < last && x0 <= x1; ++dz) {
             const int z = d[2] + dz;
             if (z < 0 || z >= nz) continue;
             const float ez2 = dz == 0 ? 0.0f : dz < 0 ? below(xk.z, sc.gmin[2], d[2], -dz) : above(xk.z, sc.gmin[2], d[2], dz);
@@ -504,7 +541,7 @@ __device__ __forceinline__ void neighbors_one(const KParams& p, int k, const flo
     } else {
         const int R = p.radius;
         const int x0 = max(d[0] - R, 0), x1 = min(d[0] + R, nx - 1);
-        for (int dz = -R; dz <= R && c < cap && x0 <= x1; ++dz) {
+        for (int dz = -R; dz <= R && o < last && x0 <= x1; ++dz) {
             const int z = d[2] + dz;
             if (z < 0 || z >= nz) continue;
             // distance from the particle to the z slab of this plane of cells
@@ -512,7 +549,7 @@ __device__ __forceinline__ void neighbors_one(const KParams& p, int k, const flo
                                     : xk.z - (sc.gmin[2] + (float)(z + 1) * p.cell);
             const float ez = dz == 0 ? 0.0f : fmaxf(gz - m, 0.0f);
             if (ez * ez > hm2) continue;
-            for (int dy = -R; dy <= R && c < cap; ++dy) {
+            for (int dy = -R; dy <= R && o < last; ++dy) {
                 const int y = d[1] + dy;
                 if (y < 0 || y >= ny) continue;
                 const float gy = dy > 0 ? cell_from(p, sc.gmin[1], y) - xk.y
@@ -539,8 +576,9 @@ __device__ __forceinline__ void neighbors_one(const KParams& p, int k, const flo
             }
         }
     }
+    int c = (int)(o / step);
     ncnt[k] = c;
-    for (; c % p.pad != 0; ++c) list[(size_t)c * p.stride] = p.pad_slot;
+    for (; (c & (p.pad - 1)) != 0; ++c, o += step) *at(o) = p.pad_slot;
 }
 
 // nvb tiles of blockDim.x slots; the grid strides over them (a grid of nvb
@@ -1022,21 +1060,24 @@ template <typename K> static int resident_grid(const KParams& p, K kernel, int n
     return (int)(g < nvb ? g : nvb);
 }
 
-// Particles up to which SEARCH_WIDE threads share one (cells of h/2: 17.0 us against
-// 22.5 at 32,768 particles, 23.0 against 23.1 at 46,656, 28.8 against 24.6 at 64,000).
-constexpr int SEARCH_WIDE_MAX_N = 45056;
+// Particles up to which SEARCH_WIDE threads share one: its time grows with the
+// particles, one thread's walk takes the same until the device is full. Cells of h/2,
+// shared against not: 18.2 / 20.6 us at 32,768 particles, 20.1 / 20.5 at 39,304, 22.9 /
+// 21.1 at 46,656; cells of h: 14.0 / 14.9 at 13,824, 17.6 / 15.2 at 21,952.
+constexpr int SEARCH_WIDE_MAX_N[3] = {0, 16384, 40960};  // by stencil radius
 
 void launch_neighbors(const KParams& p, const float4* x, const int* cell_start, int* nbr, int* ncnt, cudaStream_t st) {
-    if (p.n <= SEARCH_WIDE_MAX_N && !p.persistent && p.radius <= 2) {
+    if (p.radius <= 2 && p.n <= SEARCH_WIDE_MAX_N[p.radius] && !p.persistent) {
         const int b = blocks_for(p.n, SEARCH_WIDE_THREADS / SEARCH_WIDE);
         if (p.radius == 1) launch(p.pdl, k_neighbors_wide<1>, b, SEARCH_WIDE_THREADS, 0, st, p, x, cell_start, nbr, ncnt);
         else launch(p.pdl, k_neighbors_wide<2>, b, SEARCH_WIDE_THREADS, 0, st, p, x, cell_start, nbr, ncnt);
         return;
     }
     const int b = blocks_for(p.n, p.block);
-    if (p.radius == 1) launch(p.pdl, k_neighbors<1>, resident_grid(p, k_neighbors<1>, b), p.block, 0, st, p, b, x, cell_start, nbr, ncnt);
-    else if (p.radius == 2) launch(p.pdl, k_neighbors<2>, resident_grid(p, k_neighbors<2>, b), p.block, 0, st, p, b, x, cell_start, nbr, ncnt);
-    else launch(p.pdl, k_neighbors<0>, resident_grid(p, k_neighbors<0>, b), p.block, 0, st, p, b, x, cell_start, nbr, ncnt);
+    auto go = [&](auto k) { launch(p.pdl, k, resident_grid(p, k, b), p.block, 0, st, p, b, x, cell_start, nbr, ncnt); };
+    if (p.radius == 1) go(k_neighbors<1>);
+    else if (p.radius == 2) go(k_neighbors<2>);
+    else go(k_neighbors<0>);
 }
 
 void launch_gather_rows(const int* slots, int count, int n, const float* feat, const float* lam_acc, float* out_feat,

@@ -35,6 +35,8 @@ void launch_scatter(bool pdl, int n, const int* cell, const int* ticket, const i
 void launch_reorder(const KParams& p, bool predict_on, const float4* x, const float4* v, const int* perm,
                     const int* cell, const int* cell_start, const int* tmp, float4* xp, float4* vp, float4* xold,
                     int* perm_out, int* cell_sorted, const float* lam_in, float* lam_out, int* err, cudaStream_t st);
+// x has SEARCH_SLACK slots more than there are particles (read and dropped).
+constexpr int SEARCH_SLACK = 4;
 void launch_neighbors(const KParams& p, const float4* x, const int* cell_start, int* nbr, int* ncnt, cudaStream_t st);
 void launch_lambda(const KParams& p, bool debug, const float4* x, const int* nbr, const int* ncnt, float4* xl,
                    float* rho, const IterCtl& ctl, cudaStream_t st);

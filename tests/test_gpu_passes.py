@@ -1,6 +1,7 @@
 """The neighbour passes at the sizes where their variants change, bit for bit
 against the oracle: eight threads per particle up to 9,472 particles (148 SMs x 4
-blocks x 16), the search with eight threads up to 45,056, and the layout for a
+blocks x 16), the search with eight threads up to 40,960 (16,384
+in cells of h), and the layout for a
 device that is not full up to 113,664 threads (148 SMs x 3 blocks x 256), a particle
 taking one, two or four threads with one or two, four and eight pair lanes. Also
 the searched lists where rows leave the grid, for cells from h/3 to 3h/2, and
@@ -29,6 +30,7 @@ def block_of(n, iters=2):
 
 @pytest.mark.parametrize("n,lanes,cell", [(9472, 2, 0.5), (9473, 2, 0.5), (9472, 1, 1.0), (9473, 1, 1.0),
                                           (9473, 4, 0.5), (9473, 8, 0.5), (45056, 2, 0.5), (45057, 2, 1.0),
+                                          (16384, 2, 1.0), (16385, 2, 1.0), (40960, 2, 0.5), (40961, 2, 0.5),
                                           (56833, 4, 0.5), (28417, 8, 0.5), (113664, 2, 0.5), (113665, 2, 0.5),
                                           (113665, 1, 1.0), (113664, 1, 0.5)])
 def test_variant_boundaries_bitexact(n, lanes, cell):
