@@ -465,7 +465,11 @@ int enqueue_substep(pbf_solver* s, cudaStream_t st) {
     const bool warm = s->ext.warm_start && s->mlp_w;
     const bool feats = warm || s->ext.record_features;
     P(ST_REORDER, [&] {
-        launch_reorder(kp, true, s->Sx, s->Sv, s->Sperm, s->cell, s->cell_start, s->tmp, s->Px, s->Pv, s->Pxold,
+        // (corrections write the velocities anew from the positions; only the feature
+        // pass, or curl with no correction before it, reads the predicted ones: 4.7 M
+        // particles 122 -> 97 us without them)
+        float4* vp = feats || s->para.iterations == 0 ? s->Pv : nullptr;
+        launch_reorder(kp, true, s->Sx, s->Sv, s->Sperm, s->cell, s->cell_start, s->tmp, s->Px, vp, s->Pxold,
                        s->Pperm, s->cell_sorted, feats ? s->lam_acc : nullptr, feats ? s->lam_prev_sorted : nullptr,
                        err, st);
     });

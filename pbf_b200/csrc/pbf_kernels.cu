@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(256, 8) k_reorder(KParams p, const float4* __r
     f3 vi = make3(v[i]);
     if (PREDICT) predict(p, sc, xi, vi);
     xp[dst] = make_float4(xi.x, xi.y, xi.z, 0.0f);
-    vp[dst] = make_float4(vi.x, vi.y, vi.z, 0.0f);
+    if (vp) vp[dst] = make_float4(vi.x, vi.y, vi.z, 0.0f);
     xold[dst] = make_float4(x4.x, x4.y, x4.z, 0.0f);
     perm_out[dst] = perm[i];
     cell_sorted[dst] = c;

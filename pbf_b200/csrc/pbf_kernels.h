@@ -32,6 +32,8 @@ void launch_scan_silent_tile(const int* in, int* out, int m, void* status_ws, in
 // (pdl here and KParams::pdl: programmatic dependent launch on the kernel before)
 void launch_scatter(bool pdl, int n, const int* cell, const int* ticket, const int* cell_start, int* tmp, int* err,
                     cudaStream_t st);
+// vp may be null: the velocities are then not written (a substep with corrections and
+// without features takes them from the corrected positions).
 void launch_reorder(const KParams& p, bool predict_on, const float4* x, const float4* v, const int* perm,
                     const int* cell, const int* cell_start, const int* tmp, float4* xp, float4* vp, float4* xold,
                     int* perm_out, int* cell_sorted, const float* lam_in, float* lam_out, int* err, cudaStream_t st);
