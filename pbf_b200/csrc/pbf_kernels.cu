@@ -84,35 +84,69 @@ __global__ void __launch_bounds__(256, 8) k_hash(KParams p, const float4* __rest
 // ticket, so every predecessor is already running and the wait always ends; the
 // wait is bounded anyway and reports DEVERR_SCAN_TIMEOUT.
 //
-// The workspace is the status words, then the ticket counter and the epoch. With
-// KEEP (the solver's own workspace, zeroed once) the last ticket's block resets
-// the counter and advances the epoch, which invalidates this run's words, so a
-// substep needs no memset; other callers' workspaces are cleared before the launch.
+// The workspace is the status words, then the ticket counter. With KEEP (the
+// solver's own workspace, zeroed once, its scans all of one size) tickets go on from
+// run to run and the epoch is a ticket's run, which invalidates the words of the run
+// before, so a substep needs no memset; other callers' workspaces are cleared before
+// the launch.
 // KEEP also writes the cleared counts only where there were any: most cells of a
 // large grid are empty, and the pass is bound by its bytes (65.6 M keys, 4.7 M
 // particles: 194 us -> 144 us with 524 MB instead of 786).
 // ---------------------------------------------------------------------------
 constexpr long long SCAN_SPIN_LIMIT = 1ll << 22;
+// What the pass waits for is the chain of prefixes, so a tile publishes its aggregate
+// before it scans its items, one atomic gives tile and epoch, and the words are
+// relaxed accesses (5 M counts: 13.2 us -> 9.9; 65.6 M keys: 148 -> 131; 25,000: 4.4
+// -> 3.3). More words per poll cost more than the hops they save (65.6 M keys, two and
+// four per lane: 138 and 162 us), a window of the whole block more again (302).
 // Tiles of 8,192 counts, or of 16,384 above 2^22 counts, where half as many tiles
-// shorten the look-back chains (65.6 M keys, mostly empty: 144 us against 173 with
-// 8,192 and 234 with 4,096). The solver's own scan takes 4,096 up to 2^19 counts,
-// where 8,192 leave most SMs idle (25,000 keys: 4.3 against 4.7 us; 1.02 M keys:
-// 8.8 against 7.4). A look-back window of the whole block instead of a warp was
-// slower at every size (two barriers per window and more polls: 1.02 M keys 10.4
-// against 8.8 us at 4,096, 65.6 M keys 302 against 234).
+// make a shorter chain (65.6 M keys, mostly empty: 131 us against 165 with 8,192 and
+// 191 with 4,096; 5 M counts: 9.9 against 13.2 and 13.5). The solver's own scan takes
+// 4,096 up to 2^19 counts, where 8,192 leave most SMs idle (1.02 M keys: 5.8 us with
+// 8,192, 7.3 with 4,096).
 constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_SMALL_MAX = 1 << 19;
 constexpr int SCAN_LARGE_MIN = (1 << 22) + 1;
 static int scan_tile(int m) { return m >= SCAN_LARGE_MIN ? 16384 : 8192; }
 constexpr unsigned SCAN_EPOCHS = 1u << 30;
 
-__device__ __forceinline__ void st_release_u64(unsigned long long* a, unsigned long long v) {
-    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(a), "l"(v) : "memory");
+// Status words carry their value with them and order nothing else: relaxed accesses.
+__device__ __forceinline__ void st_status(unsigned long long* a, unsigned long long v) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(a), "l"(v) : "memory");
 }
-__device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long* a) {
+__device__ __forceinline__ unsigned long long ld_status(const unsigned long long* a) {
     unsigned long long v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(a) : "memory");
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(a) : "memory");
     return v;
+}
+
+// Sum of all tiles before `tile`, by one whole warp: windows of 32 predecessors, the
+// nearest on lane 0. A window is polled until the words up to its nearest inclusive
+// prefix (or all of them) are there. False, with the sum so far, when spin_limit
+// polls of a window did not suffice.
+__device__ __forceinline__ bool look_back(const unsigned long long* status, int tile, unsigned long long ep,
+                                          long long spin_limit, int& excl) {
+    const int lane = threadIdx.x & 31;
+    excl = 0;
+    for (int pos = tile - 1; pos >= 0; pos -= 32) {
+        for (long long spins = 0;; ++spins) {
+            const unsigned long long w =
+                pos >= lane ? ld_status(&status[pos - lane]) : ep | (2ull << 32);  // before tile 0: an empty prefix
+            const unsigned flag = (w & ~0x3ffffffffull) == ep ? (unsigned)(w >> 32) & 3u : 0u;
+            const unsigned there = __ballot_sync(0xffffffffu, flag != 0u), prefix = __ballot_sync(0xffffffffu, flag == 2u);
+            const int last = prefix ? __ffs(prefix) - 1 : 31;  // lanes up to here count
+            const bool wait = (~there & (0xffffffffu >> (31 - last))) != 0u;
+            if (wait && spins < spin_limit) {
+                __nanosleep(32);
+                continue;
+            }
+            excl += __reduce_add_sync(0xffffffffu, flag != 0u && lane <= last ? (int)(unsigned)w : 0);
+            if (wait) return false;
+            if (prefix) return true;
+            break;
+        }
+    }
+    return true;
 }
 
 // VEC: cnt and out are 16-byte aligned; each lane moves four consecutive counts
@@ -131,17 +165,12 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan(int* __restrict__ cnt, in
     __shared__ int s_excl;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     if (t == 0) {
-        int* counter = reinterpret_cast<int*>(status + tiles);
-        unsigned* epoch = reinterpret_cast<unsigned*>(counter + 1);
-        const unsigned e = KEEP ? *reinterpret_cast<volatile unsigned*>(epoch) : 0u;
-        __threadfence();  // the epoch is read before the ticket that lets it advance
-        const int tile = atomicAdd(counter, 1);
-        if (KEEP && tile == tiles - 1) {  // every block has its ticket and its epoch
-            *counter = 0;
-            *epoch = (e + 1) % SCAN_EPOCHS;
-        }
+        const unsigned long long ticket = atomicAdd(status + tiles, 1ull);
+        // (without KEEP the counter starts from zero)
+        const unsigned long long e = !KEEP ? 0ull : ticket >> 32 ? ticket / (unsigned)tiles : (unsigned)ticket / (unsigned)tiles;
+        const int tile = (int)(ticket - e * (unsigned)tiles);
         s_tile = tile;
-        s_epoch = e;
+        s_epoch = (unsigned)(e % SCAN_EPOCHS);
     }
     __syncthreads();
     const int tile = s_tile;
@@ -154,7 +183,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan(int* __restrict__ cnt, in
     // round is scanned across the warp and carried into the next.
     const long long wbase = (long long)tile * TILE + (long long)warp * (32 * ITEMS);
     int item[ITEMS];
-    int carry = 0;  // warp-exclusive offset of the round
+    int sum = 0;
     unsigned filled = 0u;  // rounds (int4 groups) of this lane that hold a count
     if (VEC) {
 #pragma unroll
@@ -170,9 +199,39 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan(int* __restrict__ cnt, in
         }
 #pragma unroll
         for (int r = 0; r < ITEMS / 4; ++r) {
+            const int tot = item[4 * r] + item[4 * r + 1] + item[4 * r + 2] + item[4 * r + 3];
+            if (KEEP) filled |= tot != 0 ? 1u << r : 0u;
+            sum += tot;
+        }
+    } else {
+#pragma unroll
+        for (int q = 0; q < ITEMS; ++q) {
+            const long long idx = wbase + q * 32 + lane;
+            item[q] = idx < m ? cnt[idx] : 0;
+            sum += item[q];
+        }
+    }
+    // the tile's aggregate first, for the tiles that wait for it
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if (lane == 0) s_warp[warp] = sum;  // the warp's total
+    __syncthreads();
+    // every thread: the sum of the warps before its own, and of all
+    int before = 0, total = 0;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) {
+        const int v = s_warp[w];
+        before += w < warp ? v : 0;
+        total += v;
+    }
+    const bool publish = tile != silent_tile;
+    if (t == 0 && publish) st_status(&status[tile], ep | ((tile == 0 ? 2ull : 1ull) << 32) | (unsigned)total);
+    // exclusive prefixes within the warp's range, round by round
+    int carry = 0;
+    if (VEC) {
+#pragma unroll
+        for (int r = 0; r < ITEMS / 4; ++r) {
             const int a0 = item[4 * r], a1 = a0 + item[4 * r + 1], a2 = a1 + item[4 * r + 2];
             const int tot = a2 + item[4 * r + 3];
-            if (KEEP) filled |= tot != 0 ? 1u << r : 0u;
             int incl = tot;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -181,17 +240,12 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan(int* __restrict__ cnt, in
             }
             const int ex = carry + incl - tot;
             carry += __shfl_sync(0xffffffffu, incl, 31);
-            item[4 * r] = ex;  // exclusive prefixes within the warp's range
+            item[4 * r] = ex;
             item[4 * r + 1] = ex + a0;
             item[4 * r + 2] = ex + a1;
             item[4 * r + 3] = ex + a2;
         }
     } else {
-#pragma unroll
-        for (int q = 0; q < ITEMS; ++q) {
-            const long long idx = wbase + q * 32 + lane;
-            item[q] = idx < m ? cnt[idx] : 0;
-        }
 #pragma unroll
         for (int q = 0; q < ITEMS; ++q) {
             int incl = item[q];
@@ -202,60 +256,24 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan(int* __restrict__ cnt, in
             }
             const int excl_q = carry + incl - item[q];
             carry += __shfl_sync(0xffffffffu, incl, 31);
-            item[q] = excl_q;  // now the exclusive prefix within the warp's range
+            item[q] = excl_q;
         }
     }
-    if (lane == 0) s_warp[warp] = carry;  // the warp's total
-    __syncthreads();
-    // every thread: the sum of the warps before its own, and of all
-    int before = 0, total = 0;
-#pragma unroll
-    for (int w = 0; w < WARPS; ++w) {
-        const int v = s_warp[w];
-        before += w < warp ? v : 0;
-        total += v;
-    }
-    // decoupled look-back by one warp, 32 predecessors per window
-    const bool publish = tile != silent_tile;
-    if (t == 0 && publish)
-        st_release_u64(&status[tile], ep | ((tile == 0 ? 2ull : 1ull) << 32) | (unsigned)total);
     if (warp == 0) {
-        int excl = 0;
-        bool done = tile == 0;
-        for (int pos = tile - 1; !done; pos -= 32) {
-            const int look = pos - lane;
-            bool prefix = true;  // before tile 0: an empty prefix
-            int val = 0;
-            if (look >= 0) {
-                long long spins = 0;
-                unsigned long long s = ld_acquire_u64(&status[look]);
-                while ((s & ~0x3ffffffffull) != ep || ((s >> 32) & 3ull) == 0ull) {
-                    if (++spins > spin_limit) {
-                        atomicOr(err, DEVERR_SCAN_TIMEOUT);
-                        if (host_err) *(volatile int*)host_err = DEVERR_SCAN_TIMEOUT;
-                        s = 2ull << 32;  // give up: treat as prefix 0 so the tile finishes
-                        break;
-                    }
-                    __nanosleep(32);
-                    s = ld_acquire_u64(&status[look]);
-                }
-                prefix = ((s >> 32) & 3ull) == 2ull;
-                val = (int)(unsigned)(s & 0xffffffffull);
+        int e;
+        const bool ok = look_back(status, tile, ep, spin_limit, e);
+        if (lane == 0) {
+            s_excl = e;
+            if (!ok) {
+                atomicOr(err, DEVERR_SCAN_TIMEOUT);
+                if (host_err) *(volatile int*)host_err = DEVERR_SCAN_TIMEOUT;
             }
-            const unsigned pm = __ballot_sync(0xffffffffu, prefix);
-            const int stop = pm ? __ffs(pm) - 1 : 31;
-            int contrib = lane <= stop ? val : 0;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) contrib += __shfl_xor_sync(0xffffffffu, contrib, o);
-            excl += contrib;
-            done = pm != 0u;
         }
-        if (lane == 0) s_excl = excl;
     }
     __syncthreads();
     const int excl = s_excl;
     if (t == 0 && publish && tile > 0)
-        st_release_u64(&status[tile], ep | (2ull << 32) | (unsigned)(excl + total));
+        st_status(&status[tile], ep | (2ull << 32) | (unsigned)(excl + total));
     const int off = excl + before;
     if (VEC) {
 #pragma unroll

@@ -1,8 +1,7 @@
 """The neighbour passes at the sizes where their variants change, bit for bit
 against the oracle: eight threads per particle up to 9,472 particles (148 SMs x 4
-blocks x 16), the search with eight threads up to 40,960 (16,384
-in cells of h), and the layout for a
-device that is not full up to 113,664 threads (148 SMs x 3 blocks x 256), a particle
+blocks x 16), the search with eight threads up to 40,960 (16,384 in
+cells of h), and the layout for a device that is not full up to 113,664 threads (148 SMs x 3 blocks x 256), a particle
 taking one, two or four threads with one or two, four and eight pair lanes. Also
 the searched lists where rows leave the grid, for cells from h/3 to 3h/2, and
 s_corr exponents other than four, which have kernels of their own; and the warm
@@ -14,7 +13,7 @@ import torch
 
 from pbf_b200 import Solver, autotune, learned, scenes
 
-from test_gpu_parity import assert_substep_bitexact, make_pair
+from test_gpu_parity import assert_substep_bitexact, make_pair, mismatch
 
 pytestmark = pytest.mark.gpu
 
@@ -40,6 +39,22 @@ def test_variant_boundaries_bitexact(n, lanes, cell):
     s.step(1)
     orc.substep()
     assert_substep_bitexact(s, orc)
+    s.close()
+    orc.close()
+
+
+@pytest.mark.parametrize("n", [1200, 46000])
+def test_no_corrections_bitexact(n):
+    """A substep without corrections keeps the predicted velocities, over several
+    substeps (the scan's status words outlive each)."""
+    sc = block_of(n, iters=0)
+    s, orc = make_pair(sc)
+    s.step(3)
+    for _ in range(3):
+        orc.substep()
+    for f in ("x", "v", "curl"):
+        assert mismatch(s.fetch(f)[:, :3], orc.get(f))[0] == 0, f
+    assert np.array_equal(s.fetch("perm"), orc.get("perm"))
     s.close()
     orc.close()
 
