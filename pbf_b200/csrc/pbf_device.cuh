@@ -106,12 +106,14 @@ struct IterCtl {
     float* lam_acc;                // when set, the lambda pass adds its lambda here (the
                                    // substep's total lambda: warm-start feature and target)
     // device-side loop: the counter the other pass reads receives *loop_k + loop_add;
-    // the dp pass also sets the loop's condition (handle) for slots below max_slot
+    // the dp pass also sets the loop's condition (handle); passes at slots from max_slot
+    // on (the rest of a body that holds several corrections) do nothing
     int* loop_next = nullptr;
     int loop_add = 1;
     int max_slot = 0;
     cudaGraphConditionalHandle handle = 0;
     __device__ __forceinline__ int cur_slot() const { return loop_k ? slot + *loop_k : slot; }
+    __device__ __forceinline__ bool past_end() const { return loop_next && cur_slot() >= max_slot; }
 };
 
 // ---- deterministic sine ------------------------------------------------------

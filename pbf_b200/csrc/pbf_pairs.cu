@@ -364,7 +364,7 @@ __device__ __forceinline__ float lambda_list(const KParams& p, const Team<L>& tm
 // delta-p pass its counter.
 __device__ __forceinline__ bool lambda_skip(const IterCtl& ctl) {
     if (ctl.loop_next && blockIdx.x == 0 && threadIdx.x == 0) *ctl.loop_next = *ctl.loop_k + ctl.loop_add;
-    return ctl.done && *ctl.done;
+    return ctl.done && (*ctl.done || ctl.past_end());
 }
 
 // nvb tiles of blockDim.x slots' teams; the grid strides over them (a grid of
@@ -843,7 +843,7 @@ __device__ __forceinline__ bool dp_skip(const IterCtl& ctl) {
     // the lambda pass just measured the positions this pass would correct;
     // when they are within tolerance the loop ends here
     const int sl = ctl.cur_slot();
-    const bool over = *ctl.done != 0;
+    const bool over = *ctl.done != 0 || ctl.past_end();
     const bool met = !over && sl >= ctl.min_slot && __longlong_as_double((long long)ctl.max_bits[sl]) <= ctl.tol;
     if (lead) {
         if (met) {

@@ -59,6 +59,24 @@ def test_no_corrections_bitexact(n):
     orc.close()
 
 
+@pytest.mark.parametrize("tol", [1e-9, 0.02])
+@pytest.mark.parametrize("max_it", [1, 2, 3, 5, 6])
+@pytest.mark.parametrize("n", [1200, 12000])
+def test_adaptive_loop_ends_bitexact(n, max_it, tol):
+    """The correction loop, two corrections per body, ended by its cap or by the
+    tolerance after even and odd numbers of corrections."""
+    sc = block_of(n, iters=1)
+    s, orc = make_pair(sc, adaptive=1, density_tol=tol, max_iterations=max_it, debug=0)
+    for _ in range(3):
+        s.step(1)
+        want = orc.substep_adaptive(float(np.float32(tol)), 1, max_it)
+        assert s.stats()["last_iterations"] == want
+        for f in ("x", "v"):
+            assert mismatch(s.fetch(f)[:, :3], orc.get(f))[0] == 0, f
+    s.close()
+    orc.close()
+
+
 @pytest.mark.parametrize("exponent", [1.0, 3.0, 3.5])
 @pytest.mark.parametrize("n", [1200, 12000])
 def test_scorr_exponents_bitexact(n, exponent):
