@@ -65,7 +65,9 @@ __device__ __forceinline__ float dot3(float ax, float ay, float az, float bx, fl
 // small sprites). Most fragments lie behind what is already there, so a fragment
 // reads the pixel first, possibly a stale value, which is never below the current
 // one, and divides exactly and takes the atomic minimum only when an approximate
-// quotient, far closer than its margin, does not already place it behind.
+// quotient, far closer than its margin, does not already place it behind. The
+// approximation is clamped as the depth is: all fragments behind the eye have depth 1
+// and -z decides between them.
 __global__ void __launch_bounds__(256) k_splat(Cam c, const float* __restrict__ pos, int n, int stride,
                                                unsigned long long* depth, unsigned long long* thick) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -109,8 +111,12 @@ __global__ void __launch_bounds__(256) k_splat(Cam c, const float* __restrict__ 
             // surfacePos = viewPos.xyz + radius * vNormal; depth = -surfacePos.z
             const float sx = vx + c.radius * nx, sy = vy + c.radius * ny, sz = vz + c.radius * nz;
             const float qz = row4(c.P, 2, sx, sy, sz), qw = row4(c.P, 3, sx, sy, sz);
-            // behind (an empty pixel's bits are a NaN, which compares false)
-            if (0.5f * __fdividef(qz, qw) + 0.5f > __uint_as_float((unsigned)(cur >> 32)) + 1e-5f) continue;
+            // behind (an empty pixel's bits are a NaN, which compares false); __fdividef
+            // is close for divisors of 2^-126 to 2^126 only
+            const float aw = fabsf(qw);
+            if (aw >= 0x1p-126f && aw <= 0x1p126f &&
+                __saturatef(0.5f * __fdividef(qz, qw) + 0.5f) > __uint_as_float((unsigned)(cur >> 32)) + 1e-5f)
+                continue;
             float fd = 0.5f * (qz / qw) + 0.5f;  // gl_FragDepth
             fd = fminf(fmaxf(fd, 0.0f), 1.0f);
             const unsigned long long key =
@@ -128,7 +134,9 @@ constexpr int SMOOTH_W = 64, SMOOTH_H = SMOOTH_Y + 2 * SMOOTH_STEPS;
 // Depth texture (0 where no sprite: the reference clears it to 0), in both images
 // the smoothing alternates between, and thickness, one smoothing tile per block;
 // tiles with fluid enter the list (tiles[0]: their number) the smoothing runs over.
-// A smoothing step keeps empty pixels empty, so the others stay as written here.
+// A smoothing step leaves an empty pixel's +0 as it is, so the other tiles stay as
+// written here. (Fluid in front of the eye's plane only is listed too: a step turns
+// depths that are not above 0 into +0.)
 __global__ void __launch_bounds__(256) k_resolve(const unsigned long long* __restrict__ depth,
                                                  const unsigned long long* __restrict__ thick, float* __restrict__ z,
                                                  float* __restrict__ z1, float* __restrict__ zraw,
@@ -144,7 +152,7 @@ __global__ void __launch_bounds__(256) k_resolve(const unsigned long long* __res
         z1[o] = v;
         zraw[o] = v;
         th[o] = (float)(long long)thick[o] * (1.0f / kThickScale);
-        any = any || v > 0.0f;
+        any = any || __float_as_uint(v) != 0u;
     }
     if (__syncthreads_or(any) && threadIdx.x == 0) tiles[1 + atomicAdd(tiles, 1)] = blockIdx.y * gridDim.x + blockIdx.x;
 }

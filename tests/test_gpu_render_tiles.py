@@ -26,3 +26,29 @@ def test_smoothing_tile_edges(w, h, iters):
             assert np.array_equal(r.read(name).view(np.uint32), want[name].view(np.uint32)), name
         assert np.abs(r.read("color") - want["color"]).max() <= 2e-5
     r.close()
+
+
+@pytest.mark.parametrize("iters", [0, 6, 13])
+def test_sprites_behind_the_eye(iters):
+    """Particles nearer to the eye than their radius: sprites whose front lies behind
+    the eye have depths below 0, all of window depth 1. The smallest key is kept
+    whatever the order of arrival (the second group's blocks start after the first's
+    are done: what lies between is behind the eye and draws nothing), and smoothing
+    turns such depths into 0, also in tiles without any other."""
+    import math
+    import torch
+    w, h = 210, 50
+    cam = render.make_camera((0.0, 0.0, 1.0), (0.0, 0.0, 0.0), (0.0, 1.0, 0.0), math.radians(45.0), w, h, 0.3,
+                             smooth_iterations=iters)
+    first = np.float32([[-0.1, 0.0, 0.8], [-0.11, 0.01, 0.82], [1.2, 0.3, -3.0]])
+    second = np.float32([[-0.12, 0.0, 0.78], [-0.1, 0.02, 0.81], [-0.11, 0.0, 0.82], [1.6, -0.3, -4.0]])
+    between = np.full((600000, 3), 2.0, np.float32)
+    r = render.Renderer(w, h)
+    r.frame(cam, positions=torch.from_numpy(np.concatenate([first, between, second])).cuda(), stride=3)
+    want = RO.render(cam, np.concatenate([first, second]), w, h)
+    tiles = [want["depth_raw"][y:y + 16, x:x + 52] for y in range(0, h, 16) for x in range(0, w, 52)]
+    assert any((t < 0).any() and not (t > 0).any() for t in tiles)
+    for name in ("depth_raw", "depth", "thickness", "normal", "room"):
+        assert np.array_equal(r.read(name).view(np.uint32), want[name].view(np.uint32)), name
+    assert np.abs(r.read("color") - want["color"]).max() <= 2e-5
+    r.close()
