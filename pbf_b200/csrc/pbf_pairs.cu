@@ -23,7 +23,9 @@
 // a position no particle comes near). A padding entry contributes +0 or -0 to every
 // sum, which leaves the sum unchanged: no accumulator is ever -0 (they start at +0,
 // and in round-to-nearest x + (-x) = +0 and +0 + (-0) = +0). So no entry is tested
-// for the end of its list.
+// for the end of its list, but for the correction with an s_corr exponent that is not
+// a small whole number: a negative one takes a padding entry's weight of 0 to infinity,
+// which times a gradient of 0 is no zero.
 #include "pbf_kernels.h"
 #include "pbf_mlp.h"
 #include "pbf_mlp_dev.cuh"
@@ -49,6 +51,9 @@ __device__ __forceinline__ bool2v below(float2 a, float s, bool2v valid) { retur
 // which components are entries of a list with `left` of them left
 __device__ __forceinline__ bool entries_left(float, int left) { return left > 0; }
 __device__ __forceinline__ bool2v entries_left(float2, int left) { return {left > 0, left > 1}; }
+// which components are gathered particles, not the padding slot
+__device__ __forceinline__ bool is_entry(const float4 (&a)[1]) { return a[0].x != PAD_POSITION; }
+__device__ __forceinline__ bool2v is_entry(const float4 (&a)[2]) { return {a[0].x != PAD_POSITION, a[1].x != PAD_POSITION}; }
 // the first butterfly step: the two lanes of a thread
 __device__ __forceinline__ float fold(float a) { return a; }
 __device__ __forceinline__ float fold(float2 a) { return a.x + a.y; }
@@ -786,7 +791,9 @@ __device__ __forceinline__ void dp_pair(const KParams& p, const f3& xk, float lk
     T3<T> r, g;
     T w;
     pair_terms<T, true>(p, xk, xj, r, w, g);
-    const T s = dp_weight<N4>(p, addw(lk, xj), w);
+    T s = dp_weight<N4>(p, addw(lk, xj), w);
+    // (a padding entry's weight is finite for whole exponents: 0^n = 0)
+    if (!N4 && p.n_int == 0) s = keep_only(s, is_entry(xj));
     a = {vfma(s, g.x, a.x), vfma(s, g.y, a.y), vfma(s, g.z, a.z)};
 }
 struct DpOut {

@@ -94,6 +94,33 @@ def test_scorr_exponents_bitexact(n, exponent):
         assert_substep_bitexact(s, orc)
 
 
+@pytest.mark.parametrize("lanes", [1, 2, 8])
+@pytest.mark.parametrize("n", [1200, 12000])
+def test_scorr_negative_exponent(n, lanes):
+    """A negative exponent makes an entry of weight 0 infinite: none but the list's own
+    entries may enter the sums. powf is good for 4 ulp there and 1 here, and the sums
+    of up to 63 terms follow: 5e-7 + 63 * 6e-8 < 5e-6 of the terms' magnitudes."""
+    sc = block_of(n, iters=1)
+    sc.pos += np.random.RandomState(9).uniform(-0.004, 0.004, size=sc.pos.shape).astype(np.float32)
+    sc.para.n = -0.25
+    s, orc = make_pair(sc, pair_lanes=lanes)
+    s.step(1)
+    orc.substep()
+    want, x, lam = orc.get("dp"), orc.get("xpred").astype(np.float64), orc.get("lambda").astype(np.float64)
+    nbr = orc.get("nbr").reshape(n, -1)
+    j = np.where(nbr < 0, np.arange(n)[:, None], nbr)
+    r = np.linalg.norm(x[:, None] - x[j], axis=2)
+    h = float(sc.para.h)
+    w = np.maximum(h * h - r * r, 1e-30) ** 3 / (h * h - float(sc.para.deltaq) ** 2) ** 3
+    size = np.abs(lam[:, None]) + np.abs(lam[j]) + float(sc.para.k) * w ** -0.25 * s.ext.scorr_scale
+    g = 45.0 / (np.pi * h ** 6) * np.maximum(h - r, 0.0) ** 2
+    terms = np.where(nbr >= 0, size * g, 0.0).sum(1) / float(sc.para.restRho)
+    assert np.isfinite(want).all()
+    assert (np.abs(s.fetch("dp")[:, :3] - want).max(1) <= 5e-6 * terms + 1e-7 * np.abs(want).max(1) + 1e-12).all()
+    s.close()
+    orc.close()
+
+
 @pytest.mark.parametrize("cell", [1.0 / 3.0, 0.5, 0.7, 1.0, 1.5])
 @pytest.mark.parametrize("n", [2100, 46000])
 def test_search_around_the_grid_bitexact(cell, n):
