@@ -191,6 +191,10 @@ KParams make_kparams(const pbf_solver& s) {
     k.visc_c = (e.flags & PBF_FLAG_XSPH_RHO) ? (float)((double)p.c / (double)p.restRho) : p.c;
     k.vort_eps = p.vorticityConfinementEpilon;
     for (int a = 0; a < 3; ++a) k.g[a] = e.gravity[a];
+    float corner = 0.0f;
+    for (const SceneView& v : s.scenes_h)
+        corner = std::max(corner, std::fabs(v.gmin[0]) + std::fabs(v.gmin[1]) + std::fabs(v.gmin[2]));
+    k.clip = p.h * 1e-3f + 1e-6f * corner;
     k.sc0 = s.scenes_h[0];
     k.scenes = s.scenes_d;
     k.sid = s.sid;

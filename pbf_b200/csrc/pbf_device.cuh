@@ -65,6 +65,7 @@ struct KParams {
     // kernel constants, all computed on the host (pbf_capi.cu: make_kparams)
     float h, h2, cell, inv_cell, poly6_c, spiky_c, inv_wdq, nk, scorr_scale, n_exp;
     float rho0, rho0sq, eps, dt, jit, rmin, visc_c, vort_eps;
+    float clip;                 // the search's clipping margin: 1e-3 h + 1e-6 of the largest grid corner's coordinates
     float g[3];
     SceneView sc0;              // the scene when there is one
     const SceneView* scenes;    // device table when nscenes > 1

@@ -383,11 +383,16 @@ __global__ void __launch_bounds__(256, 8) k_reorder(KParams p, const float4* __r
 // applied to the sorted slots. Rows and row ends that lie farther than h from the
 // particle are skipped: a row (dy, dz) is visited only where the distance from the
 // particle to its y and z slabs leaves room within h, and only over the x cells
-// within the remaining half-width. The clipping is conservative (a margin of
-// 1e-3 h plus 1e-6 of the coordinates, far above float rounding), so every
+// within the remaining half-width. The clipping is conservative (clip_margin), so every
 // candidate it drops fails the r^2 <= h^2 test and the lists do not change. Cell 0
 // of an axis reaches one cell below the grid, because cell_dims truncates.
 // ---------------------------------------------------------------------------
+// Above the rounding of the keys and of the cell edges they are compared with: 4 x 2^-24
+// of the distance from the grid's corner, whose coordinates are in KParams::clip.
+__device__ __forceinline__ float clip_margin(const KParams& p, const f3& x) {
+    return p.clip + 1e-6f * (fabsf(x.x) + fabsf(x.y) + fabsf(x.z));
+}
+
 // Where cell t (or a slab of cells) starts along an axis with origin g.
 __device__ __forceinline__ float cell_from(const KParams& p, float g, int t) {
     return g + (float)(t == 0 ? -1 : t) * p.cell;
@@ -420,7 +425,7 @@ __device__ __forceinline__ void neighbors_one(const KParams& p, int k, const flo
     cell_dims(p, sc, xk, d);
     const int nx = sc.dims[0], ny = sc.dims[1], nz = sc.dims[2];
     const int cap = p.max_nbr;
-    const float m = p.h * 1e-3f + 1e-6f * (fabsf(xk.x) + fabsf(xk.y) + fabsf(xk.z));
+    const float m = clip_margin(p, xk);
     const float hm2 = (p.h + m) * (p.h + m);
     // entry i of the list is i step units after entry 0
     const unsigned step = (unsigned)p.stride / 32, last = (unsigned)cap * step;
@@ -634,7 +639,7 @@ __global__ void __launch_bounds__(SEARCH_WIDE_THREADS) k_neighbors_wide(KParams 
     int d[3];
     cell_dims(p, sc, xk, d);
     const int nx = sc.dims[0], ny = sc.dims[1], nz = sc.dims[2];
-    const float m = p.h * 1e-3f + 1e-6f * (fabsf(xk.x) + fabsf(xk.y) + fabsf(xk.z));
+    const float m = clip_margin(p, xk);
     const float hm2 = (p.h + m) * (p.h + m);
     // squared distance, less the margin, to the slab of cells i away (i < 0: below)
     auto slab2 = [&](float q, float g, int cell, int i) {

@@ -146,6 +146,31 @@ def test_search_around_the_grid_bitexact(cell, n):
     orc.close()
 
 
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("persistent", [0, 1])
+@pytest.mark.parametrize("cell", [0.4, 0.5, 1.0])
+def test_search_far_from_the_grids_corner_bitexact(cell, persistent, axis):
+    """A row of particles around the origin of a grid whose corner lies 1,000,000 h away
+    along the row, where keys are rounded by up to 4e-2 h. persistent = 1 takes the
+    search with one thread per particle."""
+    n, far = 1500, 100000.0
+    rng = np.random.RandomState(11)
+    sc = scenes.dam_break(4, (1, 1, 1), stable=True, iterations=1)
+    pos = rng.uniform(0.049, 0.051, size=(n, 3))
+    pos[:, axis] = rng.uniform(-4.0, 4.0, size=n)
+    sc.pos, sc.vel = pos.astype(np.float32), np.zeros((n, 3), np.float32)
+    sc.para.nParticles = n
+    sc.grid_space[axis], sc.boundary[axis], sc.boundary[3 + axis] = -far, -4.2, 4.2
+    dims = [int(np.ceil(1 / cell))] * 3
+    dims[axis] = int((far + 4.5) / (0.1 * cell))
+    s, orc = make_pair(sc, cell_scale=cell, grid_dims=dims, persistent=persistent)
+    s.step(1)
+    orc.substep()
+    assert_substep_bitexact(s, orc)
+    s.close()
+    orc.close()
+
+
 @pytest.mark.parametrize("n,lanes,block,persistent,record", [(75776, 2, 256, 0, 0), (75777, 2, 256, 0, 1),
                                                              (75777, 1, 128, 0, 0), (80001, 8, 256, 0, 1),
                                                              (80001, 4, 64, 1, 0), (160000, 2, 256, 0, 0)])
