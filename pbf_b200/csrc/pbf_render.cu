@@ -62,12 +62,18 @@ __device__ __forceinline__ float dot3(float ax, float ay, float az, float bx, fl
 
 // Sprite depth and thickness of one particle per thread (a warp per sprite with a
 // pixel per lane was slower: 69 against 57 us for 4.2 M fragments, its lanes idle on
-// small sprites). Most fragments lie behind what is already there, so a fragment
-// reads the pixel first, possibly a stale value, which is never below the current
+// small sprites). A few particles are bound by a thread's own chain of fragments, whose
+// atomics nobody waits for. Particles that fill the device are bound by the atomics, and
+// most fragments lie behind what is already there: with LOOK a fragment reads the pixel
+// first, one pixel ahead and possibly a stale value, which is never below the current
 // one, and divides exactly and takes the atomic minimum only when an approximate
 // quotient, far closer than its margin, does not already place it behind. The
 // approximation is clamped as the depth is: all fragments behind the eye have depth 1
-// and -z decides between them.
+// and -z decides between them. With and without, 800 x 800: 262,144 particles 54 / 60 us
+// (sprites of 3 pixels) and 718 / 815 (17); 1 M 1,877 / 2,527; but 110,592 particles 333
+// / 370 and 49 / 42 (6), 20,000 295 / 134, 200 263 / 128 (a read in the chain, not ahead:
+// 309).
+template <bool LOOK>
 __global__ void __launch_bounds__(256) k_splat(Cam c, const float* __restrict__ pos, int n, int stride,
                                                unsigned long long* depth, unsigned long long* thick) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -97,13 +103,16 @@ __global__ void __launch_bounds__(256) k_splat(Cam c, const float* __restrict__ 
         // vNormal.xy = vec2(2, -2) * gl_PointCoord + vec2(-1, 1)
         const float t = 0.5f - ((float)yy + 0.5f - wy) / size;
         const float ny = -2.0f * t + 1.0f;
+        const unsigned long long* row = depth + (size_t)yy * c.w;
+        unsigned long long next = LOOK ? __ldca(row + x0) : 0ull;
         for (int xx = x0; xx <= x1; ++xx) {
+            const unsigned long long cur = LOOK ? next : ~0ull;
+            if (LOOK && xx < x1) next = __ldca(row + xx + 1);
             const float s = ((float)xx + 0.5f - wx) / size + 0.5f;
             const float nx = 2.0f * s + -1.0f;
             const float d2 = nx * nx + ny * ny;
             if (d2 > 1.0f) continue;
             const size_t pix = (size_t)yy * c.w + xx;
-            const unsigned long long cur = __ldca(depth + pix);
             const float nz = sqrtf(1.0f - d2);
             // thickness = 2 * vNormal.z * radius, summed (GL_ONE, GL_ONE blending)
             const float th = 2.0f * nz * c.radius;
@@ -111,12 +120,14 @@ __global__ void __launch_bounds__(256) k_splat(Cam c, const float* __restrict__ 
             // surfacePos = viewPos.xyz + radius * vNormal; depth = -surfacePos.z
             const float sx = vx + c.radius * nx, sy = vy + c.radius * ny, sz = vz + c.radius * nz;
             const float qz = row4(c.P, 2, sx, sy, sz), qw = row4(c.P, 3, sx, sy, sz);
-            // behind (an empty pixel's bits are a NaN, which compares false); __fdividef
-            // is close for divisors of 2^-126 to 2^126 only
-            const float aw = fabsf(qw);
-            if (aw >= 0x1p-126f && aw <= 0x1p126f &&
-                __saturatef(0.5f * __fdividef(qz, qw) + 0.5f) > __uint_as_float((unsigned)(cur >> 32)) + 1e-5f)
-                continue;
+            if (LOOK) {
+                // behind (an empty pixel's bits are a NaN, which compares false); __fdividef
+                // is close for divisors of 2^-126 to 2^126 only
+                const float aw = fabsf(qw);
+                if (aw >= 0x1p-126f && aw <= 0x1p126f &&
+                    __saturatef(0.5f * __fdividef(qz, qw) + 0.5f) > __uint_as_float((unsigned)(cur >> 32)) + 1e-5f)
+                    continue;
+            }
             float fd = 0.5f * (qz / qw) + 0.5f;  // gl_FragDepth
             fd = fminf(fmaxf(fd, 0.0f), 1.0f);
             const unsigned long long key =
@@ -425,7 +436,11 @@ int render_points(pbf_render* r, const float* pos, int n, int stride, const pbf_
     const Cam c = make_cam(*cam, r->w, r->h);
     const dim3 g2((r->w + 255) / 256, r->h);
     k_room<<<g2, 256, 0, st>>>(c, r->room, r->depth, r->thick64, r->tiles);
-    if (n > 0) k_splat<<<(n + 255) / 256, 256, 0, st>>>(c, pos, n, stride, r->depth, r->thick64);
+    if (n > 0) {
+        // (half of the device's threads: see k_splat)
+        const auto splat = n >= 1024 * r->sms ? k_splat<true> : k_splat<false>;
+        splat<<<(n + 255) / 256, 256, 0, st>>>(c, pos, n, stride, r->depth, r->thick64);
+    }
     const dim3 gs((r->w + SMOOTH_X - 1) / SMOOTH_X, (r->h + SMOOTH_Y - 1) / SMOOTH_Y);
     k_resolve<<<gs, 256, 0, st>>>(r->depth, r->thick64, r->z0, r->z1, r->zraw, r->thick, r->w, r->h, r->tiles);
     const float Fy = cam->proj[0], Fx = cam->proj[5];  // the reference's names: Fy = P[0][0], Fx = P[1][1]
