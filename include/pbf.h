@@ -218,6 +218,12 @@ int pbf_host_fence(pbf_solver* s, void* stream);
  * sets the staging up again. */
 int pbf_debug_fail_staging_alloc(int k);
 
+/* Testing hook (host-side fault injection, no reference counterpart): the k-th kernel
+ * launch from here on that goes into a substep's capture (1-based; the scan and the
+ * adaptive loop's bookkeeping not counted) is refused by the runtime; 0 turns it off. The
+ * pbf_step that captures returns PBF_ERR_CUDA and leaves the handle as it was. */
+int pbf_debug_fail_launch(int k);
+
 /* Testing hook (failure injection on the device without a fault, no reference
  * counterpart; the reference's CHECK_CUDA exits the process instead,
  * kernels/cudaPBFSolver.cuh:5-10). Runs one production kernel with a wait that

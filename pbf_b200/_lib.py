@@ -122,6 +122,7 @@ _PROTOS = [
     ("pbf_step_host", C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_void_p]),
     ("pbf_host_fence", C.c_int, [C.c_void_p, C.c_void_p]),
     ("pbf_debug_fail_staging_alloc", C.c_int, [C.c_int]),
+    ("pbf_debug_fail_launch", C.c_int, [C.c_int]),
     ("pbf_debug_expire_wait", C.c_int, [C.c_int, C.POINTER(C.c_int)]),
     ("pbf_measure_fp32_peak", C.c_int, [C.POINTER(C.c_double), C.POINTER(C.c_double)]),
     ("pbf_resize", C.c_int, [C.c_void_p, C.c_int]),

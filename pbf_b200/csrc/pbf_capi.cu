@@ -21,6 +21,7 @@
 
 #include "../../include/pbf.h"
 #include "pbf_kernels.h"
+#include "pbf_launch.cuh"
 #include "pbf_mlp.h"
 
 using namespace pbf;
@@ -238,6 +239,9 @@ cudaError_t staging_malloc(void** p, size_t bytes) {
     if (g_fail_staging_alloc.load() > 0 && g_fail_staging_alloc.fetch_sub(1) == 1) return cudaErrorMemoryAllocation;
     return cudaMalloc(p, bytes);
 }
+
+// The same for the launches of the substep's kernels (pbf_debug_fail_launch).
+std::atomic<int> g_fail_launch{0};
 
 // Mapped host words in which scans report an expired wait, one per call in flight: a page
 // of them per context, made by its first scan and given back with the context. Pages are
@@ -504,7 +508,9 @@ int capture_correction_loop(pbf_solver* s, cudaStream_t st, int first, int min_i
         launch_dp(kl, dbg, s->Q, s->nbr, s->ncnt, s->Pxold, s->Px, nullptr, s->dp_dbg, d, bs);
     }
     cudaGraph_t out = nullptr;
+    const cudaError_t launched = cudaGetLastError();
     CK(cudaStreamEndCapture(bs, &out));
+    if (launched != cudaSuccess) return fail(PBF_ERR_CUDA, "correction loop's launches: %s", cudaGetErrorString(launched));
     const int rc = count_kernel_nodes(body, &s->loop_kernel_nodes);
     s->loop_kernel_nodes /= kLoopUnroll;  // of one correction
     return rc;
@@ -568,11 +574,13 @@ int enqueue_substep(pbf_solver* s, cudaStream_t st) {
             P(ST_LAMBDA, [&] {
                 launch_features(kp, s->Px, s->Pv, s->nbr, s->ncnt, s->lam_prev_sorted, s->Q, s->feat, s->lam_acc, st);
             });
+            int rc = 0;
             if (warm)
                 P(ST_MLP, [&] {
-                    mlp_infer(s->mlp_w, s->mlp_b, s->feat, n, s->lam0, s->Q, s->lam_acc, s->ext.warm_clamp,
-                              s->ext.warm_floor, err, st);
+                    rc = mlp_infer(s->mlp_w, s->mlp_b, s->feat, n, s->lam0, s->Q, s->lam_acc, s->ext.warm_clamp,
+                                   s->ext.warm_floor, err, st);
                 });
+            if (rc) return fail(PBF_ERR_CUDA, "warm-start network: launch failed");
         }
         const bool last = !s->ext.adaptive && iters == 1;
         P(ST_DP, [&] {
@@ -651,12 +659,18 @@ int build_graph(pbf_solver* s) {
     }
     s->prof.clear();
     s->loop_kernel_nodes = 0;
+    cudaGetLastError();  // (what failed before is not the capture's)
     CK(cudaStreamBeginCapture(s->cap_stream, cudaStreamCaptureModeThreadLocal));
-    const int rc = enqueue_substep(s, s->cap_stream);
+    int rc = enqueue_substep(s, s->cap_stream);
+    // A refused launch adds no node and need not end the capture: a graph without one of
+    // the substep's kernels must not run.
+    const cudaError_t launched = cudaGetLastError();
+    if (!rc && launched != cudaSuccess) rc = fail(PBF_ERR_CUDA, "substep's launches: %s", cudaGetErrorString(launched));
     cudaError_t e = cudaStreamEndCapture(s->cap_stream, &s->graph);
     if (rc) {
         if (s->graph) cudaGraphDestroy(s->graph);
         s->graph = nullptr;
+        cudaGetLastError();
         return rc;
     }
     if (e != cudaSuccess) return fail(PBF_ERR_CUDA, "graph capture: %s", cudaGetErrorString(e));
@@ -884,6 +898,8 @@ int create_common(const pbf_solver_parameter* para, int nscenes, const pbf_scene
 
 }  // namespace
 
+bool pbf::refuse_launch() { return g_fail_launch.load() > 0 && g_fail_launch.fetch_sub(1) == 1; }
+
 namespace pbf {
 // Current positions of a solver (float4, slot order) for the renderer.
 int solver_positions(pbf_solver* s, const float4** x, int* n) {
@@ -1066,6 +1082,12 @@ int pbf_measure_fp32_peak(double* scalar_tflops, double* packed_tflops) {
 int pbf_debug_fail_staging_alloc(int k) {
     if (k < 0) return fail(PBF_ERR_INVALID, "k must be >= 0");
     g_fail_staging_alloc.store(k);
+    return PBF_OK;
+}
+
+int pbf_debug_fail_launch(int k) {
+    if (k < 0) return fail(PBF_ERR_INVALID, "k must be >= 0");
+    g_fail_launch.store(k);
     return PBF_OK;
 }
 

@@ -15,11 +15,15 @@ namespace pbf {
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// Launches k, with programmatic stream serialisation when pdl is set; 0 on success.
+// True when this launch is to be refused (pbf_debug_fail_launch; pbf_capi.cu).
+bool refuse_launch();
+
+// Launches k, with programmatic stream serialisation when pdl is set; 0 on success. (A
+// refused launch is also the runtime's last error, which the substep's capture checks.)
 template <typename... P, typename... A>
 int launch(bool pdl, void (*k)(P...), int grid, int block, size_t smem, cudaStream_t st, A... args) {
     cudaLaunchConfig_t c{};
-    c.gridDim = dim3((unsigned)grid);
+    c.gridDim = dim3(refuse_launch() ? 0u : (unsigned)grid);  // (the runtime refuses an empty grid)
     c.blockDim = dim3((unsigned)block);
     c.dynamicSmemBytes = smem;
     c.stream = st;
