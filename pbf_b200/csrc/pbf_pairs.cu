@@ -1322,7 +1322,9 @@ static bool wide(const KParams& p) {
 template <int NV, typename K, typename... A>
 static void launch_wide(const KParams& p, K kernel, cudaStream_t st, A... args) {
     const int smem = wide_smem<NV>(p.max_nbr);  // at most 69 KB (127 entries of two float4)
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (smem > 48 * 1024 &&
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+        return;  // (the runtime's last error: the capture fails)
     const int per = WIDE_THREADS / WIDE;
     launch(p.pdl, kernel, (p.n + per - 1) / per, WIDE_THREADS, smem, st, p, args...);
 }

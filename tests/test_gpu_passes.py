@@ -146,6 +146,29 @@ def test_search_around_the_grid_bitexact(cell, n):
     orc.close()
 
 
+@pytest.mark.parametrize("lanes", [1, 2, 4, 8])
+@pytest.mark.parametrize("cap", [1, 5, 64, 127])
+@pytest.mark.parametrize("n,cell", [(2100, 0.5), (12000, 1.0), (46000, 0.5), (46000, 1.0)])
+def test_neighbour_caps_bitexact(n, cell, cap, lanes):
+    """Lists cut at caps from 1 to 127, in a cloud with about 150 particles within h: the
+    padding goes past the cap into rows of its own, and the eight-thread kernels size
+    their shared memory by it (more than 48 KB from 81 entries on)."""
+    rng = np.random.RandomState(cap)
+    side = (4.19e-3 * n / 150.0) ** (1.0 / 3.0)
+    sc = scenes.dam_break(4, (24, 24, 24), stable=True, iterations=2)
+    sc.pos = rng.uniform(0.2, 0.2 + side, size=(n, 3)).astype(np.float32)
+    sc.vel = np.zeros((n, 3), np.float32)
+    sc.para.nParticles = n
+    s, orc = make_pair(sc, pair_lanes=lanes, cell_scale=cell, max_neighbors=cap,
+                       grid_dims=autotune.dims_for_scale(sc.ext_overrides["grid_dims"], cell))
+    s.step(1)
+    orc.substep()
+    assert (orc.get("ncnt") == cap).any()
+    assert_substep_bitexact(s, orc)
+    s.close()
+    orc.close()
+
+
 @pytest.mark.parametrize("axis", [0, 1, 2])
 @pytest.mark.parametrize("persistent", [0, 1])
 @pytest.mark.parametrize("cell", [0.4, 0.5, 1.0])
