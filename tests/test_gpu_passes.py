@@ -43,6 +43,27 @@ def test_variant_boundaries_bitexact(n, lanes, cell):
     orc.close()
 
 
+@pytest.mark.parametrize("n,lanes,cell", [(9472, 2, 0.5), (9473, 2, 0.5), (9472, 1, 1.0), (9473, 1, 1.0),
+                                          (9473, 4, 0.5), (9473, 8, 0.5), (16385, 2, 1.0), (40961, 2, 0.5),
+                                          (56833, 4, 0.5), (28417, 8, 0.5), (113664, 2, 0.5), (113665, 2, 0.5),
+                                          (113665, 1, 1.0), (113664, 1, 0.5)])
+def test_variant_boundaries_of_released_kernels_bitexact(n, lanes, cell):
+    """The same sizes without debug fields, as users run them: other instances of the
+    kernels, launched programmatically dependent on one another, the graph of one substep
+    replayed after itself."""
+    sc = block_of(n)
+    s, orc = make_pair(sc, debug=0, pair_lanes=lanes, cell_scale=cell,
+                       grid_dims=autotune.dims_for_scale(sc.ext_overrides["grid_dims"], cell))
+    s.step(3)
+    orc.substep(3)
+    assert s.stats()["error_bits"] == 0
+    assert np.array_equal(s.fetch("perm"), orc.get("perm"))
+    for f in ("x", "v", "curl"):
+        assert mismatch(s.fetch(f)[:, :3], orc.get(f))[0] == 0, f
+    s.close()
+    orc.close()
+
+
 @pytest.mark.parametrize("n", [1200, 46000])
 def test_no_corrections_bitexact(n):
     """A substep without corrections keeps the predicted velocities, over several
