@@ -36,10 +36,11 @@ __device__ __forceinline__ float gelu(float z) {
     return 0.5f * z * (1.0f + tanh_fast(u));
 }
 
-// GELU of two values with packed FP32 arithmetic (same expression order)
+// GELU of two values with packed FP32 arithmetic. z + 0.044715 z^3 is one fused
+// multiply-add, said so: the code generator fuses a packed product into the addition
+// that is its only use (pbf_packed.cuh), and every kernel must give the same bits.
 __device__ __forceinline__ float2 gelu2(float2 z) {
-    const float2 z3 = vmul(vmul(vmul(bc<float2>(GELU_A), z), z), z);
-    const float2 u = vmul(bc<float2>(GELU_C), vadd(z, z3));
+    const float2 u = vmul(bc<float2>(GELU_C), vfma(vmul(vmul(bc<float2>(GELU_A), z), z), z, z));
     const float2 t = make_float2(tanh_fast(u.x), tanh_fast(u.y));
     return vmul(vmul(bc<float2>(0.5f), z), vadd(bc<float2>(1.0f), t));
 }

@@ -7,8 +7,10 @@
 namespace pbf {
 
 // The float2 forms are the PTX f32x2 instructions with an explicit .rn rounding
-// modifier, which the compiler never contracts (a multiply feeding an add stays
-// two rounded operations, as in the scalar code built with -fmad=false).
+// modifier. All the same the code generator has been seen to fuse a packed product whose
+// only use is a packed addition into one fma, whatever -fmad says (scalar code built with
+// -fmad=false is left alone): a product that meets an addition is therefore written as
+// vfma, or as vfma(a, b, +0) where both roundings are wanted (and -0 cannot occur).
 __device__ __forceinline__ unsigned long long as_u64(float2 a) {
     return (unsigned long long)__float_as_uint(a.x) | ((unsigned long long)__float_as_uint(a.y) << 32);
 }
