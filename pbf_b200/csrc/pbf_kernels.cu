@@ -158,6 +158,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan(int* __restrict__ cnt, in
                                                        unsigned long long* __restrict__ status, int tiles,
                                                        int* __restrict__ err, int* host_err, int silent_tile,
                                                        long long spin_limit, int* __restrict__ zero, int nzero) {
+    static_assert(VEC || !KEEP, "the solver's arrays are aligned");
     constexpr int TILE = SCAN_THREADS * ITEMS, WARPS = SCAN_THREADS / 32;
     __shared__ int s_tile;
     __shared__ unsigned s_epoch;
@@ -297,10 +298,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan(int* __restrict__ cnt, in
 #pragma unroll
         for (int q = 0; q < ITEMS; ++q) {
             const long long idx = wbase + q * 32 + lane;
-            if (idx < m) {
-                out[idx] = off + item[q];
-                if (KEEP) cnt[idx] = 0;
-            }
+            if (idx < m) out[idx] = off + item[q];
         }
     }
     if (tile == tiles - 1 && t == 0) out[m] = excl + total;  // the grand total

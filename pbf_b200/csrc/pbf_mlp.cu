@@ -24,7 +24,7 @@ namespace pbf {
 using namespace tc;
 
 constexpr int TILE = 128;
-constexpr int TMEM_COLS = 256;      // tile GEMM and backward (at most 2 CTAs per SM by smem)
+constexpr int TMEM_COLS = 256;      // tile GEMM, and training (two products at columns 0 and 128; one CTA per SM by smem)
 constexpr int TMEM_COLS_FWD = 128;  // forward: layers 1 and 3 share columns [0, 64), so 4 CTAs fit an SM
 
 // ---------------------------------------------------------------------------
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(TR_THREADS, 1) k_mlp_train(TrainIO io) {
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const int m = 32 * (warp & 3) + lane;  // this thread's row of the tile
     const int cq = warp >> 2, c0 = 16 * cq;  // and its 16 columns
-    if (warp == 0) tmem_alloc(&tmem_slot, 256);
+    if (warp == 0) tmem_alloc(&tmem_slot, TMEM_COLS);
     if (t == 0) mbar_init(&mbar, 1);
     // what stays zero: rows 64.. of dZ^T, the rows after the ones rows
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(TR_THREADS, 1) k_mlp_train(TrainIO io) {
     }
     fence_before_sync();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tbase, 256);
+    if (warp == 0) tmem_dealloc(tbase, TMEM_COLS);
 }
 
 struct AdamIO {

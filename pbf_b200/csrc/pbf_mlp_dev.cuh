@@ -30,13 +30,8 @@ __device__ __forceinline__ float tanh_fast(float x) {
     return y;
 }
 
-// GELU, tanh form: 0.5 z (1 + tanh(sqrt(2/pi) (z + 0.044715 z^3)))
-__device__ __forceinline__ float gelu(float z) {
-    const float u = GELU_C * (z + GELU_A * z * z * z);
-    return 0.5f * z * (1.0f + tanh_fast(u));
-}
-
-// GELU of two values with packed FP32 arithmetic. z + 0.044715 z^3 is one fused
+// GELU, tanh form, 0.5 z (1 + tanh(sqrt(2/pi) (z + 0.044715 z^3))), of two values with
+// packed FP32 arithmetic. z + 0.044715 z^3 is one fused
 // multiply-add, said so: the code generator fuses a packed product into the addition
 // that is its only use (pbf_packed.cuh), and every kernel must give the same bits.
 __device__ __forceinline__ float2 gelu2(float2 z) {

@@ -35,10 +35,6 @@ __device__ __forceinline__ float2 vfma(float2 a, float2 b, float2 c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(as_u64(a)), "l"(as_u64(b)), "l"(as_u64(c)));
     return as_f2(d);
 }
-__device__ __forceinline__ float vneg(float a) { return -a; }
-__device__ __forceinline__ float2 vneg(float2 a) { return make_float2(-a.x, -a.y); }
-// a - b is a + (-b) exactly, signed zeros included
-template <typename T> __device__ __forceinline__ T vsub(T a, T b) { return vadd(a, vneg(b)); }
 __device__ __forceinline__ float vmax(float a, float b) { return fmaxf(a, b); }
 __device__ __forceinline__ float2 vmax(float2 a, float b) { return make_float2(fmaxf(a.x, b), fmaxf(a.y, b)); }
 
