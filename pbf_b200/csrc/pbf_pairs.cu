@@ -843,8 +843,9 @@ __device__ __forceinline__ void dp_list(const KParams& p, const Team<L>& tm, con
 
 // Adaptive loop: true when this correction is not to be applied (the loop ended
 // before, or ends here because the positions it would correct are within
-// tolerance).
-__device__ __forceinline__ bool dp_skip(const IterCtl& ctl) {
+// tolerance). LOOP: in the device-side loop. The other kernels hold no call that sets a
+// graph's condition: the profiler refuses graph nodes of kernels that do.
+template <bool LOOP> __device__ __forceinline__ bool dp_skip(const IterCtl& ctl) {
     if (!ctl.done) return false;
     const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
     // the lambda pass just measured the positions this pass would correct;
@@ -858,7 +859,7 @@ __device__ __forceinline__ bool dp_skip(const IterCtl& ctl) {
             *ctl.conv_slot = sl;
         }
         if (!over && !met) atomicAdd(ctl.iters, 1);
-        if (ctl.loop_next) {
+        if constexpr (LOOP) {
             *ctl.loop_next = *ctl.loop_k + ctl.loop_add;
             cudaGraphSetConditional(ctl.handle, !over && !met && sl + 1 < ctl.max_slot ? 1u : 0u);
         }
@@ -866,12 +867,12 @@ __device__ __forceinline__ bool dp_skip(const IterCtl& ctl) {
     return over || met;
 }
 
-template <bool DEBUG, bool N4, bool ROOMY, int L, int V>
+template <bool DEBUG, bool N4, bool ROOMY, bool LOOP, int L, int V>
 __global__ void __launch_bounds__(256, ROOMY ? ROOMY_BLOCKS : L == 1 && (N4 || V == 1) ? 5 : 4) k_dp(KParams p, int nvb, const float4* __restrict__ xl,
                                                             const int* __restrict__ nbr, const int* __restrict__ ncnt,
                                                             DpOut o, IterCtl ctl) {
     pdl_wait();
-    if (dp_skip(ctl)) return;
+    if (dp_skip<LOOP>(ctl)) return;
     for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
         const Team<L> tm = team_of<L>(vb);
         if (tm.k < p.n) dp_list<DEBUG, N4, L, V>(p, tm, xl, nbr, ncnt, o);  // uniform over the team
@@ -1176,12 +1177,12 @@ __global__ void __launch_bounds__(WIDE_THREADS) k_lambda_wide(KParams p, const f
     }
 }
 
-template <bool DEBUG, bool N4>
+template <bool DEBUG, bool N4, bool LOOP>
 __global__ void __launch_bounds__(WIDE_THREADS) k_dp_wide(KParams p, const float4* __restrict__ xl,
                                                           const int* __restrict__ nbr, const int* __restrict__ ncnt,
                                                           DpOut o, IterCtl ctl) {
     pdl_wait();
-    if (dp_skip(ctl)) return;
+    if (dp_skip<LOOP>(ctl)) return;
     const WideTeam w = wide_team<1>(p.max_nbr);
     const bool on = w.k < p.n;
     const int cnt = on ? ncnt[w.k] : 0;
@@ -1352,7 +1353,10 @@ void launch_dp(const KParams& p, bool debug, const float4* xl, const int* nbr, c
     const DpOut o{xold, xout, vout, dp};
     if (wide(p)) {
         with_flags(debug, p.n_int == 4, [&](auto d, auto n4) {
-            launch_wide<1>(p, k_dp_wide<decltype(d)::value, decltype(n4)::value>, st, xl, nbr, ncnt, o, ctl);
+            with_flag(ctl.loop_next != nullptr, [&](auto lp) {
+                auto* k = k_dp_wide<decltype(d)::value, decltype(n4)::value, decltype(lp)::value>;
+                launch_wide<1>(p, k, st, xl, nbr, ncnt, o, ctl);
+            });
         });
         return;
     }
@@ -1360,8 +1364,8 @@ void launch_dp(const KParams& p, bool debug, const float4* xl, const int* nbr, c
         constexpr int L = decltype(c)::L, V = decltype(c)::V;
         const int b = team_blocks(p.n, L, p.block);
         with_flags(debug, p.n_int == 4, [&](auto d, auto n4) {
-            with_flag(roomy(p, L), [&](auto r) {
-                auto* k = k_dp<decltype(d)::value, decltype(n4)::value, decltype(r)::value, L, V>;
+            with_flags(roomy(p, L), ctl.loop_next != nullptr, [&](auto r, auto lp) {
+                auto* k = k_dp<decltype(d)::value, decltype(n4)::value, decltype(r)::value, decltype(lp)::value, L, V>;
                 launch(p.pdl, k, pass_grid(p, k, b), p.block, 0, st, p, b, xl, nbr, ncnt, o, ctl);
             });
         });
