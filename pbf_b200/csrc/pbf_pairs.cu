@@ -737,7 +737,7 @@ __global__ void __launch_bounds__(256, 3) k_features_warm(KParams p, int nvb, co
 // the first 4 KB of each tile's H (layer 0 has read it before its epilogue writes
 // there), the next step's rows loaded during this one's layers. 50 KB and 128 TMEM
 // columns: four blocks per SM. Bound by the GELU epilogues' instructions (2,000 per
-// row; 57 % of the issue slots, 43 % of the MUFU's): 262,144 rows take 27.2 us, 28.6
+// row; 56 % of the issue slots, 44 % of the MUFU's): 262,144 rows take 27.2 us, 28.6
 // with one bias per shared load and no early loads, 29.3 in blocks of one tile.
 constexpr int WR_SMEM = FW_SX + 2 * FW_H_TILE;
 constexpr int WR_BLOCKS = 4;
