@@ -1112,8 +1112,8 @@ template <typename K> static int resident_grid(const KParams& p, K kernel, int n
 
 // Particles up to which SEARCH_WIDE threads share one: its time grows with the
 // particles, one thread's walk takes the same until the device is full. Cells of h/2,
-// shared against not: 18.2 / 20.6 us at 32,768 particles, 20.1 / 20.5 at 39,304, 22.9 /
-// 21.1 at 46,656; cells of h: 14.0 / 14.9 at 13,824, 17.6 / 15.2 at 21,952.
+// shared against not: 18.2 / 20.6 us at 32,768 particles, 20.4 / 20.5 at 39,304, 22.9 /
+// 21.1 at 46,656; cells of h: 14.1 / 14.9 at 13,824, 17.6 / 15.2 at 21,952.
 constexpr int SEARCH_WIDE_MAX_N[3] = {0, 16384, 40960};  // by stencil radius
 
 void launch_neighbors(const KParams& p, const float4* x, const int* cell_start, int* nbr, int* ncnt, cudaStream_t st) {
